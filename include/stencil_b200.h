@@ -64,7 +64,8 @@ int sb200_launch_naive(const float* p_cur, const float* p_prev, const float* vel
  * update by the TMA z-marching pencil kernel (FP32, FMA-contracted; within 1e-6
  * relative L2 of the reference order per step).  Grids whose row pitch is not a
  * multiple of 16 bytes (nx % 4 != 0) or with pointers not 16-byte aligned run
- * the naive kernel instead.  Aliasing rules as sb200_launch_naive. */
+ * in the reference order instead (sb200_launch_naive's bits).  Aliasing rules as
+ * sb200_launch_naive. */
 int sb200_launch_tiled(const float* p_cur, const float* p_prev, const float* vel2,
                        float* p_next, const sb200_grid* grid, void* stream);
 
@@ -85,8 +86,8 @@ int sb200_wave_step_f32(const float* p, const float* p_prev, const float* vel2, 
 
 /* sb200_wave_step_f32 evaluated in the reference's operation order with no FMA
  * contraction (the kernel behind sb200_launch_naive): bit-identical to the
- * reference CPU path built with -ffp-contract=off, at about a third of the
- * pencil kernel's throughput.  For callers that need reproducible bits. */
+ * reference CPU path built with -ffp-contract=off, at about 0.85 of the pencil
+ * kernel's throughput.  For callers that need reproducible bits. */
 int sb200_wave_step_exact_f32(const float* p, const float* p_prev, const float* vel2,
                               float* p_next, const sb200_grid* grid, int64_t src_index,
                               float src_amp, void* stream);

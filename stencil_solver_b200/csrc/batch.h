@@ -19,7 +19,8 @@ struct PencilArgs {
     int64_t sy, sz;
     int tiles_x, tiles_y, zlen;
     Weights w;  // acoustic: weights * dt^2; heat: weights * alpha*dt
-    float dt2;  // acoustic: dt^2 (source term)
+    float dt2;  // acoustic: dt^2 (source term); reference order also heat: alpha*dt
+    float inv_dx2, inv_dy2, inv_dz2, one;  // reference order (one = 1)
     int src_x, src_y, src_z;  // -1 when there is no source
     float src_w;
     const float* src_wavelet;

@@ -119,10 +119,56 @@ int default_variant(int kind) {
     return 0;
 }
 
+// Tile of the reference-order steps: 59 separately rounded operations a point leave them
+// short of warps rather than of bytes, and the one-row tile runs 4 CTAs per SM (384^3
+// acoustic: 162 us against 170-175 for the two-row tiles).
+int exact_variant(bool heat) {
+    const char* want = heat ? "t32x16_r1_s8" : "t32x16_r1_s8_a4";
+    const int kind = heat ? SB200_KIND_HEAT_F32 : SB200_KIND_WAVE_F32;
+    for (int v = 0; v < variant_count(kind); ++v)
+        if (std::strcmp(variant_name(kind, v), want) == 0) return v;
+    return 0;
+}
+
+// z splits of an interior of inz planes ranked by how well their CTA count fills whole
+// waves.  A wave is SMs x resident CTAs; a split whose CTA count leaves the last wave
+// mostly empty wastes that fraction of the machine, and every extra split re-reads
+// hplanes halo planes of p (the share pshare of the traffic).
+template <class Ctas>
+std::vector<int> rank_splits(int inz, int resident, int hplanes, double pshare, Ctas ctas_of,
+                             int max_n) {
+    const double slots = double(sm_count()) * std::max(1, resident);
+    std::vector<std::pair<double, int>> scored;
+    for (int zc = 1; zc <= 16 && zc <= inz; ++zc) {
+        const double ctas = double(ctas_of(zc));
+        const double waves = std::ceil(ctas / slots);
+        const double fill = ctas / (waves * slots);
+        const int zlen = (inz + zc - 1) / zc;
+        const double halo = double(zlen) / double(zlen + hplanes) * pshare + (1.0 - pshare);
+        scored.emplace_back(-(fill * halo), zc);
+    }
+    std::stable_sort(scored.begin(), scored.end());
+    std::vector<int> out;
+    for (const auto& s : scored) {
+        if (static_cast<int>(out.size()) >= max_n) break;
+        out.push_back(s.second);
+    }
+    if (out.empty()) out.push_back(1);
+    return out;
+}
+
+// Family of steps with a choice of their own beyond the public kinds: the reference
+// order on the pencil tiles, and the ragged kernels.
+enum Internal : int { kExactWave = 4, kExactHeat, kRaggedWave, kRaggedHeat };
+
 PencilConfig choose(int kind, const GridDesc& g) {
     {
         std::lock_guard<std::mutex> lock(g_cfg_mu);
-        const Override& o = g_override[kind];
+        // the reference order runs the same tiles: an override of the kind holds for it too
+        const int of = kind == kExactWave   ? SB200_KIND_WAVE_F32
+                       : kind == kExactHeat ? SB200_KIND_HEAT_F32
+                                            : kind;
+        const Override o = of < 4 ? g_override[of] : Override();
         if (o.variant >= 0) {
             PencilConfig c;
             c.variant = o.variant;
@@ -131,7 +177,7 @@ PencilConfig choose(int kind, const GridDesc& g) {
         }
     }
     PencilConfig c;
-    if (tuned_choice(kind, g, &c)) return c;
+    if (kind < 4 && tuned_choice(kind, g, &c)) return c;
     // Heuristic pick, memoised per (kind, extents, device): launches stay cheap
     // on the host.
     static std::mutex memo_mu;
@@ -142,11 +188,33 @@ PencilConfig choose(int kind, const GridDesc& g) {
     std::lock_guard<std::mutex> lock(memo_mu);
     auto it = memo.find(key);
     if (it != memo.end()) return it->second;
-    c.variant = default_variant(kind);
-    c.zchunks = zchunk_ranking(kind, c.variant, g, 1).front();
+    const int inz = static_cast<int>(g.nz - 8);
+    if (kind >= kRaggedWave) {
+        // a chunk's start costs about three planes (401 x 357 x 301, acoustic: 2, 4, 6, 8
+        // and 12 chunks 150, 153, 156, 157 and 159 us)
+        c.zchunks = rank_splits(
+                        inz, ragged_resident(kind == kRaggedHeat, g), 3, 1.0,
+                        [&](int zc) { return ragged_ctas(g, zc); }, 1)
+                        .front();
+    } else if (kind >= kExactWave) {
+        const bool heat = kind == kExactHeat;
+        c.variant = exact_variant(heat);
+        c.zchunks = rank_splits(
+                        inz, pencil_f32_resident(heat, c.variant, true), 8, heat ? 0.5 : 0.25,
+                        [&](int zc) { return pencil_f32_ctas(heat, c.variant, g, zc); }, 1)
+                        .front();
+    } else {
+        c.variant = default_variant(kind);
+        c.zchunks = zchunk_ranking(kind, c.variant, g, 1).front();
+    }
     memo[key] = c;
     return c;
 }
+
+// Grids whose reference-order steps stay on the one-thread-per-point kernel: a staged
+// sweep first fills its rings (64^3 acoustic: 5.2 us against 6.2 aligned and 6.6 ragged;
+// 88^3 8.2 against 8.2; 96^3 9.7 against 8.2; 128^3 17.3 against 12.3).
+constexpr int64_t kNaivePoints = int64_t(1) << 19;
 
 bool pencil_ok(const GridDesc& g, std::initializer_list<const void*> ptrs) {
     if (g.nx % 4 != 0) return false;
@@ -179,8 +247,25 @@ int pencil_maps(bool heat, int v, const GridDesc& g, const void* field, const vo
     return SB200_OK;
 }
 
+int ragged_maps(bool heat, const GridDesc& g, const void* field, const void* prev, const void* vel2,
+                PencilMaps* m, const char* where) {
+    const PencilBoxes b = ragged_boxes(heat, g);
+    const int64_t rows = g.ny * g.nz;
+    int rc = tensor_map_rows4(&m->p, field, g.nx, rows, b.halo_x, b.halo_y);
+    m->prev = m->p;
+    m->vel2 = m->p;
+    if (!rc && b.aux_tma) {
+        rc = tensor_map_rows4(&m->prev, prev, g.nx, rows, b.tile_x, b.tile_y);
+        if (!rc) rc = tensor_map_rows4(&m->vel2, vel2, g.nx, rows, b.tile_x, b.tile_y);
+    }
+    if (rc)
+        return fail(SB200_ERR_CUDA, std::string(where) + ": tensor map encode failed (" +
+                                        std::to_string(rc) + ")");
+    return SB200_OK;
+}
+
 int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_next,
-              const sb200_grid* grid, const SourceDesc& src, void* stream, bool allow_pencil,
+              const sb200_grid* grid, const SourceDesc& src, void* stream, bool exact,
               const char* where) {
     const int64_t src_index = src.idx;
     GridDesc g;
@@ -193,15 +278,46 @@ int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_n
         return fail(SB200_ERR_INVALID, std::string(where) + ": source index outside the grid");
     if (!g.has_interior()) return SB200_OK;  // no interior point: nothing to update
     auto st = static_cast<cudaStream_t>(stream);
-    if (allow_pencil && pencil_ok(g, {p, p_prev, vel2, p_next})) {
-        const PencilConfig cfg = choose(SB200_KIND_WAVE_F32, g);
+    const bool staged = g.interior() >= kNaivePoints;
+    if ((staged || !exact) && pencil_ok(g, {p, p_prev, vel2, p_next})) {
+        const PencilConfig cfg = choose(exact ? int(kExactWave) : int(SB200_KIND_WAVE_F32), g);
         PencilMaps maps;
         if (int rc = pencil_maps(false, cfg.variant, g, p, p_prev, vel2, &maps, where)) return rc;
         return finish_launch(launch_wave_pencil_f32(maps, p_prev, vel2, p_next, g, src, cfg,
+                                                    device_error_ptr(), st, exact),
+                             where);
+    }
+    if (staged && ragged_ok(g) && aligned16(p) && aligned16(p_prev) && aligned16(vel2)) {
+        PencilMaps maps;
+        if (int rc = ragged_maps(false, g, p, p_prev, vel2, &maps, where)) return rc;
+        return finish_launch(launch_wave_ragged_f32(maps, p_next, g, src,
+                                                    choose(kRaggedWave, g).zchunks,
                                                     device_error_ptr(), st),
                              where);
     }
     return finish_launch(launch_wave_naive(p, p_prev, vel2, p_next, g, src, st), where);
+}
+
+int heat_step(const float* u, float* u_next, const GridDesc& g, float alpha_dt, void* stream,
+              bool exact, const char* where) {
+    auto st = static_cast<cudaStream_t>(stream);
+    PencilMaps maps;
+    const bool staged = g.interior() >= kNaivePoints;
+    if ((staged || !exact) && pencil_ok(g, {u, u_next})) {
+        const PencilConfig cfg = choose(exact ? int(kExactHeat) : int(SB200_KIND_HEAT_F32), g);
+        if (int rc = pencil_maps(true, cfg.variant, g, u, nullptr, nullptr, &maps, where)) return rc;
+        return finish_launch(launch_heat_pencil_f32(maps, u_next, g, alpha_dt, cfg,
+                                                    device_error_ptr(), st, exact),
+                             where);
+    }
+    if (staged && ragged_ok(g) && aligned16(u)) {
+        if (int rc = ragged_maps(true, g, u, nullptr, nullptr, &maps, where)) return rc;
+        return finish_launch(launch_heat_ragged_f32(maps, u_next, g, alpha_dt,
+                                                    choose(kRaggedHeat, g).zchunks,
+                                                    device_error_ptr(), st),
+                             where);
+    }
+    return finish_launch(launch_heat_naive(u, u_next, g, alpha_dt, st), where);
 }
 
 // Two acoustic steps in one sweep (leap2_f32.cu).  outputs_may_alias lets the
@@ -286,7 +402,7 @@ int wave_step_f16(const uint16_t* p, uint16_t* p_prev_next, const uint16_t* k,
 // engine; the public entry points wrap these.
 int dispatch_wave_f32(const float* p, const float* p_prev, const float* vel2, float* p_next,
                       const sb200_grid* grid, const SourceDesc& src, void* stream, bool exact) {
-    return wave_step(p, p_prev, vel2, p_next, grid, src, stream, !exact,
+    return wave_step(p, p_prev, vel2, p_next, grid, src, stream, exact,
                      exact ? "sb200_wave_step_exact_f32" : "sb200_wave_step_f32");
 }
 
@@ -307,40 +423,20 @@ int set_error(int code, const std::string& msg) { return fail(code, msg); }
 
 int* device_error_word() { return device_error_ptr(); }
 
-// A wave is SMs x resident CTAs; a split whose CTA count leaves the last wave
-// mostly empty wastes that fraction of the machine, and every extra split
-// re-reads 8 halo planes of p (p is 1 of 4 streams for the acoustic kernels,
-// 1 of 2 for heat).
 std::vector<int> zchunk_ranking(int kind, int v, const GridDesc& g, int max_n) {
     const bool f16 = kind == SB200_KIND_WAVE_F16;
     const bool heat = kind == SB200_KIND_HEAT_F32;
     const bool two = kind == SB200_KIND_WAVE2_F32;
-    const int inz = static_cast<int>(g.nz - 8);
     const int resident = two ? leap2_resident(v)
                              : (f16 ? pencil_f16_resident(v) : pencil_f32_resident(heat, v));
-    const double slots = double(sm_count()) * std::max(1, resident);
-    std::vector<std::pair<double, int>> scored;
-    for (int zc = 1; zc <= 16 && zc <= inz; ++zc) {
-        const double ctas = double(two ? leap2_ctas(v, g, zc)
-                                       : (f16 ? pencil_f16_ctas(v, g, zc)
-                                              : pencil_f32_ctas(heat, v, g, zc)));
-        const double waves = std::ceil(ctas / slots);
-        const double fill = ctas / (waves * slots);
-        const int zlen = (inz + zc - 1) / zc;
-        // two steps: p is 4 of the pair's 20 B and a chunk reads 16 halo planes
-        const double pshare = two ? 0.2 : (heat ? 0.5 : 0.25);
-        const int hplanes = two ? 16 : 8;
-        const double halo = double(zlen) / double(zlen + hplanes) * pshare + (1.0 - pshare);
-        scored.emplace_back(-(fill * halo), zc);
-    }
-    std::stable_sort(scored.begin(), scored.end());
-    std::vector<int> out;
-    for (const auto& s : scored) {
-        if (static_cast<int>(out.size()) >= max_n) break;
-        out.push_back(s.second);
-    }
-    if (out.empty()) out.push_back(1);
-    return out;
+    // two steps: p is 4 of the pair's 20 B and a chunk reads 16 halo planes
+    return rank_splits(
+        static_cast<int>(g.nz - 8), resident, two ? 16 : 8, two ? 0.2 : (heat ? 0.5 : 0.25),
+        [&](int zc) {
+            return two ? leap2_ctas(v, g, zc)
+                       : (f16 ? pencil_f16_ctas(v, g, zc) : pencil_f32_ctas(heat, v, g, zc));
+        },
+        max_n);
 }
 
 }  // namespace sb200
@@ -377,19 +473,19 @@ int sb200_upload_fd_coefficients(void) {
 
 int sb200_launch_naive(const float* p_cur, const float* p_prev, const float* vel2,
                        float* p_next, const sb200_grid* grid, void* stream) {
-    return wave_step(p_cur, p_prev, vel2, p_next, grid, host_source(-1, 0.f), stream, false,
+    return wave_step(p_cur, p_prev, vel2, p_next, grid, host_source(-1, 0.f), stream, true,
                      "sb200_launch_naive");
 }
 
 int sb200_launch_tiled(const float* p_cur, const float* p_prev, const float* vel2,
                        float* p_next, const sb200_grid* grid, void* stream) {
-    return wave_step(p_cur, p_prev, vel2, p_next, grid, host_source(-1, 0.f), stream, true,
+    return wave_step(p_cur, p_prev, vel2, p_next, grid, host_source(-1, 0.f), stream, false,
                      "sb200_launch_tiled");
 }
 
 int sb200_launch_slab(const float* p_cur, const float* p_prev, const float* vel2,
                       float* p_next, const sb200_grid* grid, void* stream) {
-    return wave_step(p_cur, p_prev, vel2, p_next, grid, host_source(-1, 0.f), stream, true,
+    return wave_step(p_cur, p_prev, vel2, p_next, grid, host_source(-1, 0.f), stream, false,
                      "sb200_launch_slab");
 }
 
@@ -397,7 +493,7 @@ int sb200_wave_step_f32(const float* p, const float* p_prev, const float* vel2, 
                         const sb200_grid* grid, int64_t src_index, float src_amp,
                         void* stream) {
     return wave_step(p, p_prev, vel2, p_next, grid, host_source(src_index, src_amp), stream,
-                     true, "sb200_wave_step_f32");
+                     false, "sb200_wave_step_f32");
 }
 
 int sb200_wave_step2_f32(const float* p, const float* p_prev, const float* vel2, float* p_next,
@@ -427,7 +523,7 @@ int sb200_wave_step_exact_f32(const float* p, const float* p_prev, const float* 
                               float* p_next, const sb200_grid* grid, int64_t src_index,
                               float src_amp, void* stream) {
     return wave_step(p, p_prev, vel2, p_next, grid, host_source(src_index, src_amp), stream,
-                     false, "sb200_wave_step_exact_f32");
+                     true, "sb200_wave_step_exact_f32");
 }
 
 int sb200_wave_step_dev_f32(const float* p, const float* p_prev, const float* vel2,
@@ -441,7 +537,7 @@ int sb200_wave_step_dev_f32(const float* p, const float* p_prev, const float* ve
     s.wavelet = wavelet;
     s.step = step;
     s.step_offset = step_offset;
-    return wave_step(p, p_prev, vel2, p_next, grid, s, stream, exact == 0,
+    return wave_step(p, p_prev, vel2, p_next, grid, s, stream, exact != 0,
                      "sb200_wave_step_dev_f32");
 }
 
@@ -462,9 +558,7 @@ int sb200_heat_step_exact_f32(const float* u, float* u_next, const sb200_grid* g
     if (!std::isfinite(alpha))
         return fail(SB200_ERR_INVALID, "sb200_heat_step_exact_f32: alpha must be finite");
     if (!g.has_interior()) return SB200_OK;
-    return finish_launch(
-        launch_heat_naive(u, u_next, g, alpha * g.dt, static_cast<cudaStream_t>(stream)),
-        "sb200_heat_step_exact_f32");
+    return heat_step(u, u_next, g, alpha * g.dt, stream, true, "sb200_heat_step_exact_f32");
 }
 
 int sb200_heat_step_f32(const float* u, float* u_next, const sb200_grid* grid, float alpha,
@@ -477,19 +571,7 @@ int sb200_heat_step_f32(const float* u, float* u_next, const sb200_grid* grid, f
     if (!std::isfinite(alpha))
         return fail(SB200_ERR_INVALID, "sb200_heat_step_f32: alpha must be finite");
     if (!g.has_interior()) return SB200_OK;
-    const float alpha_dt = alpha * g.dt;
-    auto st = static_cast<cudaStream_t>(stream);
-    if (pencil_ok(g, {u, u_next})) {
-        const PencilConfig cfg = choose(SB200_KIND_HEAT_F32, g);
-        PencilMaps maps;
-        if (int rc = pencil_maps(true, cfg.variant, g, u, nullptr, nullptr, &maps,
-                                 "sb200_heat_step_f32"))
-            return rc;
-        return finish_launch(
-            launch_heat_pencil_f32(maps, u_next, g, alpha_dt, cfg, device_error_ptr(), st),
-            "sb200_heat_step_f32");
-    }
-    return finish_launch(launch_heat_naive(u, u_next, g, alpha_dt, st), "sb200_heat_step_f32");
+    return heat_step(u, u_next, g, alpha * g.dt, stream, false, "sb200_heat_step_f32");
 }
 
 int sb200_wave_prepass_f32(const float* p, float* p_prev, const float* vel2, float* r,

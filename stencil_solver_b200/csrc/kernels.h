@@ -105,19 +105,36 @@ cudaError_t launch_learned_step(const PencilMaps& maps, float* next, const GridD
 // Laplacian weights of the pencil kernels (C_r / dx_a^2, times `scale`: dt^2 for
 // the acoustic step, alpha dt for heat), rounded once from double.
 Weights fold_weights(const GridDesc& g, float scale);
+// The centre's weight of a heat step: 1 + alpha dt (c0/dx^2 + c0/dy^2 + c0/dz^2).
+float heat_centre(const GridDesc& g, float alpha_dt);
 
 cudaError_t launch_wave_pencil_f32(const PencilMaps& maps, const float* prev, const float* vel2,
                                    float* next, const GridDesc& g, const SourceDesc& src,
-                                   const PencilConfig& cfg, int* err, cudaStream_t stream);
+                                   const PencilConfig& cfg, int* err, cudaStream_t stream,
+                                   bool exact = false);
 cudaError_t launch_heat_pencil_f32(const PencilMaps& maps, float* u_next, const GridDesc& g,
                                    float alpha_dt, const PencilConfig& cfg, int* err,
-                                   cudaStream_t stream);
+                                   cudaStream_t stream, bool exact = false);
 // The acoustic tile `cfg.variant` in prepass mode: r = p + beta dt^2 v^2 lap p,
 // prev += 2 beta dt^2 v^2 lap p (maps as for the acoustic step, prev read and
 // written in place).
 cudaError_t launch_prepass_pencil_f32(const PencilMaps& maps, float* prev, const float* vel2,
                                       float* r, const GridDesc& g, float beta,
                                       const PencilConfig& cfg, int* err, cudaStream_t stream);
+// Reference-order steps of grids with any row length (ragged_f32.cu).  Preconditions:
+// ragged_ok(g), 16-byte aligned p (u), p_prev and vel2 (maps: tensor_map_rows4 with
+// ragged_boxes), has_interior().  next may alias p_prev.
+bool ragged_ok(const GridDesc& g);
+PencilBoxes ragged_boxes(bool heat, const GridDesc& g);
+int ragged_resident(bool heat, const GridDesc& g);
+void ragged_prepare();
+int64_t ragged_ctas(const GridDesc& g, int zchunks);
+cudaError_t launch_wave_ragged_f32(const PencilMaps& maps, float* next, const GridDesc& g,
+                                   const SourceDesc& src, int zchunks, int* err,
+                                   cudaStream_t stream);
+cudaError_t launch_heat_ragged_f32(const PencilMaps& maps, float* u_next, const GridDesc& g,
+                                   float alpha_dt, int zchunks, int* err,
+                                   cudaStream_t stream);
 // Two acoustic steps per sweep (leap2_f32.cu): out1 = p at t+dt, out2 = p at
 // t+2dt, the same bits as two launch_wave_pencil_f32 steps.  maps: p with the
 // leap2_boxes(v) halo box, p_prev and vel2 with its tile box.  p, p_prev, vel2,
@@ -136,7 +153,7 @@ cudaError_t launch_leap2_f32(const PencilMaps& maps, float* out1, float* out2, c
 
 // Resident CTAs per SM of a variant (occupancy query; analytic if that fails).
 // The first call per device also sets the variant's shared-memory attribute.
-int pencil_f32_resident(bool heat, int v);
+int pencil_f32_resident(bool heat, int v, bool exact = false);
 // Sets up every variant on the current device (before a stream capture, whose
 // launches must not be the first ones).
 void pencil_f32_prepare();
@@ -193,5 +210,9 @@ cudaError_t launch_field_stats(const void* field, bool half, const GridDesc& g, 
 // it to *out.  Returns 0 or a CUresult / -1 (driver entry point unavailable).
 int tensor_map_3d(CUtensorMap* out, const void* base, int64_t nx, int64_t ny, int64_t nz,
                   int esize, int box_x, int box_y);
+// The same for an FP32 field seen as lines of four rows: 4 nx words by rows / 4 (a line
+// is a multiple of 16 bytes whatever nx is).
+int tensor_map_rows4(CUtensorMap* out, const void* base, int64_t nx, int64_t rows, int box_x,
+                     int box_y);
 
 }  // namespace sb200

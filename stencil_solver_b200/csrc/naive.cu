@@ -4,9 +4,9 @@
 // in exactly the order of its CPU branch (stencil_naive.cu:151-169): every product and sum
 // goes through __fmul_rn / __fadd_rn, so nvcc cannot contract them into FMAs and the
 // result is bit-identical to the oracle's FP32 restatement built with -ffp-contract=off.
-// They serve as launch_naive, as the fallback for grids the TMA pencil kernels cannot map
-// (row pitch not a multiple of 16 bytes, unaligned base pointers), and as an in-repo
-// cross-check of the pencil kernels.
+// They serve the reference-order steps of grids below 2^19 interior points and of fields
+// whose base is not 16-byte aligned (larger grids: pencil_f32.cu in that order, and
+// ragged_f32.cu where nx % 4 != 0).
 #include "kernels.h"
 #include "sb200_common.cuh"
 

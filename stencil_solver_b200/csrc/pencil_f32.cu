@@ -42,7 +42,13 @@ namespace sb200 {
 
 namespace {
 
-enum Mode : int { kModeAcoustic = 0, kModeHeat = 1, kModePrepass = 2 };
+enum Mode : int {
+    kModeAcoustic = 0,
+    kModeHeat = 1,
+    kModePrepass = 2,
+    kModeExact = 3,      // acoustic in the reference's operation order
+    kModeHeatExact = 4,  // heat in the reference's operation order
+};
 
 template <int TX, int TY, int RPT, int S, int AUX>
 struct Shape {
@@ -71,6 +77,59 @@ struct Ring {
     uint32_t aux = 0;
 };
 
+// Laplacian of the thread's RPT x 4 points in the reference's operation order
+// (src/kernels/stencil_naive.cu:151-169): per axis c0 p / d^2, then for r = 1..4
+// (c_r (p[+r] + p[-r])) / d^2 added, every product and sum rounded by itself, and
+// (x + y) + z.  A product meets its sum as fma(product, one, sum) with `one` = 1 from
+// the kernel's arguments: the same rounding as an add, and nothing that the
+// compiler can contract (it does contract mul.rn.f32x2 into add.rn.f32x2).
+template <int RPT, int SX>
+__device__ __forceinline__ void ordered_lap(const float4 (&q)[9][RPT], const int u, const float* pc,
+                                            const PencilArgs& a, const float2 one,
+                                            float2 (&lap)[RPT][2]) {
+    const float2 c2[R + 1] = {dup2(C0), dup2(C1), dup2(C2), dup2(C3), dup2(C4)};
+    const float2 ix2 = dup2(a.inv_dx2), iy2 = dup2(a.inv_dy2), iz2 = dup2(a.inv_dz2);
+    const int cs = (u + 4) % 9;
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) {
+        const float4 c = q[cs][j];
+        float2 lx[2], ly[2], lz[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float2 t = mul2(c2[0], pair_of(c, h));
+            lx[h] = mul2(t, ix2);
+            ly[h] = mul2(t, iy2);
+            lz[h] = mul2(t, iz2);
+        }
+#pragma unroll
+        for (int r = 1; r <= R; ++r) {
+            const float4 yu = j + r < RPT ? q[cs][j + r < RPT ? j + r : 0] : lds128(pc + (j + r) * SX);
+            const float4 yd = j - r >= 0 ? q[cs][j - r >= 0 ? j - r : 0] : lds128(pc + (j - r) * SX);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 sy = add2(pair_of(yu, h), pair_of(yd, h));
+                ly[h] = fma2(mul2(mul2(c2[r], sy), iy2), one, ly[h]);
+                const float2 sz = add2(pair_of(q[(u + 4 + r) % 9][j], h),
+                                       pair_of(q[(u + 4 - r + 9) % 9][j], h));
+                lz[h] = fma2(mul2(mul2(c2[r], sz), iz2), one, lz[h]);
+            }
+        }
+        const float4 lf = lds128(pc + j * SX - 4);
+        const float4 rt = lds128(pc + j * SX + 4);
+        const float win[12] = {lf.x, lf.y, lf.z, lf.w, c.x, c.y, c.z, c.w, rt.x, rt.y, rt.z, rt.w};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int e = 4 + 2 * h;  // window index of the pair's first lane
+#pragma unroll
+            for (int r = 1; r <= R; ++r) {
+                const float2 s = make_float2(win[e + r] + win[e - r], win[e + 1 + r] + win[e + 1 - r]);
+                lx[h] = fma2(mul2(mul2(c2[r], s), ix2), one, lx[h]);
+            }
+            lap[j][h] = add2(add2(lx[h], ly[h]), lz[h]);
+        }
+    }
+}
+
 // One tile: columns [x0, x0+TX) x [y0, y0+TY) of the interior, marched over the
 // z chunk zc.  All threads of the CTA call it; `sm`, `full` and `auxf` are the
 // CTA's rings, initialised by the caller.  Returns false when a bounded wait gave
@@ -81,8 +140,9 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
                                             int tile_x, int tile_y, int zc, float* sm,
                                             uint64_t* full, uint64_t* auxf, Ring& ring) {
     using P = Shape<TX, TY, RPT, S, AUX>;
-    constexpr bool HEAT = MODE == kModeHeat;
+    constexpr bool HEAT = MODE == kModeHeat || MODE == kModeHeatExact;
     constexpr bool PRE = MODE == kModePrepass;
+    constexpr bool EXACT = MODE == kModeExact || MODE == kModeHeatExact;
     constexpr bool kAuxTma = !HEAT && AUX > 0;
     constexpr int NAUX = AUX > 0 ? AUX : 1;
     float* aux = sm + S * P::PLANE;  // AUX stages of [p_prev tile | vel2 tile]
@@ -146,7 +206,7 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
 
     // Source ownership: which (row, lane element) of this thread, if any.
     int src_j = -1, src_i = -1;
-    if (MODE == kModeAcoustic && a.src_z >= 0 && a.src_x >= gx && a.src_x < gx + 4 && a.src_y >= gy &&
+    if ((MODE == kModeAcoustic || MODE == kModeExact) && a.src_z >= 0 && a.src_x >= gx && a.src_x < gx + 4 && a.src_y >= gy &&
         a.src_y < gy + RPT && xin) {
         src_j = a.src_y - gy;
         src_i = a.src_x - gx;
@@ -160,6 +220,7 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
         az2[r] = dup2(a.w.az[r]);
     }
     const float2 cx2 = dup2(a.w.cx), cy2 = dup2(a.w.cy), cz2 = dup2(a.w.cz), neg1 = dup2(-1.f);
+    const float2 one = dup2(a.one);  // EXACT: see ordered_lap
 
     float4 q[9][RPT];
     bool bad = false;
@@ -206,72 +267,76 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
                 }
                 const float* pc = plane(i + 4) + soff;
 
-                // y: neighbour rows outside the own block from shared memory, own
-                // rows from the queue centre, accumulated from zero in row order
-                // (farthest rows, smallest weights, first).
-                // Pairs of points (lanes 0-1, 2-3 of a float4) as packed f32x2:
-                // per lane exactly the scalar operations in the same order.
-                float2 ya[RPT][2];
+                float2 lap[RPT][2];
+                if constexpr (EXACT) {
+                    ordered_lap<RPT, P::SX>(q, u, pc, a, one, lap);
+                } else {
+                    // y: neighbour rows outside the own block from shared memory, own
+                    // rows from the queue centre, accumulated from zero in row order
+                    // (farthest rows, smallest weights, first).
+                    // Pairs of points (lanes 0-1, 2-3 of a float4) as packed f32x2:
+                    // per lane exactly the scalar operations in the same order.
+                    float2 ya[RPT][2];
 #pragma unroll
-                for (int j = 0; j < RPT; ++j) ya[j][0] = ya[j][1] = make_float2(0.f, 0.f);
+                    for (int j = 0; j < RPT; ++j) ya[j][0] = ya[j][1] = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int k = -R; k < RPT + R; ++k) {
-                    const float4 row = (k >= 0 && k < RPT) ? q[cs][k] : lds128(pc + k * P::SX);
+                    for (int k = -R; k < RPT + R; ++k) {
+                        const float4 row = (k >= 0 && k < RPT) ? q[cs][k] : lds128(pc + k * P::SX);
 #pragma unroll
-                    for (int j = 0; j < RPT; ++j) {
-                        const int d = k > j ? k - j : j - k;
-                        if (d >= 1 && d <= R) {
-                            ya[j][0] = fma2(ay2[d - 1], pair_of(row, 0), ya[j][0]);
-                            ya[j][1] = fma2(ay2[d - 1], pair_of(row, 1), ya[j][1]);
+                        for (int j = 0; j < RPT; ++j) {
+                            const int d = k > j ? k - j : j - k;
+                            if (d >= 1 && d <= R) {
+                                ya[j][0] = fma2(ay2[d - 1], pair_of(row, 0), ya[j][0]);
+                                ya[j][1] = fma2(ay2[d - 1], pair_of(row, 1), ya[j][1]);
+                            }
                         }
                     }
-                }
-                // Acoustic / prepass: lap per axis (centre cancelled against the
-                // r = 1 pair first), combined as (x + y) + z.  Heat: u + lap in two
-                // chains -- the y rows plus the x pairs, and the z pairs -- whose
-                // sum takes the centre through one FMA with heat_c, so `lap` holds
-                // the new value itself.
-                float2 lap[RPT][2];
+                    // Acoustic / prepass: lap per axis (centre cancelled against the
+                    // r = 1 pair first), combined as (x + y) + z.  Heat: u + lap in two
+                    // chains -- the y rows plus the x pairs, and the z pairs -- whose
+                    // sum takes the centre through one FMA with heat_c, so `lap` holds
+                    // the new value itself.
 #pragma unroll
-                for (int j = 0; j < RPT; ++j) {
-                    const float4 c = q[cs][j];
-                    const float4 lf = lds128(pc + j * P::SX - 4);
-                    const float4 rt = lds128(pc + j * P::SX + 4);
-                    const float win[12] = {lf.x, lf.y, lf.z, lf.w, c.x, c.y,
-                                           c.z,  c.w,  rt.x, rt.y, rt.z, rt.w};
+                    for (int j = 0; j < RPT; ++j) {
+                        const float4 c = q[cs][j];
+                        const float4 lf = lds128(pc + j * P::SX - 4);
+                        const float4 rt = lds128(pc + j * P::SX + 4);
+                        const float win[12] = {lf.x, lf.y, lf.z, lf.w, c.x, c.y,
+                                               c.z,  c.w,  rt.x, rt.y, rt.z, rt.w};
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const float2 ce = pair_of(c, h);
-                        if constexpr (HEAT) {
-                            const int e = 4 + 2 * h;  // window index of the pair's first lane
-                            float2 txy = ya[j][h];
-                            float2 tz = make_float2(0.f, 0.f);
-#pragma unroll
-                            for (int r = 1; r <= R; ++r) {
-                                const float2 up = pair_of(q[(u + 4 + r) % 9][j], h);
-                                const float2 dn = pair_of(q[(u + 4 - r + 9) % 9][j], h);
-                                tz = r == 1 ? mul2(az2[0], add2(up, dn))
-                                            : fma2(az2[r - 1], add2(up, dn), tz);
-                                const float2 s = make_float2(win[e + r] + win[e - r],
-                                                             win[e + 1 + r] + win[e + 1 - r]);
-                                txy = fma2(ax2[r - 1], s, txy);
-                            }
-                            lap[j][h] = fma2(dup2(a.heat_c), ce, add2(txy, tz));
-                        } else {
-                            float2 tz = mul2(cz2, ce);
-                            float2 tx = mul2(cx2, ce);
-#pragma unroll
-                            for (int r = 1; r <= R; ++r) {
-                                const float2 up = pair_of(q[(u + 4 + r) % 9][j], h);
-                                const float2 dn = pair_of(q[(u + 4 - r + 9) % 9][j], h);
-                                tz = fma2(az2[r - 1], add2(up, dn), tz);
+                        for (int h = 0; h < 2; ++h) {
+                            const float2 ce = pair_of(c, h);
+                            if constexpr (HEAT) {
                                 const int e = 4 + 2 * h;  // window index of the pair's first lane
-                                const float2 s = make_float2(win[e + r] + win[e - r],
-                                                             win[e + 1 + r] + win[e + 1 - r]);
-                                tx = fma2(ax2[r - 1], s, tx);
+                                float2 txy = ya[j][h];
+                                float2 tz = make_float2(0.f, 0.f);
+#pragma unroll
+                                for (int r = 1; r <= R; ++r) {
+                                    const float2 up = pair_of(q[(u + 4 + r) % 9][j], h);
+                                    const float2 dn = pair_of(q[(u + 4 - r + 9) % 9][j], h);
+                                    tz = r == 1 ? mul2(az2[0], add2(up, dn))
+                                                : fma2(az2[r - 1], add2(up, dn), tz);
+                                    const float2 s = make_float2(win[e + r] + win[e - r],
+                                                                 win[e + 1 + r] + win[e + 1 - r]);
+                                    txy = fma2(ax2[r - 1], s, txy);
+                                }
+                                lap[j][h] = fma2(dup2(a.heat_c), ce, add2(txy, tz));
+                            } else {
+                                float2 tz = mul2(cz2, ce);
+                                float2 tx = mul2(cx2, ce);
+#pragma unroll
+                                for (int r = 1; r <= R; ++r) {
+                                    const float2 up = pair_of(q[(u + 4 + r) % 9][j], h);
+                                    const float2 dn = pair_of(q[(u + 4 - r + 9) % 9][j], h);
+                                    tz = fma2(az2[r - 1], add2(up, dn), tz);
+                                    const int e = 4 + 2 * h;  // window index of the pair's first lane
+                                    const float2 s = make_float2(win[e + r] + win[e - r],
+                                                                 win[e + 1 + r] + win[e + 1 - r]);
+                                    tx = fma2(ax2[r - 1], s, tx);
+                                }
+                                const float2 ty = fma2(cy2, ce, ya[j][h]);
+                                lap[j][h] = add2(add2(tx, ty), tz);
                             }
-                            const float2 ty = fma2(cy2, ce, ya[j][h]);
-                            lap[j][h] = add2(add2(tx, ty), tz);
                         }
                     }
                 }
@@ -290,7 +355,13 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
                 for (int j = 0; j < RPT; ++j) {
                     const float4 c = q[cs][j];
                     float4 o;
-                    if (HEAT) {
+                    if (MODE == kModeHeatExact) {
+                        // 2u - u is exact, so the reference's heat arithmetic is u + k*lap
+                        const float2 k2 = dup2(a.dt2);
+                        const float2 o0 = fma2(mul2(k2, lap[j][0]), one, pair_of(c, 0));
+                        const float2 o1 = fma2(mul2(k2, lap[j][1]), one, pair_of(c, 1));
+                        o = make_float4(o0.x, o0.y, o1.x, o1.y);
+                    } else if (HEAT) {
                         o = make_float4(lap[j][0].x, lap[j][0].y, lap[j][1].x, lap[j][1].y);
                     } else if (PRE) {
                         // weights carry beta dt^2: r = c + vv lap, p_prev += 2 vv lap
@@ -308,19 +379,30 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
                         // exact), as fma(-1, pv, c + c)
                         const float2 t0 = fma2(neg1, pair_of(pv[j], 0), add2(pair_of(c, 0), pair_of(c, 0)));
                         const float2 t1 = fma2(neg1, pair_of(pv[j], 1), add2(pair_of(c, 1), pair_of(c, 1)));
-                        const float2 o0 = fma2(pair_of(vv[j], 0), lap[j][0], t0);
-                        const float2 o1 = fma2(pair_of(vv[j], 1), lap[j][1], t1);
+                        const float2 v0 = pair_of(vv[j], 0), v1 = pair_of(vv[j], 1);
+                        float2 o0, o1;
+                        if constexpr (EXACT) {  // (2c - pv) + (dt^2 v^2) lap, each rounded
+                            const float2 k2 = dup2(a.dt2);
+                            o0 = fma2(mul2(mul2(k2, v0), lap[j][0]), one, t0);
+                            o1 = fma2(mul2(mul2(k2, v1), lap[j][1]), one, t1);
+                        } else {
+                            o0 = fma2(v0, lap[j][0], t0);
+                            o1 = fma2(v1, lap[j][1], t1);
+                        }
                         o = make_float4(o0.x, o0.y, o1.x, o1.y);
                         if (src_j == j && z == a.src_z) {
                             const float wv = a.src_wavelet
                                                  ? a.src_wavelet[*a.src_step + a.src_off]
                                                  : a.src_w;
                             const float kv = a.dt2 * f4get(vv[j], src_i);
-                            const float add = kv * wv;
-                            if (src_i == 0) o.x = o.x + add;
-                            if (src_i == 1) o.y = o.y + add;
-                            if (src_i == 2) o.z = o.z + add;
-                            if (src_i == 3) o.w = o.w + add;
+                            // contracted, or the product rounded first
+                            auto plus = [&](float x) {
+                                return EXACT ? __fadd_rn(x, __fmul_rn(kv, wv)) : fmaf(kv, wv, x);
+                            };
+                            if (src_i == 0) o.x = plus(o.x);
+                            if (src_i == 1) o.y = plus(o.y);
+                            if (src_i == 2) o.z = plus(o.z);
+                            if (src_i == 3) o.w = plus(o.w);
                             if (a.trace)
                                 a.trace[(a.src_step ? *a.src_step : 0) + a.src_off] =
                                     f4get(o, src_i);
@@ -492,6 +574,8 @@ struct Variant {
     LaunchFn launch;
     ResidentFn resident;
     LaunchFn launch_prepass;  // acoustic tiles only: the same shape in prepass mode
+    LaunchFn launch_exact;    // the same shape in the reference's operation order
+    ResidentFn resident_exact;
 };
 
 // The prepass launcher of an acoustic tile (heat tiles have none).
@@ -508,7 +592,9 @@ constexpr LaunchFn prepass_launcher() {
         TX, TY, RPT, S, AUX, NAME,                                                           \
             &launch_variant<TX, TY, RPT, S, AUX, HEAT ? kModeHeat : kModeAcoustic>,          \
             &resident_variant<TX, TY, RPT, S, AUX, HEAT ? kModeHeat : kModeAcoustic>,        \
-            prepass_launcher<TX, TY, RPT, S, AUX, HEAT>()                                    \
+            prepass_launcher<TX, TY, RPT, S, AUX, HEAT>(),                                   \
+            &launch_variant<TX, TY, RPT, S, AUX, HEAT ? kModeHeatExact : kModeExact>,        \
+            &resident_variant<TX, TY, RPT, S, AUX, HEAT ? kModeHeatExact : kModeExact>       \
     }
 
 // Index 0 of each table is the default when no tuned choice exists.
@@ -548,6 +634,12 @@ PencilArgs base_args(int tile_x, int tile_y, const GridDesc& g, int zchunks, int
     a.zlen = (inz + zc - 1) / zc;
     a.src_x = a.src_y = a.src_z = -1;
     a.err = err;
+    // Host-side reciprocals in float, as the reference launcher computes them
+    // (stencil_naive.cu:96-99).
+    a.inv_dx2 = 1.0f / (g.dx * g.dx);
+    a.inv_dy2 = 1.0f / (g.dy * g.dy);
+    a.inv_dz2 = 1.0f / (g.dz * g.dz);
+    a.one = 1.0f;
     return a;
 }
 
@@ -576,6 +668,11 @@ Weights fold_weights(const GridDesc& g, float scale) {
     return w;
 }
 
+float heat_centre(const GridDesc& g, float alpha_dt) {
+    return static_cast<float>(1.0 + double(C0) * alpha_dt *
+                                        (1.0 / (double(g.dx) * g.dx) + 1.0 / (double(g.dy) * g.dy) +
+                                         1.0 / (double(g.dz) * g.dz)));
+}
 
 int pencil_f32_variant_count(bool heat) { return heat ? kNumHeat : kNumWave; }
 
@@ -594,11 +691,14 @@ PencilBoxes pencil_f32_boxes(bool heat, int v) {
     return b;
 }
 
-int pencil_f32_resident(bool heat, int v) { return variant_of(heat, v).resident(); }
+int pencil_f32_resident(bool heat, int v, bool exact) {
+    const Variant& x = variant_of(heat, v);
+    return exact ? x.resident_exact() : x.resident();
+}
 
 void pencil_f32_prepare() {
-    for (int v = 0; v < kNumWave; ++v) kWave[v].resident();
-    for (int v = 0; v < kNumHeat; ++v) kHeat[v].resident();
+    for (const Variant& v : kWave) v.resident(), v.resident_exact();
+    for (const Variant& v : kHeat) v.resident(), v.resident_exact();
 }
 
 int64_t pencil_f32_ctas(bool heat, int v, const GridDesc& g, int zchunks) {
@@ -607,7 +707,8 @@ int64_t pencil_f32_ctas(bool heat, int v, const GridDesc& g, int zchunks) {
 
 cudaError_t launch_wave_pencil_f32(const PencilMaps& maps, const float* prev, const float* vel2,
                                    float* next, const GridDesc& g, const SourceDesc& src,
-                                   const PencilConfig& cfg, int* err, cudaStream_t stream) {
+                                   const PencilConfig& cfg, int* err, cudaStream_t stream,
+                                   bool exact) {
     if (!g.has_interior()) return cudaSuccess;
     const Variant& v = kWave[cfg.variant];
     PencilArgs a = base_args(v.tx, v.ty, g, cfg.zchunks, err);
@@ -626,7 +727,7 @@ cudaError_t launch_wave_pencil_f32(const PencilMaps& maps, const float* prev, co
         a.src_off = src.step_offset;
         a.trace = src.trace;
     }
-    return v.launch(maps, a, ctas_of(a, g), stream);
+    return (exact ? v.launch_exact : v.launch)(maps, a, ctas_of(a, g), stream);
 }
 
 cudaError_t launch_prepass_pencil_f32(const PencilMaps& maps, float* prev, const float* vel2,
@@ -645,17 +746,15 @@ cudaError_t launch_prepass_pencil_f32(const PencilMaps& maps, float* prev, const
 
 cudaError_t launch_heat_pencil_f32(const PencilMaps& maps, float* u_next, const GridDesc& g,
                                    float alpha_dt, const PencilConfig& cfg, int* err,
-                                   cudaStream_t stream) {
+                                   cudaStream_t stream, bool exact) {
     if (!g.has_interior()) return cudaSuccess;
     const Variant& v = kHeat[cfg.variant];
     PencilArgs a = base_args(v.tx, v.ty, g, cfg.zchunks, err);
     a.next = u_next;
+    a.dt2 = alpha_dt;
     a.w = fold_weights(g, alpha_dt);
-    a.heat_c = static_cast<float>(
-        1.0 + double(C0) * alpha_dt *
-                  (1.0 / (double(g.dx) * g.dx) + 1.0 / (double(g.dy) * g.dy) +
-                   1.0 / (double(g.dz) * g.dz)));
-    return v.launch(maps, a, ctas_of(a, g), stream);
+    a.heat_c = heat_centre(g, alpha_dt);
+    return (exact ? v.launch_exact : v.launch)(maps, a, ctas_of(a, g), stream);
 }
 
 // ── batched shots ─────────────────────────────────────────────────────────────

@@ -483,6 +483,7 @@ private:
         // queries, the kernel choice, tensor maps) happens before the capture.
         pencil_f32_prepare();
         pencil_f16_prepare();
+        ragged_prepare();
         int v = 0, z = 0;
         sb200_pencil_choice(heat_ ? SB200_KIND_HEAT_F32
                                   : (fp16_ ? SB200_KIND_WAVE_F16 : SB200_KIND_WAVE_F32),

@@ -40,9 +40,12 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder() {
 
 }  // namespace
 
-int tensor_map_3d(CUtensorMap* out, const void* base, int64_t nx, int64_t ny, int64_t nz,
-                  int esize, int box_x, int box_y) {
-    const Key key{reinterpret_cast<uintptr_t>(base), nx, ny, nz, esize, box_x, box_y};
+namespace {
+
+// Encodes (or takes from the cache) a map of `rank` dimensions: extents n, line strides
+// in bytes of dimensions 1.., the box.
+int cached_map(CUtensorMap* out, const Key& key, const void* base, int rank, const int64_t* n,
+               const int64_t* stride, int esize, const cuuint32_t* box) {
     std::lock_guard<std::mutex> lock(g_mu);
     if (!g_cache) g_cache = new std::map<Key, std::unique_ptr<CUtensorMap>>();
     auto it = g_cache->find(key);
@@ -57,21 +60,37 @@ int tensor_map_3d(CUtensorMap* out, const void* base, int64_t nx, int64_t ny, in
 
     auto map = std::make_unique<CUtensorMap>();
     std::memset(map.get(), 0, sizeof(CUtensorMap));
-    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(nx), static_cast<cuuint64_t>(ny),
-                                static_cast<cuuint64_t>(nz)};
-    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(nx) * esize,
-                                   static_cast<cuuint64_t>(nx) * ny * esize};
-    const cuuint32_t box[3] = {static_cast<cuuint32_t>(box_x), static_cast<cuuint32_t>(box_y), 1};
+    cuuint64_t dims[3], strides[2];
+    for (int d = 0; d < rank; ++d) dims[d] = static_cast<cuuint64_t>(n[d]);
+    for (int d = 0; d + 1 < rank; ++d) strides[d] = static_cast<cuuint64_t>(stride[d]);
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapDataType dt =
         esize == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16;
-    const CUresult r = enc(map.get(), dt, 3, const_cast<void*>(base), dims, strides, box, estr,
+    const CUresult r = enc(map.get(), dt, rank, const_cast<void*>(base), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return static_cast<int>(r);
     *out = *map;
     (*g_cache)[key] = std::move(map);
     return 0;
+}
+
+}  // namespace
+
+int tensor_map_3d(CUtensorMap* out, const void* base, int64_t nx, int64_t ny, int64_t nz,
+                  int esize, int box_x, int box_y) {
+    const int64_t n[3] = {nx, ny, nz}, stride[2] = {nx * esize, nx * ny * esize};
+    const cuuint32_t box[3] = {static_cast<cuuint32_t>(box_x), static_cast<cuuint32_t>(box_y), 1};
+    return cached_map(out, Key{reinterpret_cast<uintptr_t>(base), nx, ny, nz, esize, box_x, box_y},
+                      base, 3, n, stride, esize, box);
+}
+
+int tensor_map_rows4(CUtensorMap* out, const void* base, int64_t nx, int64_t rows, int box_x,
+                     int box_y) {
+    const int64_t n[2] = {4 * nx, rows / 4}, stride[1] = {16 * nx};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_x), static_cast<cuuint32_t>(box_y)};
+    return cached_map(out, Key{reinterpret_cast<uintptr_t>(base), nx, rows, 0, 4, box_x, box_y}, base,
+                      2, n, stride, 4, box);
 }
 
 }  // namespace sb200

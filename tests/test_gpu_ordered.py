@@ -1,0 +1,59 @@
+"""Reference-order steps on the kernels that stage planes by TMA (2^19 interior points
+and more): grids of any row length (rows as lines of four), and the pencil tiles in
+that order on aligned grids; below, the one-thread-per-point kernel.  Bit for bit the
+oracle, halos (and everything outside the interior) untouched."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import oracle
+import stencil_solver_b200 as sb
+
+pytestmark = pytest.mark.gpu
+
+# (nz, ny, nx): one interior plane and column-thin grids; rows of every residue modulo
+# 4 words and planes of every residue; one below, at and above both ragged tiles
+# (64 x 16, 32 x 32); the last size of the one-thread-per-point kernel and the first
+# staged one
+RAGGED = [(9, 733, 741), (10, 520, 521), (2060, 9, 265), (900, 603, 9), (137, 72, 71),
+          (133, 72, 73), (71, 137, 74), (75, 90, 105), (41, 250, 73), (12, 23, 41),
+          (9, 9, 9), (88, 88, 89), (89, 89, 89)]
+ALIGNED = [(9, 733, 740), (133, 72, 72), (75, 90, 108), (12, 24, 40), (2060, 9, 264)]
+
+
+def case(shape, seed):
+    rng = np.random.default_rng(seed)
+    cur, prev = (rng.standard_normal(shape).astype(np.float32) for _ in range(2))
+    vel2 = rng.uniform(1500.0, 4500.0, shape).astype(np.float32) ** 2
+    return cur, prev, vel2
+
+
+@pytest.mark.parametrize("shape", RAGGED + ALIGNED, ids=str)
+def test_steps_bit_for_bit(torch_cuda, shape):
+    nz, ny, nx = shape
+    d, dt = (10.0, 7.5, 12.0), np.float32(1e-3)
+    g = sb.Grid(nx, ny, nz, *d, float(dt))
+    cur, prev, vel2 = case(shape, nx * ny + nz)
+    dev = [torch_cuda.from_numpy(a).cuda() for a in (cur, prev, vel2)]
+    ref = oracle.wave_step(cur, prev, vel2, *d, dt, out=prev.copy())
+    # the source at the far interior corner; in place over p_prev
+    src, amp = g.index(nx - 5, ny - 5, nz - 5), np.float32(0.37)
+    ref.reshape(-1)[src] += np.float32(dt * dt) * vel2.reshape(-1)[src] * amp
+    for step in (sb.wave_step_exact, sb.wave_step) if nx % 4 else (sb.wave_step_exact,):
+        out = dev[1].clone()
+        step(dev[0], out, dev[2], out, g, src, float(amp))
+        assert np.array_equal(out.cpu().numpy(), ref)
+    # an output that no 16-byte store could reach
+    room = torch_cuda.zeros(cur.size + 1, device="cuda")
+    out = room[1:].view(shape)
+    sb.launch_naive(*dev, out, g)
+    assert np.array_equal(out.cpu().numpy(), oracle.wave_step(cur, prev, vel2, *d, dt))
+    # u + (alpha dt) lap: the wave arithmetic with p_prev = u, dt = 1 and v^2 = alpha dt
+    k = np.full(shape, np.float32(900.0) * dt, np.float32)
+    heat = oracle.wave_step(cur, cur, k, *d, np.float32(1.0), out=prev.copy())
+    for step in (sb.heat_step_exact, sb.heat_step) if nx % 4 else (sb.heat_step_exact,):
+        out = dev[1].clone()
+        step(dev[0], out, g, 900.0)
+        assert np.array_equal(out.cpu().numpy(), heat)
+    assert sb.device_error() == 0
