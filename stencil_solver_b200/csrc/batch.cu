@@ -51,6 +51,7 @@ constexpr int kZlens[] = {0, 128, 64, 32};
 // Stability monitor of one shot: a non-finite value or max |p| above the limit
 // (FP64 statistics {sum p^2, max |p|, non-finite count}) sets its flag.
 __global__ void batch_monitor_kernel(const double* stats3, int* flag, double limit) {
+    launch_order();
     if (!(stats3[2] == 0.0) || !(stats3[1] <= limit)) *flag = 1;
 }
 
@@ -275,10 +276,11 @@ public:
                      : sb200_field_stats_f32(reinterpret_cast<const float*>(arena_ + h.off[par]),
                                              &gg, stats_ + 3 * s, scratch_, scratch_len_, st_);
             if (rc) return rc;
-            batch_monitor_kernel<<<1, 1, 0, st_>>>(stats_ + 3 * s, mon_ + s,
-                                                   f16_ ? 1e300 : monitor_limit_);
+            if (int r2 = cuda(launch_after(batch_monitor_kernel, 1, 1, 0, st_, stats_ + 3 * s, mon_ + s,
+                                           f16_ ? 1e300 : monitor_limit_)))
+                return r2;
         }
-        return cuda(cudaGetLastError());
+        return SB200_OK;
     }
 
     int set_monitor_limit(float limit) {
@@ -588,7 +590,9 @@ private:
             if (int rc = sb200_field_stats_f16(reinterpret_cast<const uint16_t*>(arena_ + h.off[par]),
                                                &gg, 1.f, stats_ + 3 * s, scratch_, scratch_len_, st_))
                 return rc;
-            batch_monitor_kernel<<<1, 1, 0, st_>>>(stats_ + 3 * s, mon_ + s, 1e300);
+            if (int rc = cuda(launch_after(batch_monitor_kernel, 1, 1, 0, st_, stats_ + 3 * s, mon_ + s,
+                                           1e300)))
+                return rc;
             if (int rc = sb200_f16_renorm(stats_ + 3 * s, reinterpret_cast<sb200_f16_scale*>(scale_ + s),
                                           bound_ + s * cap_, &queue_->step, 0.f, kTarget, st_))
                 return rc;

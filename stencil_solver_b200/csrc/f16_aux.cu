@@ -51,6 +51,7 @@ __global__ void k_bf16_kernel(const float* __restrict__ vel2, uint16_t* __restri
 
 __global__ void renorm_kernel(const double* stats3, F16Scale* scale, const float* bound,
                               const int* step, float bound_host, float target) {
+    launch_order();
     const double a_old = scale->a;
     const double m = stats3[1] / a_old;  // stats were taken in stored units
     const double b = bound ? double(bound[*step]) : double(bound_host);
@@ -90,8 +91,7 @@ cudaError_t launch_k_bf16(const float* vel2, uint16_t* k, int64_t n, float dt2_o
 
 cudaError_t launch_f16_renorm(const double* stats3, F16Scale* scale, const float* bound,
                               const int* step, float bound_host, float target, cudaStream_t st) {
-    renorm_kernel<<<1, 1, 0, st>>>(stats3, scale, bound, step, bound_host, target);
-    return cudaGetLastError();
+    return launch_after(renorm_kernel, 1, 1, 0, st, stats3, scale, bound, step, bound_host, target);
 }
 
 }  // namespace sb200

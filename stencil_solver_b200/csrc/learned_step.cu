@@ -319,6 +319,8 @@ __global__ void __launch_bounds__(LNT, 3)
     learned_step_kernel(const __grid_constant__ CUtensorMap pmap,
                         const __grid_constant__ CUtensorMap qmap,
                         const __grid_constant__ CUtensorMap vmap, const LearnedArgs a) {
+    // (before the TMEM allocation: a block that waits for the previous grid holds none)
+    launch_order();
     extern __shared__ unsigned char dyn[];
     __shared__ __align__(8) uint64_t full[PS];  // the fused path uses the first LS
     __shared__ __align__(8) uint64_t auxf[PAUX];
@@ -752,8 +754,9 @@ namespace {
 // hold a value at or above the flag threshold in a chunk only where a star of p
 // reaches one, i.e. where chunk_active holds for p's flags (L is a 25-point
 // star); such chunks get every bit (their face slabs are not resolved further).
-__global__ void flags_compose_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out,
+__global__ void flags_compose_kernel(const uint8_t* in, uint8_t* out,
                                      int tiles_x, int tiles_y, int zchunks) {
+    launch_order();
     const int64_t n = int64_t(tiles_x) * tiles_y * zchunks;
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -778,9 +781,8 @@ cudaError_t launch_flags_compose(const uint8_t* in, uint8_t* out, const GridDesc
     const LearnedChunks c = learned_step_chunks(g, sms, true);
     const int64_t n = int64_t(c.tiles_x) * c.tiles_y * c.zchunks;
     if (n == 0) return cudaSuccess;
-    flags_compose_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(
-        in, out, c.tiles_x, c.tiles_y, c.zchunks);
-    return cudaGetLastError();
+    return launch_after(flags_compose_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0, stream,
+                        in, out, c.tiles_x, c.tiles_y, c.zchunks);
 }
 
 LearnedChunks learned_step_chunks(const GridDesc& g, int sms, bool flagged) {
@@ -846,8 +848,8 @@ cudaError_t launch_learned_step(const PencilMaps& maps, float* next, const GridD
     }
     a.b3 = net.b3;
     a.err = err;
-    learned_step_kernel<<<ctas, LNT, kLSmem, stream>>>(maps.p, maps.prev, maps.vel2, a);
-    return cudaGetLastError();
+    return launch_after(learned_step_kernel, ctas, LNT, kLSmem, stream, maps.p, maps.prev, maps.vel2,
+                        a);
 }
 
 }  // namespace sb200

@@ -418,9 +418,10 @@ __global__ void restrict2_kernel(const float* __restrict__ fine, int64_t fnx, in
 
 // field[box] += scale * pattern over a bx x by x bz box at (x0, y0, z0) (a
 // spatially extended source); cells outside the grid's interior are skipped.
-__global__ void add_box_kernel(float* __restrict__ f, int64_t nx, int64_t ny, int64_t nz, int x0,
+__global__ void add_box_kernel(float* f, int64_t nx, int64_t ny, int64_t nz, int x0,
                                int y0, int z0, int bx, int by, int bz,
-                               const float* __restrict__ pattern, float scale) {
+                               const float* pattern, float scale) {
+    launch_order();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= bx * by * bz) return;
     const int64_t x = x0 + i % bx, y = y0 + (i / bx) % by, z = z0 + i / (bx * by);
@@ -1052,9 +1053,10 @@ int sb200_add_box(float* field, const sb200_grid* grid, int x0, int y0, int z0, 
         return set_error(SB200_ERR_INVALID, "sb200_add_box: bad arguments");
     const int n = bx * by * bz;
     if (n == 0) return SB200_OK;
-    add_box_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        field, grid->nx, grid->ny, grid->nz, x0, y0, z0, bx, by, bz, pattern, scale);
-    return cuda_err(cudaGetLastError(), "sb200_add_box");
+    return cuda_err(launch_after(add_box_kernel, (n + 255) / 256, 256, 0,
+                                 static_cast<cudaStream_t>(stream), field, grid->nx, grid->ny,
+                                 grid->nz, x0, y0, z0, bx, by, bz, pattern, scale),
+                    "sb200_add_box");
 }
 
 int sb200_smooth3(float* field, float* tmp, const sb200_grid* grid, float sigma_cells,

@@ -32,6 +32,7 @@ struct NaiveArgs {
 
 template <bool kHeat>
 __global__ void __launch_bounds__(256) naive_kernel(NaiveArgs a) {
+    launch_order();
     const int64_t ix = R + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t iy = R + static_cast<int64_t>(blockIdx.y) * blockDim.y + threadIdx.y;
     const int64_t iz = R + static_cast<int64_t>(blockIdx.z) * blockDim.z + threadIdx.z;
@@ -113,26 +114,26 @@ cudaError_t launch_wave_naive(const float* cur, const float* prev, const float* 
     a.step = src.step;
     a.step_off = src.step_offset;
     a.trace = src.trace;
-    naive_kernel<false><<<naive_grid(g, block), block, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_after(naive_kernel<false>, naive_grid(g, block), block, 0, stream, a);
 }
 
 namespace {
-__global__ void set_int_kernel(int* dst, int value) { *dst = value; }
+__global__ void set_int_kernel(int* dst, int value) {
+    launch_order();
+    *dst = value;
+}
 }  // namespace
 
 cudaError_t launch_set_int(int* dst, int value, cudaStream_t stream) {
-    set_int_kernel<<<1, 1, 0, stream>>>(dst, value);
-    return cudaGetLastError();
+    return launch_after(set_int_kernel, 1, 1, 0, stream, dst, value);
 }
 
 cudaError_t launch_heat_naive(const float* u, float* u_next, const GridDesc& g, float alpha_dt,
                               cudaStream_t stream) {
     if (!g.has_interior()) return cudaSuccess;
     const dim3 block(32, 4, 2);
-    naive_kernel<true><<<naive_grid(g, block), block, 0, stream>>>(
-        make_args(u, nullptr, nullptr, u_next, g, alpha_dt, -1, 0.0f));
-    return cudaGetLastError();
+    return launch_after(naive_kernel<true>, naive_grid(g, block), block, 0, stream,
+                        make_args(u, nullptr, nullptr, u_next, g, alpha_dt, -1, 0.0f));
 }
 
 }  // namespace sb200

@@ -520,6 +520,7 @@ __global__ void __launch_bounds__(ShapeH<TX, TY, S, AUX>::NT, ShapeH<TX, TY, S, 
     __shared__ __align__(8) uint64_t auxf[AUX];
     uint16_t* sm = reinterpret_cast<uint16_t*>(smem_align<128>(dsmem));
     if (threadIdx.x == 0) init_rings_f16<S, AUX>(full, auxf);
+    launch_order();
     __syncthreads();
     int b = blockIdx.x;
     const int tx = b % a.tiles_x;
@@ -545,6 +546,7 @@ __global__ void __launch_bounds__(ShapeH<TX, TY, S, AUX>::NT, ShapeH<TX, TY, S, 
     __shared__ int s_item;
     uint16_t* sm = reinterpret_cast<uint16_t*>(smem_align<128>(dsmem));
     if (threadIdx.x == 0) init_rings_f16<S, AUX>(full, auxf);
+    launch_order();
     RingH ring;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(&queue->next, 1);
@@ -617,29 +619,25 @@ int resident_f16() {
 }
 
 template <int TX, int TY, int S, int AUX, int UNR, int UPD>
-void launch_f16_form(const PencilMaps& m, const F16Args& a, unsigned ctas, int phase,
+cudaError_t launch_f16_form(const PencilMaps& m, const F16Args& a, unsigned ctas, int phase,
                      cudaStream_t stream) {
     using P = ShapeH<TX, TY, S, AUX>;
     if (phase == 1)
-        pencil_f16_kernel<TX, TY, S, AUX, 1, UNR, UPD><<<ctas, P::NT, P::SMEM, stream>>>(m.p, m.prev,
-                                                                                     m.vel2, a);
-    else if (phase == 2)
-        pencil_f16_kernel<TX, TY, S, AUX, 2, UNR, UPD><<<ctas, P::NT, P::SMEM, stream>>>(m.p, m.prev,
-                                                                                     m.vel2, a);
-    else
-        pencil_f16_kernel<TX, TY, S, AUX, 0, UNR, UPD><<<ctas, P::NT, P::SMEM, stream>>>(m.p, m.prev,
-                                                                                     m.vel2, a);
+        return launch_after(pencil_f16_kernel<TX, TY, S, AUX, 1, UNR, UPD>, ctas, P::NT, P::SMEM,
+                            stream, m.p, m.prev, m.vel2, a);
+    if (phase == 2)
+        return launch_after(pencil_f16_kernel<TX, TY, S, AUX, 2, UNR, UPD>, ctas, P::NT, P::SMEM,
+                            stream, m.p, m.prev, m.vel2, a);
+    return launch_after(pencil_f16_kernel<TX, TY, S, AUX, 0, UNR, UPD>, ctas, P::NT, P::SMEM, stream,
+                        m.p, m.prev, m.vel2, a);
 }
 
 template <int TX, int TY, int S, int AUX, int UNR>
 cudaError_t launch_f16(const PencilMaps& m, const F16Args& a, unsigned ctas, int phase,
                        bool exact_y, cudaStream_t stream) {
     resident_f16<TX, TY, S, AUX, UNR>();  // sets the attributes once per device
-    if (exact_y)
-        launch_f16_form<TX, TY, S, AUX, UNR, kFormExactY>(m, a, ctas, phase, stream);
-    else
-        launch_f16_form<TX, TY, S, AUX, UNR, kFormPlain>(m, a, ctas, phase, stream);
-    return cudaGetLastError();
+    return exact_y ? launch_f16_form<TX, TY, S, AUX, UNR, kFormExactY>(m, a, ctas, phase, stream)
+                   : launch_f16_form<TX, TY, S, AUX, UNR, kFormPlain>(m, a, ctas, phase, stream);
 }
 
 struct VariantH {
@@ -789,18 +787,17 @@ int resident_batch_f16() {
 }
 
 template <int TX, int TY, int S, int AUX, int UNR, int UPD>
-void launch_batch_f16_form(const ShotF16* shots, const int4* items, int n_items,
+cudaError_t launch_batch_f16_form(const ShotF16* shots, const int4* items, int n_items,
                            BatchQueue* queue, unsigned ctas, int phase, cudaStream_t stream) {
     using P = ShapeH<TX, TY, S, AUX>;
     if (phase == 1)
-        batch_f16_kernel<TX, TY, S, AUX, 1, UNR, UPD><<<ctas, P::NT, P::SMEM, stream>>>(shots, items,
-                                                                                    n_items, queue);
-    else if (phase == 2)
-        batch_f16_kernel<TX, TY, S, AUX, 2, UNR, UPD><<<ctas, P::NT, P::SMEM, stream>>>(shots, items,
-                                                                                    n_items, queue);
-    else
-        batch_f16_kernel<TX, TY, S, AUX, 0, UNR, UPD><<<ctas, P::NT, P::SMEM, stream>>>(shots, items,
-                                                                                    n_items, queue);
+        return launch_after(batch_f16_kernel<TX, TY, S, AUX, 1, UNR, UPD>, ctas, P::NT, P::SMEM,
+                            stream, shots, items, n_items, queue);
+    if (phase == 2)
+        return launch_after(batch_f16_kernel<TX, TY, S, AUX, 2, UNR, UPD>, ctas, P::NT, P::SMEM,
+                            stream, shots, items, n_items, queue);
+    return launch_after(batch_f16_kernel<TX, TY, S, AUX, 0, UNR, UPD>, ctas, P::NT, P::SMEM, stream,
+                        shots, items, n_items, queue);
 }
 
 template <int TX, int TY, int S, int AUX, int UNR>
@@ -808,13 +805,10 @@ cudaError_t launch_batch_f16_t(const ShotF16* shots, const int4* items, int n_it
                                BatchQueue* queue, unsigned ctas, int phase, bool exact_y,
                                cudaStream_t stream) {
     resident_batch_f16<TX, TY, S, AUX, UNR>();  // sets the attributes once per device
-    if (exact_y)
-        launch_batch_f16_form<TX, TY, S, AUX, UNR, kFormExactY>(shots, items, n_items, queue, ctas,
-                                                              phase, stream);
-    else
-        launch_batch_f16_form<TX, TY, S, AUX, UNR, kFormPlain>(shots, items, n_items, queue, ctas,
-                                                             phase, stream);
-    return cudaGetLastError();
+    return exact_y ? launch_batch_f16_form<TX, TY, S, AUX, UNR, kFormExactY>(
+                         shots, items, n_items, queue, ctas, phase, stream)
+                   : launch_batch_f16_form<TX, TY, S, AUX, UNR, kFormPlain>(
+                         shots, items, n_items, queue, ctas, phase, stream);
 }
 
 struct VariantB16 {

@@ -462,6 +462,7 @@ __device__ __forceinline__ float* setup_rings(unsigned char* dsmem, uint64_t* fu
         for (int s = 0; s < NAUX; ++s) mbar_init(&auxf[s], 1);
         fence_barrier_init();
     }
+    launch_order();
     __syncthreads();
     return reinterpret_cast<float*>(smem_align<128>(dsmem));
 }
@@ -563,9 +564,8 @@ cudaError_t launch_variant(const PencilMaps& m, const PencilArgs& a, unsigned ct
     using P = Shape<TX, TY, RPT, S, AUX>;
     // Sets the shared-memory attribute on the first call per device (cached).
     resident_variant<TX, TY, RPT, S, AUX, MODE>();
-    pencil_f32_kernel<TX, TY, RPT, S, AUX, MODE><<<ctas, P::NT, P::SMEM, stream>>>(m.p, m.prev,
-                                                                                 m.vel2, a);
-    return cudaGetLastError();
+    return launch_after(pencil_f32_kernel<TX, TY, RPT, S, AUX, MODE>, ctas, P::NT, P::SMEM, stream,
+                        m.p, m.prev, m.vel2, a);
 }
 
 struct Variant {
@@ -788,9 +788,8 @@ cudaError_t launch_batch(const ShotF32* shots, const int4* items, int n_items, B
                          unsigned ctas, cudaStream_t stream) {
     using P = Shape<TX, TY, RPT, S, AUX>;
     resident_batch<TX, TY, RPT, S, AUX>();
-    batch_f32_kernel<TX, TY, RPT, S, AUX><<<ctas, P::NT, P::SMEM, stream>>>(shots, items, n_items,
-                                                                           q);
-    return cudaGetLastError();
+    return launch_after(batch_f32_kernel<TX, TY, RPT, S, AUX>, ctas, P::NT, P::SMEM, stream, shots,
+                        items, n_items, q);
 }
 
 struct BatchVariant {

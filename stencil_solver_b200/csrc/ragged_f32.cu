@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(RaggedShape<TX, TY>::NT, 512 / RaggedShape<TX,
         for (int s = 0; s < RG; ++s) mbar_init(&full[s], 4);
         fence_barrier_init();
     }
+    launch_order();
     __syncthreads();
 
     int b = blockIdx.x;
@@ -341,9 +342,8 @@ template <int TX, int TY, bool HEAT>
 cudaError_t launch(const PencilMaps& m, const RaggedArgs& a, unsigned ctas, cudaStream_t stream) {
     using P = RaggedShape<TX, TY>;
     resident<TX, TY, HEAT>();
-    ragged_f32_kernel<TX, TY, HEAT><<<ctas, P::NT, P::smem(HEAT), stream>>>(m.p, m.prev,
-                                                                                  m.vel2, a);
-    return cudaGetLastError();
+    return launch_after(ragged_f32_kernel<TX, TY, HEAT>, ctas, P::NT, P::smem(HEAT), stream, m.p,
+                        m.prev, m.vel2, a);
 }
 
 struct Shape {

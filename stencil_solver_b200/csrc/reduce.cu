@@ -70,6 +70,7 @@ template <typename T>
 __global__ void __launch_bounds__(kStatsThreads)
     stats_partial_kernel(const T* f, int64_t nx, int64_t ny, int64_t nz, float inv_scale,
                          double* partials) {
+    launch_order();
     const int64_t ix = nx - 2 * R, iy = ny - 2 * R, iz = nz - 2 * R;
     const int64_t rows = iy * iz;
     double s = 0.0, m = 0.0, bad = 0.0;
@@ -99,6 +100,7 @@ __global__ void __launch_bounds__(kStatsThreads)
 // so repeated runs give identical bits).
 __global__ void __launch_bounds__(kStatsThreads)
     stats_final_kernel(const double* partials, int nparts, double* out) {
+    launch_order();
     double s = 0.0, m = 0.0, bad = 0.0;
     for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
         s += partials[3 * i + 0];
@@ -124,16 +126,13 @@ cudaError_t launch_field_stats(const void* field, bool half, const GridDesc& g, 
                                double* out3, double* scratch, cudaStream_t stream) {
     const int nb = stats_blocks(g);
     const float inv = 1.0f / scale;
-    if (half)
-        stats_partial_kernel<__half><<<nb, kStatsThreads, 0, stream>>>(
-            static_cast<const __half*>(field), g.nx, g.ny, g.nz, inv, scratch);
-    else
-        stats_partial_kernel<float><<<nb, kStatsThreads, 0, stream>>>(
-            static_cast<const float*>(field), g.nx, g.ny, g.nz, inv, scratch);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e =
+        half ? launch_after(stats_partial_kernel<__half>, nb, kStatsThreads, 0, stream,
+                            static_cast<const __half*>(field), g.nx, g.ny, g.nz, inv, scratch)
+             : launch_after(stats_partial_kernel<float>, nb, kStatsThreads, 0, stream,
+                            static_cast<const float*>(field), g.nx, g.ny, g.nz, inv, scratch);
     if (e != cudaSuccess) return e;
-    stats_final_kernel<<<1, kStatsThreads, 0, stream>>>(scratch, nb, out3);
-    return cudaGetLastError();
+    return launch_after(stats_final_kernel, 1, kStatsThreads, 0, stream, scratch, nb, out3);
 }
 
 }  // namespace sb200

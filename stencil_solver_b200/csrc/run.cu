@@ -27,6 +27,7 @@
 
 #include "dispatch.h"
 #include "kernels.h"
+#include "sb200_common.cuh"
 #include "stencil_b200.h"
 
 namespace sb200 {
@@ -34,6 +35,7 @@ namespace sb200 {
 namespace {
 
 __global__ void monitor_kernel(const double* stats3, int* flag, double limit) {
+    launch_order();
     if (!(stats3[2] == 0.0) || !(stats3[1] <= limit)) atomicExch(flag, 1);
 }
 
@@ -396,8 +398,7 @@ private:
     }
 
     int monitor(double limit) {
-        monitor_kernel<<<1, 1, 0, st_>>>(stats_dev_, monitor_dev_, limit);
-        return cuda(cudaGetLastError());
+        return cuda(launch_after(monitor_kernel, 1, 1, 0, st_, stats_dev_, monitor_dev_, limit));
     }
 
     // One step.  device_src: read the source sample / write the trace through
