@@ -196,9 +196,14 @@ public:
         if (f16_) return set_fields_f16(s, p, p_prev, vel2, cur);
         if (int rc = cuda(cudaMemcpyAsync(arena_ + h.off[cur], p, bytes, cudaMemcpyHostToDevice, st_)))
             return rc;
-        if (int rc = cuda(cudaMemcpyAsync(arena_ + h.off[cur ^ 1], p_prev, bytes,
-                                          cudaMemcpyHostToDevice, st_)))
+        if (p_prev == p) {
+            if (int rc = cuda(cudaMemcpyAsync(arena_ + h.off[cur ^ 1], arena_ + h.off[cur], bytes,
+                                              cudaMemcpyDeviceToDevice, st_)))
+                return rc;
+        } else if (int rc = cuda(cudaMemcpyAsync(arena_ + h.off[cur ^ 1], p_prev, bytes,
+                                                 cudaMemcpyHostToDevice, st_))) {
             return rc;
+        }
         if (int rc = cuda(cudaMemcpyAsync(arena_ + h.off[2], vel2, bytes, cudaMemcpyHostToDevice, st_)))
             return rc;
         return cuda(cudaStreamSynchronize(st_));
@@ -638,9 +643,22 @@ private:
     int set_fields_f16(int s, const float* p, const float* p_prev, const float* vel2, int cur) {
         const Shot& h = shots_[s];
         const int64_t n = h.g.size();
-        double m = 0.0;
-        for (int64_t i = 0; i < n; ++i)
-            m = std::max(m, std::max(std::fabs(double(p[i])), std::fabs(double(p_prev[i]))));
+        // the fields' largest magnitude, taken on the device (p last: it stays staged)
+        const size_t bytes = static_cast<size_t>(n) * 4;
+        unsigned* bits = reinterpret_cast<unsigned*>(stats_ + 3 * s);  // free between steps
+        unsigned w = 0;
+        if (p_prev == p) p_prev = nullptr;  // one field for both levels: copied once
+        if (int rc = cuda(cudaMemsetAsync(bits, 0, sizeof(w), st_))) return rc;
+        for (const float* f : {p_prev, p}) {
+            if (!f) continue;
+            if (int rc = cuda(cudaMemcpyAsync(staging_, f, bytes, cudaMemcpyHostToDevice, st_))) return rc;
+            if (int rc = cuda(launch_absmax(staging_, n, bits, st_))) return rc;
+        }
+        if (int rc = cuda(cudaMemcpyAsync(&w, bits, sizeof(w), cudaMemcpyDeviceToHost, st_))) return rc;
+        if (int rc = cuda(cudaStreamSynchronize(st_))) return rc;
+        float fm;
+        std::memcpy(&fm, &w, sizeof(fm));
+        const double m = fm;
         vel2_src_[s] = h.src >= 0 ? vel2[h.src] : 0.f;
         const std::vector<float> b = host_bound(s);
         const double bnd = b.empty() ? 0.0 : b[0];
@@ -651,23 +669,21 @@ private:
         const F16Scale s0{static_cast<float>(a0), 1.f};
         if (int rc = cuda(cudaMemcpyAsync(scale_ + s, &s0, sizeof(s0), cudaMemcpyHostToDevice, st_)))
             return rc;
-        const size_t bytes = static_cast<size_t>(n) * 4;
         const sb200_grid gg = to_grid(h.g);
-        struct Part {
-            const float* host;
-            int level;  // index into the shot's offsets: current, previous, K (2)
-        };
-        const Part parts[3] = {{p, cur}, {p_prev, cur ^ 1}, {vel2, 2}};
-        for (const Part& part : parts) {
-            if (int rc = cuda(cudaMemcpyAsync(staging_, part.host, bytes, cudaMemcpyHostToDevice, st_)))
+        auto level = [&](int l) { return reinterpret_cast<uint16_t*>(arena_ + h.off[l]); };
+        if (int rc = sb200_f16_pack(staging_, level(cur), n, float(a0), st_)) return rc;
+        if (!p_prev) {
+            if (int rc = cuda(cudaMemcpyAsync(level(cur ^ 1), level(cur), static_cast<size_t>(n) * 2,
+                                              cudaMemcpyDeviceToDevice, st_)))
                 return rc;
-            uint16_t* dst = reinterpret_cast<uint16_t*>(arena_ + h.off[part.level]);
-            const int rc = part.level == 2 ? sb200_k_field_bf16(staging_, dst, &gg, st_)
-                                           : sb200_f16_pack(staging_, dst, n, float(a0), st_);
-            if (rc) return rc;
-            // the staging buffer is reused by the next part
-            if (int r2 = cuda(cudaStreamSynchronize(st_))) return r2;
+        } else {
+            if (int rc = cuda(cudaMemcpyAsync(staging_, p_prev, bytes, cudaMemcpyHostToDevice, st_)))
+                return rc;
+            if (int rc = sb200_f16_pack(staging_, level(cur ^ 1), n, float(a0), st_)) return rc;
         }
+        if (int rc = cuda(cudaMemcpyAsync(staging_, vel2, bytes, cudaMemcpyHostToDevice, st_))) return rc;
+        if (int rc = sb200_k_field_bf16(staging_, level(2), &gg, st_)) return rc;
+        if (int rc = cuda(cudaStreamSynchronize(st_))) return rc;
         return upload_bound(s);
     }
 

@@ -194,6 +194,9 @@ cudaError_t launch_f16_unpack(const uint16_t* h, float* f, int64_t n, float scal
                               cudaStream_t st);
 cudaError_t launch_k_bf16(const float* vel2, uint16_t* k, int64_t n, float dt2_over_dx2,
                           cudaStream_t st);
+// *bits (a float's bit pattern, 0 to start with) raised to that of max |f[i]|; f 16-byte
+// aligned.
+cudaError_t launch_absmax(const float* f, int64_t n, unsigned* bits, cudaStream_t st);
 cudaError_t launch_f16_renorm(const double* stats3, F16Scale* scale, const float* bound,
                               const int* step, float bound_host, float target, cudaStream_t st);
 

@@ -39,7 +39,7 @@ __global__ void monitor_kernel(const double* stats3, int* flag, double limit) {
     if (!(stats3[2] == 0.0) || !(stats3[1] <= limit)) atomicExch(flag, 1);
 }
 
-constexpr int64_t kStageFloats = int64_t(1) << 24;  // host <-> device staging: 64 MB
+constexpr int64_t kStageFloats = int64_t(1) << 24;  // host <-> device staging: up to 64 MB
 
 class Run {
 public:
@@ -128,22 +128,27 @@ public:
         if (int rc = cuda(cudaMemsetAsync(monitor_dev_, 0, sizeof(int), st_))) return rc;
         if (!fp16_) {
             if (int rc = cuda(cudaMemcpyAsync(a_, p, n_ * 4, cudaMemcpyHostToDevice, st_))) return rc;
-            if (heat_) {  // both levels carry the caller's halo (never written)
-                if (int rc = cuda(cudaMemcpyAsync(b_, p, n_ * 4, cudaMemcpyHostToDevice, st_)))
+            // heat: both levels carry the caller's halo (never written)
+            if (heat_ || p_prev == p) {
+                if (int rc = cuda(cudaMemcpyAsync(b_, a_, n_ * 4, cudaMemcpyDeviceToDevice, st_)))
                     return rc;
-            } else {
-                if (int rc = cuda(cudaMemcpyAsync(b_, p_prev, n_ * 4, cudaMemcpyHostToDevice, st_)))
-                    return rc;
+            } else if (int rc = cuda(cudaMemcpyAsync(b_, p_prev, n_ * 4, cudaMemcpyHostToDevice, st_))) {
+                return rc;
+            }
+            if (!heat_) {
                 if (int rc = cuda(cudaMemcpyAsync(vel2_, vel2, n_ * 4, cudaMemcpyHostToDevice, st_)))
                     return rc;
                 vel2_host_src_ = c_.src_index >= 0 ? vel2[c_.src_index] : 0.f;
             }
             return cuda(cudaStreamSynchronize(st_));
         }
-        // FP16: initial scale from the host fields and the first window's source.
+        // FP16: initial scale from the fields' largest magnitude, taken on the device as
+        // their chunks pass through the staging buffer, and the first window's source.
+        // Fields of one chunk stay staged (one half each); longer ones are copied again
+        // to be packed.
+        const bool same = p_prev == p, held = stage_holds();
         double m = 0.0;
-        for (int64_t i = 0; i < n_; ++i)
-            m = std::max(m, std::max(std::fabs(double(p[i])), std::fabs(double(p_prev[i]))));
+        if (int rc = stage_max(p, same ? nullptr : p_prev, &m)) return rc;
         vel2_host_src_ = c_.src_index >= 0 ? vel2[c_.src_index] : 0.f;
         rebuild_bound();
         const double bnd = bound_host_.empty() ? 0.0 : bound_host_[0];
@@ -155,8 +160,20 @@ public:
         // on the run's stream: steps still queued there read the scale
         if (int rc = cuda(cudaMemcpyAsync(scale_dev_, &s0, sizeof(s0), cudaMemcpyHostToDevice, st_)))
             return rc;
-        if (int rc = stage_in(p, a_, float(a0), false)) return rc;
-        if (int rc = stage_in(p_prev, b_, float(a0), false)) return rc;
+        if (held) {
+            if (int rc = sb200_f16_pack(stage_, static_cast<uint16_t*>(a_), n_, float(a0), st_))
+                return rc;
+            if (!same)
+                if (int rc = sb200_f16_pack(stage_ + stage_half(), static_cast<uint16_t*>(b_), n_,
+                                            float(a0), st_))
+                    return rc;
+        } else {
+            if (int rc = stage_in(p, a_, float(a0), false)) return rc;
+            if (!same)
+                if (int rc = stage_in(p_prev, b_, float(a0), false)) return rc;
+        }
+        if (same)
+            if (int rc = cuda(cudaMemcpyAsync(b_, a_, n_ * 2, cudaMemcpyDeviceToDevice, st_))) return rc;
         if (int rc = stage_in(vel2, k_, 1.f, true)) return rc;
         return cuda(cudaStreamSynchronize(st_));
     }
@@ -296,9 +313,40 @@ private:
     }
     int alloc(void** p, size_t bytes) { return cuda(cudaMalloc(p, bytes)); }
 
+    // Staging: one chunk of kStageFloats values, or two whole fields where they are no
+    // longer than a chunk.
+    bool stage_holds() const { return n_ <= kStageFloats; }
+    int64_t stage_half() const { return stage_holds() ? (n_ + 63) / 64 * 64 : 0; }
     int ensure_stage() {
         if (stage_) return SB200_OK;
-        return alloc(reinterpret_cast<void**>(&stage_), size_t(kStageFloats) * 4);
+        return alloc(reinterpret_cast<void**>(&stage_),
+                     size_t(stage_holds() ? 2 * stage_half() : kStageFloats) * 4);
+    }
+
+    // *m = max |value| of the host fields p and q (q may be NULL), chunk by chunk through
+    // the staging buffer; where it holds both fields they are left there, q in the second
+    // half.
+    int stage_max(const float* p, const float* q, double* m) {
+        if (int rc = ensure_stage()) return rc;
+        unsigned* bits = reinterpret_cast<unsigned*>(stats_dev_);  // free between steps
+        if (int rc = cuda(cudaMemsetAsync(bits, 0, sizeof(unsigned), st_))) return rc;
+        for (int64_t off = 0; off < n_; off += kStageFloats) {
+            const int64_t c = std::min(kStageFloats, n_ - off);
+            for (int h = 0; h < (q ? 2 : 1); ++h) {
+                float* d = stage_ + h * stage_half();
+                if (int rc = cuda(cudaMemcpyAsync(d, (h ? q : p) + off, c * 4,
+                                                  cudaMemcpyHostToDevice, st_)))
+                    return rc;
+                if (int rc = cuda(launch_absmax(d, c, bits, st_))) return rc;
+            }
+        }
+        unsigned w = 0;
+        if (int rc = cuda(cudaMemcpyAsync(&w, bits, sizeof(w), cudaMemcpyDeviceToHost, st_))) return rc;
+        if (int rc = cuda(cudaStreamSynchronize(st_))) return rc;
+        float f;
+        std::memcpy(&f, &w, sizeof(f));
+        *m = f;
+        return SB200_OK;
     }
 
     // Host FP32 -> device FP16 (scaled) or BF16 K (vel2 -> vel2 dt^2/dx^2) by chunks.

@@ -170,3 +170,24 @@ def test_caller_wavelet_is_kept_and_bounds_the_run():
     # first step from rest: p = dt^2 vel2 w[0] at the source
     k = np.float32(np.float32(1e-3) * np.float32(1e-3)) * np.float32(2000.0 ** 2)
     assert tr[0] == np.float32(k * w[0])
+
+
+# the largest magnitude in p or p_prev, at the first, a middle and the last cell; cell
+# counts that are and are not a multiple of 4 vectors; fields longer than the staging
+@pytest.mark.parametrize("shape, at, in_prev", [((9, 9, 16), 0, False), ((9, 11, 16), -1, True),
+                                                ((33, 35, 40), 12345, True), ((64, 64, 64), -1, False),
+                                                ((257, 256, 256), -1, True)])
+def test_fp16_initial_scale_from_the_fields(torch_cuda, shape, at, in_prev):
+    rng = np.random.default_rng(7)
+    p, q = (rng.uniform(-1, 1, shape).astype(np.float32) for _ in range(2))
+    (q if in_prev else p).reshape(-1)[at] = -37.5
+    p.reshape(-1)[5] = np.nan  # passed over
+    vel2 = np.full(shape, 2.25e6, np.float32)
+    nz, ny, nx = shape
+    a = 2.0 ** np.floor(np.log2(4096.0 / 37.5))
+    with sb.Run(sb.Grid(nx, ny, nz, 10, 10, 10, 1e-3), precision=sb.PRECISION_F16) as r:
+        for prev in (q, None) if not in_prev else (q,):
+            r.set_fields(p, prev, vel2)
+            with np.errstate(invalid="ignore"):
+                want = (p * np.float32(a)).astype(np.float16).astype(np.float32) / np.float32(a)
+            assert np.array_equal(r.field(), want, equal_nan=True)
