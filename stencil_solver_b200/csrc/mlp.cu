@@ -64,9 +64,8 @@ struct NetFrag {
     float b3;
 };
 
-__device__ __forceinline__ void load_net(NetFrag& n, const float* __restrict__ prm,
-                                         const uint32_t* __restrict__ w1b,
-                                         const uint32_t* __restrict__ w2b) {
+__device__ __forceinline__ void load_net(NetFrag& n, const float* prm, const uint32_t* w1b,
+                                         const uint32_t* w2b) {
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
@@ -136,7 +135,7 @@ __device__ __forceinline__ void forward_tile(const NetFrag& n, const uint32_t (&
 
 // A fragments of rows [r0, r0+16) of a row-major BF16 feature matrix (32 per
 // row); rows at or beyond n read as zero.
-__device__ __forceinline__ void load_x(uint32_t (&x)[2][4], const uint32_t* __restrict__ X,
+__device__ __forceinline__ void load_x(uint32_t (&x)[2][4], const uint32_t* X,
                                        int64_t r0, int64_t n) {
     const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     const int64_t ra = r0 + g, rb = r0 + g + 8;
@@ -186,16 +185,39 @@ __device__ __forceinline__ uint32_t ld_pair(const uint16_t* p) {
     return *reinterpret_cast<const uint32_t*>(p);
 }
 
+// Per-warp gradients on their way to the block's sum: dW1 and dW2 rows (W1's first),
+// padded to 40 words so that the fragments' pairs hit distinct banks, and the vectors
+// [db1 | db2 | dw3 | db3 | loss].
+constexpr int GP = 40, GVEC = 3 * H + 2;
+struct alignas(16) WarpG {
+    float w[2 * H][GP];
+    float v[GVEC];
+};
+static_assert(sizeof(WarpG) % 16 == 0 && GP % 4 == 0 && OFF_W2 % 4 == 0, "16-byte rows");
+
+__device__ __forceinline__ void red_add4(float* p, float4 v) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y),
+                 "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+
 // Gradient of sum over rows of (y - t)^2 * inv_n (the caller passes 1 / n_total),
-// accumulated into grad[NPARAM] (and the loss into grad[NPARAM]).
+// accumulated into grad[NPARAM] (and the loss into grad[NPARAM]).  Bound by latency: a
+// mini-batch of 8192 rows is 4.5 kB of operands and 100 Mflop, so it is spread over as
+// many blocks as it has 64-row rounds (128 of them; 32 of 256 rows before), and the
+// warps' sums meet through plain shared-memory stores and one vector reduction per
+// four parameters (before: 2146 shared float atomics per warp, compare-and-swap loops).
+// vec: grad is 16-byte aligned.
 __global__ void __launch_bounds__(32 * kWarps)
-    mlp_grad_kernel(const float* __restrict__ prm, const uint32_t* __restrict__ w1b,
-                    const uint32_t* __restrict__ w2b, const uint32_t* __restrict__ w2tb,
-                    const uint32_t* __restrict__ X, const float* __restrict__ tgt, int64_t n,
-                    float inv_n, float* __restrict__ grad) {
-    __shared__ WarpT wt[kWarps];
-    __shared__ float red[NSLOT];
-    for (int i = threadIdx.x; i < NSLOT; i += blockDim.x) red[i] = 0.f;
+    mlp_grad_kernel(const float* prm, const uint32_t* w1b, const uint32_t* w2b,
+                    const uint32_t* w2tb, const uint32_t* X, const float* tgt, int64_t n,
+                    float inv_n, float* grad, bool vec) {
+    __shared__ union Scratch {
+        WarpT t[kWarps];
+        WarpG g[kWarps];
+    } sh;
+    WarpT(&wt)[kWarps] = sh.t;
+    launch_order();
 
     NetFrag net;
     load_net(net, prm, w1b, w2b);
@@ -328,50 +350,106 @@ __global__ void __launch_bounds__(32 * kWarps)
         __syncwarp();  // the transposes are rewritten by the next tile
     }
 
-    // Block reduction in shared memory, then one global add per parameter.
-    __syncthreads();
+    // The vectors' sums over the 8 row groups of a warp, then the block's sums over its
+    // warps, and one global reduction per four weights or per vector entry.
+    __syncthreads();  // the transposes are dead
+    WarpG& G = sh.g[wi];
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int t = 0; t < 4; ++t)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int o = 16 * m + g + 8 * (e >> 1), i = 8 * t + 2 * q + (e & 1);
-                atomicAdd(&red[OFF_W1 + o * F + i], gw1[m][t][e]);
-                atomicAdd(&red[OFF_W2 + o * H + i], gw2[m][t][e]);
+            for (int e = 0; e < 4; e += 2) {
+                const int o = 16 * m + g + 4 * e, i = 8 * t + 2 * q;
+                *reinterpret_cast<float2*>(&G.w[o][i]) = make_float2(gw1[m][t][e], gw1[m][t][e + 1]);
+                *reinterpret_cast<float2*>(&G.w[H + o][i]) =
+                    make_float2(gw2[m][t][e], gw2[m][t][e + 1]);
             }
+    auto over_rows = [](float v) {
+        v += __shfl_xor_sync(0xffffffffu, v, 4);
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+        return v + __shfl_xor_sync(0xffffffffu, v, 16);
+    };
 #pragma unroll
     for (int t = 0; t < 4; ++t)
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-            const int col = 8 * t + 2 * q + c;
-            atomicAdd(&red[OFF_B1 + col], gb1[t][c]);
-            atomicAdd(&red[OFF_B2 + col], gb2[t][c]);
-            atomicAdd(&red[OFF_W3 + col], gw3[t][c]);
+            const float v1 = over_rows(gb1[t][c]), v2 = over_rows(gb2[t][c]),
+                        v3 = over_rows(gw3[t][c]);
+            if (g == 0) {
+                const int col = 8 * t + 2 * q + c;
+                G.v[col] = v1;
+                G.v[H + col] = v2;
+                G.v[2 * H + col] = v3;
+            }
         }
-    if (q == 0) {
-        atomicAdd(&red[OFF_B3], gb3);
-        atomicAdd(&red[NPARAM], loss);
+    gb3 = over_rows(gb3);
+    loss = over_rows(loss);
+    if (lane == 0) {  // q = 0 lanes hold these two
+        G.v[3 * H] = gb3;
+        G.v[3 * H + 1] = loss;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < NSLOT; i += blockDim.x)
-        if (red[i] != 0.f) atomicAdd(&grad[i], red[i]);
+    for (int k = threadIdx.x; k < 2 * H * (F / 4); k += blockDim.x) {
+        const int o = k / (F / 4), i = 4 * (k % (F / 4));
+        float4 v = *reinterpret_cast<const float4*>(&sh.g[0].w[o][i]);
+#pragma unroll
+        for (int w = 1; w < kWarps; ++w) {
+            const float4 x = *reinterpret_cast<const float4*>(&sh.g[w].w[o][i]);
+            v = make_float4(v.x + x.x, v.y + x.y, v.z + x.z, v.w + x.w);
+        }
+        float* dst = grad + (o < H ? OFF_W1 + o * F : OFF_W2 + (o - H) * H) + i;
+        if (vec) {
+            red_add4(dst, v);
+        } else {
+            atomicAdd(dst, v.x);
+            atomicAdd(dst + 1, v.y);
+            atomicAdd(dst + 2, v.z);
+            atomicAdd(dst + 3, v.w);
+        }
+    }
+    for (int k = threadIdx.x; k < GVEC; k += blockDim.x) {
+        float v = sh.g[0].v[k];
+#pragma unroll
+        for (int w = 1; w < kWarps; ++w) v += sh.g[w].v[k];
+        const int at = k < H ? OFF_B1 + k
+                     : k < 2 * H ? OFF_B2 + k - H
+                     : k < 3 * H ? OFF_W3 + k - 2 * H
+                     : k == 3 * H ? OFF_B3 : NPARAM;
+        atomicAdd(&grad[at], v);
+    }
 }
 
-// Adam on the FP32 masters (one thread per parameter; input columns 26..31 of
-// W1 never move).
-__global__ void mlp_adam_kernel(float* __restrict__ prm, float* __restrict__ m1,
-                                float* __restrict__ m2, const float* __restrict__ grad, float lr,
-                                float b1, float b2, float eps, float c1, float c2) {
+// Adam on the FP32 masters (one thread per parameter; input columns 26..31 of W1 never
+// move), with the BF16 copies the mma kernels read; hands out the loss and leaves the
+// gradient zeroed for the next step.
+__global__ void __launch_bounds__(128)
+    mlp_adam_kernel(float* prm, float* m1, float* m2, float* grad, float lr, float b1, float b2,
+                    float eps, float c1, float c2, uint16_t* w1b, uint16_t* w2b, uint16_t* w2tb,
+                    float* loss) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NPARAM) return;
-    if (i < OFF_B1 && (i % F) >= NIN) return;
+    launch_order();
+    if (i >= NSLOT) return;
     const float gr = grad[i];
+    grad[i] = 0.f;
+    if (i == NPARAM) {
+        if (loss) *loss = gr;
+        return;
+    }
+    if (i < OFF_B1 && (i % F) >= NIN) return;
     const float a = b1 * m1[i] + (1.f - b1) * gr;
     const float v = b2 * m2[i] + (1.f - b2) * gr * gr;
     m1[i] = a;
     m2[i] = v;
-    prm[i] -= lr * (a / c1) / (sqrtf(v / c2) + eps);
+    const float p = prm[i] - lr * (a / c1) / (sqrtf(v / c2) + eps);
+    prm[i] = p;
+    if (i < OFF_B1) {
+        w1b[i] = bf16_bits(p);
+    } else if (i >= OFF_W2 && i < OFF_B2) {
+        const int k = i - OFF_W2;
+        w2b[k] = bf16_bits(p);
+        w2tb[(k % H) * H + k / H] = bf16_bits(p);
+    }
 }
 
 // BF16 copies of W1, W2 and W2^T read by the mma kernels.
@@ -697,7 +775,8 @@ struct Mlp {
     float* prm = nullptr;  // NPARAM FP32 masters
     float* m1 = nullptr;
     float* m2 = nullptr;
-    float* grad = nullptr;  // NSLOT (gradients + loss)
+    float* grad = nullptr;  // NSLOT (gradients + loss), zero between training steps
+    bool grad_zero = false;
     uint16_t* w1b = nullptr;
     uint16_t* w2b = nullptr;
     uint16_t* w2tb = nullptr;
@@ -728,6 +807,22 @@ void init_params(std::vector<float>& w, uint64_t seed) {
         for (int i = 0; i < H; ++i)
             w[OFF_W2 + o * H + i] = static_cast<float>(nd(rng) * std::sqrt(2.0 / H));
     for (int i = 0; i < H; ++i) w[OFF_W3 + i] = static_cast<float>(nd(rng) * 0.1 / std::sqrt(H));
+}
+
+// Gradient of n rows added into grad: one block per 64 rows, at most two per SM (what its
+// registers let run at once).
+int launch_grad(const Mlp& m, const uint16_t* X, const float* t, int64_t n, float* grad,
+                cudaStream_t st, const char* where) {
+    const int64_t rounds = (n + 16 * kWarps - 1) / (16 * kWarps);
+    const unsigned blocks = static_cast<unsigned>(std::min<int64_t>(rounds, int64_t(m.sms) * 2));
+    return cuda_err(launch_after(mlp_grad_kernel, blocks, 32 * kWarps, 0, st, m.prm,
+                                 reinterpret_cast<const uint32_t*>(m.w1b),
+                                 reinterpret_cast<const uint32_t*>(m.w2b),
+                                 reinterpret_cast<const uint32_t*>(m.w2tb),
+                                 reinterpret_cast<const uint32_t*>(X), t, n,
+                                 1.f / static_cast<float>(n), grad,
+                                 (reinterpret_cast<uintptr_t>(grad) & 15u) == 0),
+                    where);
 }
 
 int grid_blocks(const Mlp& m, int64_t work_units_per_block, int64_t units) {
@@ -850,35 +945,30 @@ int sb200_mlp_gradients(void* h, const uint16_t* X, const float* t, int64_t n, f
         return set_error(SB200_ERR_INVALID, "sb200_mlp_gradients: bad arguments");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int rc = cuda_err(cudaMemsetAsync(grad, 0, NSLOT * 4, st), "sb200_mlp_gradients");
-    if (rc) return rc;
-    const int blocks = grid_blocks(*m, 16 * kWarps * 4, n);
-    mlp_grad_kernel<<<blocks, 32 * kWarps, 0, st>>>(
-        m->prm, reinterpret_cast<const uint32_t*>(m->w1b), reinterpret_cast<const uint32_t*>(m->w2b),
-        reinterpret_cast<const uint32_t*>(m->w2tb), reinterpret_cast<const uint32_t*>(X), t, n,
-        1.f / static_cast<float>(n), grad);
-    return cuda_err(cudaGetLastError(), "sb200_mlp_gradients");
+    return rc ? rc : launch_grad(*m, X, t, n, grad, st, "sb200_mlp_gradients");
 }
 
 int sb200_mlp_train_step(void* h, const uint16_t* X, const float* t, int64_t n, float lr,
                          float* loss, void* stream) {
+    const char* where = "sb200_mlp_train_step";
     Mlp* m = static_cast<Mlp*>(h);
-    if (!m) return set_error(SB200_ERR_INVALID, "sb200_mlp_train_step: NULL handle");
-    if (!(lr > 0.f)) return set_error(SB200_ERR_INVALID, "sb200_mlp_train_step: lr must be positive");
-    if (int rc = sb200_mlp_gradients(h, X, t, n, m->grad, stream)) return rc;
+    if (!m) return set_error(SB200_ERR_INVALID, std::string(where) + ": NULL handle");
+    if (!(lr > 0.f)) return set_error(SB200_ERR_INVALID, std::string(where) + ": lr must be positive");
+    if (!X || !t || n <= 0) return set_error(SB200_ERR_INVALID, std::string(where) + ": bad arguments");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (!m->grad_zero)
+        if (int rc = cuda_err(cudaMemsetAsync(m->grad, 0, NSLOT * 4, st), where)) return rc;
+    m->grad_zero = false;  // until the update that zeroes it again is on its way
+    if (int rc = launch_grad(*m, X, t, n, m->grad, st, where)) return rc;
     m->host_valid = false;
     m->adam_t += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, float(m->adam_t)), c2 = 1.f - std::pow(b2, float(m->adam_t));
-    mlp_adam_kernel<<<(NPARAM + 255) / 256, 256, 0, st>>>(m->prm, m->m1, m->m2, m->grad, lr, b1, b2,
-                                                          1e-8f, c1, c2);
-    int rc = cuda_err(cudaGetLastError(), "sb200_mlp_train_step");
-    if (rc) return rc;
-    mlp_bf16_kernel<<<(H * F + 255) / 256, 256, 0, st>>>(m->prm, m->w1b, m->w2b, m->w2tb);
-    rc = cuda_err(cudaGetLastError(), "sb200_mlp_train_step");
-    if (!rc && loss)
-        rc = cuda_err(cudaMemcpyAsync(loss, m->grad + NPARAM, 4, cudaMemcpyDeviceToDevice, st),
-                      "sb200_mlp_train_step");
+    const int rc = cuda_err(launch_after(mlp_adam_kernel, (NSLOT + 127) / 128, 128, 0, st, m->prm, m->m1,
+                                         m->m2, m->grad, lr, b1, b2, 1e-8f, c1, c2, m->w1b, m->w2b,
+                                         m->w2tb, loss),
+                            where);
+    m->grad_zero = !rc;
     return rc;
 }
 

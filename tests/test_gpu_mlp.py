@@ -106,6 +106,36 @@ def test_gradients_match_oracle(torch_cuda):
         assert d <= 5e-3, (name, d)
 
 
+BLOCKS = {"W1": slice(0, 1024), "b1": slice(1024, 1056), "W2": slice(1056, 2080),
+          "b2": slice(2080, 2112), "w3": slice(2112, 2144), "b3": slice(2144, 2145)}
+
+
+# one row, a 16-row tile and a 64-row round with their neighbours, and one row more than a
+# round on every block; the gradient in a buffer that takes vector reductions and in one
+# that does not.  Tolerances: test_gradients_match_oracle's.
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 63, 64, 65, 2 * 148 * 64 + 1])
+def test_gradients_and_updates_at_block_edges(torch_cuda, n, offset):
+    torch = torch_cuda
+    w, X, t = net_and_rows(6, n)
+    Xd, td = dev(torch, X.view(np.int16)), dev(torch, t)
+    room = torch.full((sb.MLP_NPARAM + 1 + offset,), 7.0, device="cuda")
+    loss = torch.zeros(1, device="cuda")
+    with sb.Mlp() as m:
+        m.set_params(w)
+        for _ in range(3):  # the updates leave the copies and the gradient buffer in order
+            w = m.params()
+            m.gradients(Xd, td, room[offset:])
+            got = room[offset:].cpu().numpy().astype(np.float64)
+            want, ref = oracle.mlp_grad(w, X, t, round_bf16=True)
+            m.train_step(Xd, td, 1e-3, loss)
+            assert abs(got[-1] - want) <= 1e-4 * want and abs(float(loss) - want) <= 1e-4 * want
+            for name, sl in BLOCKS.items():
+                d = np.linalg.norm(got[sl] - ref[sl]) / max(np.linalg.norm(ref[sl]), 1e-12)
+                assert d <= 5e-3, (name, d)
+        assert np.all(np.abs(m.params() - w) <= 1.5e-3) and np.any(m.params() != w)
+
+
 def test_training_lowers_the_loss(torch_cuda):
     torch = torch_cuda
     rng = np.random.default_rng(5)
