@@ -103,58 +103,123 @@ int sm_count() {
     return n;
 }
 
-// Untuned default tile of a kind: the tuner's usual pick on large grids
-// (1024^3 acoustic: t64x32_r2_s8_a3; 512^3 heat: t64x16_r2_s8; FP16 1024^3:
-// h64x16_s8_a4), found by name so the tables can be reordered.
-int default_variant(int kind) {
-    const char* want = kind == SB200_KIND_WAVE_F32   ? "t64x32_r2_s8_a3"
-                       : kind == SB200_KIND_HEAT_F32 ? "t64x16_r2_s8"
-                       : kind == SB200_KIND_WAVE_F16 ? "h64x16_s8_a4"
-                                                     : "l32x32_r1_s8";
-    const int n = variant_count(kind);
-    for (int v = 0; v < n; ++v) {
-        const char* name = variant_name(kind, v);
-        if (name && std::strcmp(name, want) == 0) return v;
+// ── untuned choice: a cost model over tiles and z splits ──────────────────────
+
+// Cost of sweeping an interior of inz planes in chunks of zlen with `tiles` columns, on
+// SMs that hold `resident` CTAs each, in planes of a fully occupied SM: whole waves of
+// zlen + start planes (start: what filling a CTA's rings costs), and a last wave in which
+// the busiest SM holds k CTAs: they take (k / resident)^0.62 of a full wave's time (fewer
+// CTAs hide less latency).
+double split_cost(int64_t tiles, int inz, int zlen, int resident, int sms, double start) {
+    const int64_t ctas = tiles * ((inz + zlen - 1) / zlen);
+    const int64_t slots = int64_t(sms) * resident;
+    const int64_t rest = ctas % slots;
+    double waves = double(ctas / slots);
+    if (rest) waves += std::pow(double((rest + sms - 1) / sms) / resident, 0.62);
+    return waves * (zlen + start);
+}
+
+// (cost, z chunks) of every distinct chunk length, cheapest first.
+std::vector<std::pair<double, int>> rank_splits(int64_t tiles, int inz, int resident, double start) {
+    const int sms = std::max(1, sm_count());
+    resident = std::max(1, resident);
+    std::vector<std::pair<double, int>> out;
+    int last = 0;
+    for (int zc = 1; zc <= std::min(inz, 512); ++zc) {
+        const int zlen = (inz + zc - 1) / zc;
+        if (zlen == last) continue;
+        last = zlen;
+        out.emplace_back(split_cost(tiles, inz, zlen, resident, sms, start), (inz + zlen - 1) / zlen);
     }
-    return 0;
+    std::stable_sort(out.begin(), out.end());
+    if (out.empty()) out.emplace_back(1.0, 1);
+    return out;
+}
+
+// Tiles an untuned launch chooses from, with the cost of a point relative to the table's
+// other tiles where the step's fields fit L2 (126 MB) and where they do not (0: not
+// taken).  Model and weights were fitted to 22 grids from 64^3 to 1024^3 (cubes, thin and
+// flat boxes; graph replays), every tile at 11 to 23 splits: the picks are on average 1.0
+// % (FP32), 2.3 % (heat) and 1.1 % (FP16) from the best of them, at worst 6 to 8 %.
+// What the tables say:
+//   * acoustic, beyond L2: 16 warps per SM and wide rows.  One 64 x 32 CTA of 8 warps per
+//     SM was the default; it follows the SM clock, and full-range data holds that at 1.55
+//     GHz under the 1000 W cap.  1024^3, sustained: 2930 us (t64x32_r2_s8_a3), 2830
+//     (t64x32_r2_s6_a2, two CTAs), 2790 (t128x16_r2_s6_a2), 2670 (t128x32_r2_s7_a2, 1.33
+//     staged words a point instead of 1.41);
+//   * small grids: as many short CTAs as there are slots (acoustic 64^3 4.9 -> 3.2 us,
+//     320^3 96 -> 84 us; heat 160^3 10.5 -> 8.1 us; FP16 96^3 6.0 -> 5.2 us).
+struct Candidate {
+    const char* name;
+    double in_l2, beyond;
+};
+struct Family {
+    double start;
+    int step_bytes;  // per cell: the fields a step keeps in use
+    Candidate tiles[4];
+};
+const Family kFamilies[] = {
+    // SB200_KIND_WAVE_F32
+    {2.1, 12,
+     {{"t32x32_r2_s8_a4", 1.38, 0}, {"t64x32_r2_s6_a2", 1.04, 1.074}, {"t128x16_r2_s6_a2", 1.0, 0},
+      {"t128x32_r2_s7_a2", 0, 1.0}}},
+    // SB200_KIND_HEAT_F32
+    {6.7, 8, {{"t32x32_r2_s8", 1.05, 0}, {"t64x16_r2_s8", 1.0, 1.114}, {"t128x16_r2_s8", 0, 1.0}}},
+    // SB200_KIND_WAVE_F16
+    {4.3, 6, {{"h64x16_s8_a4", 0, 1.02}, {"h64x32_s8_a2", 1.1, 0}, {"h128x16_s8_a2", 1.0, 1.0}}},
+};
+constexpr double kL2Bytes = 126e6;
+
+int variant_by_name(int kind, const char* name) {
+    for (int v = 0; v < variant_count(kind); ++v)
+        if (std::strcmp(variant_name(kind, v), name) == 0) return v;
+    return -1;
+}
+
+int64_t column_tiles(int kind, int v, const GridDesc& g) {
+    return kind == SB200_KIND_WAVE2_F32  ? leap2_ctas(v, g, 1)
+           : kind == SB200_KIND_WAVE_F16 ? pencil_f16_ctas(v, g, 1)
+                                         : pencil_f32_ctas(kind == SB200_KIND_HEAT_F32, v, g, 1);
+}
+
+int resident_ctas(int kind, int v) {
+    return kind == SB200_KIND_WAVE2_F32  ? leap2_resident(v)
+           : kind == SB200_KIND_WAVE_F16 ? pencil_f16_resident(v)
+                                         : pencil_f32_resident(kind == SB200_KIND_HEAT_F32, v);
+}
+
+PencilConfig cheapest(int kind, const GridDesc& g) {
+    const Family& f = kFamilies[kind];
+    const bool beyond = double(g.size()) * f.step_bytes > kL2Bytes;
+    PencilConfig best;
+    double cost = 0;
+    for (const Candidate& c : f.tiles) {
+        const double weight = beyond ? c.beyond : c.in_l2;
+        const int v = c.name && weight > 0 ? variant_by_name(kind, c.name) : -1;
+        if (v < 0) continue;
+        const PencilBoxes b = kind == SB200_KIND_WAVE_F16
+                                  ? pencil_f16_boxes(v)
+                                  : pencil_f32_boxes(kind == SB200_KIND_HEAT_F32, v);
+        const int resident = resident_ctas(kind, v);
+        const auto s =
+            rank_splits(column_tiles(kind, v, g), static_cast<int>(g.nz - 8), resident, f.start)
+                .front();
+        const double t = s.first * weight * b.points * resident;
+        if (cost == 0 || t < cost) {
+            cost = t;
+            best.variant = v;
+            best.zchunks = s.second;
+        }
+    }
+    return best;
 }
 
 // Tile of the reference-order steps: 59 separately rounded operations a point leave them
 // short of warps rather than of bytes, and the one-row tile runs 4 CTAs per SM (384^3
 // acoustic: 162 us against 170-175 for the two-row tiles).
 int exact_variant(bool heat) {
-    const char* want = heat ? "t32x16_r1_s8" : "t32x16_r1_s8_a4";
-    const int kind = heat ? SB200_KIND_HEAT_F32 : SB200_KIND_WAVE_F32;
-    for (int v = 0; v < variant_count(kind); ++v)
-        if (std::strcmp(variant_name(kind, v), want) == 0) return v;
-    return 0;
-}
-
-// z splits of an interior of inz planes ranked by how well their CTA count fills whole
-// waves.  A wave is SMs x resident CTAs; a split whose CTA count leaves the last wave
-// mostly empty wastes that fraction of the machine, and every extra split re-reads
-// hplanes halo planes of p (the share pshare of the traffic).
-template <class Ctas>
-std::vector<int> rank_splits(int inz, int resident, int hplanes, double pshare, Ctas ctas_of,
-                             int max_n) {
-    const double slots = double(sm_count()) * std::max(1, resident);
-    std::vector<std::pair<double, int>> scored;
-    for (int zc = 1; zc <= 16 && zc <= inz; ++zc) {
-        const double ctas = double(ctas_of(zc));
-        const double waves = std::ceil(ctas / slots);
-        const double fill = ctas / (waves * slots);
-        const int zlen = (inz + zc - 1) / zc;
-        const double halo = double(zlen) / double(zlen + hplanes) * pshare + (1.0 - pshare);
-        scored.emplace_back(-(fill * halo), zc);
-    }
-    std::stable_sort(scored.begin(), scored.end());
-    std::vector<int> out;
-    for (const auto& s : scored) {
-        if (static_cast<int>(out.size()) >= max_n) break;
-        out.push_back(s.second);
-    }
-    if (out.empty()) out.push_back(1);
-    return out;
+    return heat ? variant_by_name(SB200_KIND_HEAT_F32, "t32x16_r1_s8")
+                : variant_by_name(SB200_KIND_WAVE_F32, "t32x16_r1_s8_a4");
 }
 
 // Family of steps with a choice of their own beyond the public kinds: the reference
@@ -189,23 +254,23 @@ PencilConfig choose(int kind, const GridDesc& g) {
     auto it = memo.find(key);
     if (it != memo.end()) return it->second;
     const int inz = static_cast<int>(g.nz - 8);
+    const double start = kFamilies[SB200_KIND_WAVE_F32].start;
     if (kind >= kRaggedWave) {
-        // a chunk's start costs about three planes (401 x 357 x 301, acoustic: 2, 4, 6, 8
-        // and 12 chunks 150, 153, 156, 157 and 159 us)
-        c.zchunks = rank_splits(
-                        inz, ragged_resident(kind == kRaggedHeat, g), 3, 1.0,
-                        [&](int zc) { return ragged_ctas(g, zc); }, 1)
-                        .front();
+        c.zchunks = rank_splits(ragged_ctas(g, 1), inz, ragged_resident(kind == kRaggedHeat, g), start)
+                        .front()
+                        .second;
     } else if (kind >= kExactWave) {
         const bool heat = kind == kExactHeat;
         c.variant = exact_variant(heat);
-        c.zchunks = rank_splits(
-                        inz, pencil_f32_resident(heat, c.variant, true), 8, heat ? 0.5 : 0.25,
-                        [&](int zc) { return pencil_f32_ctas(heat, c.variant, g, zc); }, 1)
-                        .front();
-    } else {
-        c.variant = default_variant(kind);
+        c.zchunks = rank_splits(pencil_f32_ctas(heat, c.variant, g, 1), inz,
+                                pencil_f32_resident(heat, c.variant, true), start)
+                        .front()
+                        .second;
+    } else if (kind == SB200_KIND_WAVE2_F32) {
+        c.variant = std::max(0, variant_by_name(kind, "l32x32_r1_s8"));
         c.zchunks = zchunk_ranking(kind, c.variant, g, 1).front();
+    } else {
+        c = cheapest(kind, g);
     }
     memo[key] = c;
     return c;
@@ -424,19 +489,14 @@ int set_error(int code, const std::string& msg) { return fail(code, msg); }
 int* device_error_word() { return device_error_ptr(); }
 
 std::vector<int> zchunk_ranking(int kind, int v, const GridDesc& g, int max_n) {
-    const bool f16 = kind == SB200_KIND_WAVE_F16;
-    const bool heat = kind == SB200_KIND_HEAT_F32;
-    const bool two = kind == SB200_KIND_WAVE2_F32;
-    const int resident = two ? leap2_resident(v)
-                             : (f16 ? pencil_f16_resident(v) : pencil_f32_resident(heat, v));
-    // two steps: p is 4 of the pair's 20 B and a chunk reads 16 halo planes
-    return rank_splits(
-        static_cast<int>(g.nz - 8), resident, two ? 16 : 8, two ? 0.2 : (heat ? 0.5 : 0.25),
-        [&](int zc) {
-            return two ? leap2_ctas(v, g, zc)
-                       : (f16 ? pencil_f16_ctas(v, g, zc) : pencil_f32_ctas(heat, v, g, zc));
-        },
-        max_n);
+    // (two steps per sweep: a chunk reads 16 halo planes)
+    const auto ranked =
+        rank_splits(column_tiles(kind, v, g), static_cast<int>(g.nz - 8), resident_ctas(kind, v),
+                    kind == SB200_KIND_WAVE2_F32 ? 6.0 : kFamilies[kind].start);
+    std::vector<int> out;
+    for (const auto& s : ranked)
+        if (static_cast<int>(out.size()) < max_n) out.push_back(s.second);
+    return out;
 }
 
 }  // namespace sb200

@@ -61,6 +61,7 @@ struct PencilBoxes {
     int halo_x = 0, halo_y = 0;  // p / u box: tile + 4-cell halo on each side
     int tile_x = 0, tile_y = 0;  // p_prev / vel2 box
     bool aux_tma = false;        // whether p_prev / vel2 go through TMA
+    int points = 0;              // points of the tile per plane
 };
 
 // FP32 pencil kernels.  Preconditions (checked by the caller): nx % 4 == 0,
@@ -161,9 +162,8 @@ void pencil_f16_prepare();
 // Number of CTAs a launch uses (for occupancy/wave reasoning in the tuner).
 int64_t pencil_f32_ctas(bool heat, int v, const GridDesc& g, int zchunks);
 
-// z splits of variant v on grid g ranked by how well their CTA count fills whole
-// waves (SMs x resident CTAs), discounted by the 8 halo planes each extra split
-// re-reads; the first max_n (capi.cu).
+// z splits of variant v on grid g, cheapest first by the cost model of untuned launches;
+// the first max_n (capi.cu).
 std::vector<int> zchunk_ranking(int kind, int v, const GridDesc& g, int max_n);
 
 // Tuned (variant, zchunks) for kind on grid g on the current device, if the

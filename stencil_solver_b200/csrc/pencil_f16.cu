@@ -664,6 +664,8 @@ const VariantH kF16[] = {
     SB200_VARIANT_H(64, 16, 8, 4, 4, "h64x16_s8_a4"),
     SB200_VARIANT_H(64, 32, 8, 4, 4, "h64x32_s8_a4"),
     SB200_VARIANT_H(128, 16, 8, 4, 4, "h128x16_s8_a4"),
+    SB200_VARIANT_H(64, 32, 8, 2, 4, "h64x32_s8_a2"),
+    SB200_VARIANT_H(128, 16, 8, 2, 4, "h128x16_s8_a2"),
 };
 constexpr int kNumF16 = sizeof(kF16) / sizeof(kF16[0]);
 
@@ -679,6 +681,7 @@ PencilBoxes pencil_f16_boxes(int v) {
     b.halo_y = kF16[v].ty + 2 * R;
     b.tile_x = kF16[v].tx;
     b.tile_y = kF16[v].ty;
+    b.points = b.tile_x * b.tile_y;
     b.aux_tma = true;
     return b;
 }

@@ -54,7 +54,7 @@ template <int TX, int TY, int RPT, int S, int AUX>
 struct Shape {
     static_assert(TX % 4 == 0, "TX must be a multiple of 4 (16-byte TMA origin)");
     static_assert(TY % RPT == 0, "TY must be a multiple of RPT");
-    static_assert(S >= 8, "ring must hold the 8 planes the queue start-up reads");
+    static_assert(S >= 6, "planes z..z+4 staged, plus one in flight");
     static constexpr int SX = TX + 2 * R;
     static constexpr int SY = TY + 2 * R;
     static_assert(SX <= 256 && SY <= 256, "TMA box extent is at most 256");
@@ -224,20 +224,26 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
 
     float4 q[9][RPT];
     bool bad = false;
-    // Start-up: planes 0..7 (z = zb-4 .. zb+3) fill queue slots 0..7.
-#pragma unroll
-    for (int jj = 0; jj < 8; ++jj) {
+    // Start-up: planes 0..7 (z = zb-4 .. zb+3) fill queue slots 0..7; a ring shorter than
+    // that takes the last of them into the stages that planes 0 and 1 leave.
+    auto feed_start = [&](int jj) {
         if (!wait_plane(jj)) bad = true;
         const float* pl = plane(jj) + soff;
 #pragma unroll
         for (int j = 0; j < RPT; ++j) q[jj][j] = lds128(pl + j * P::SX);
-    }
+    };
+#pragma unroll
+    for (int jj = 0; jj < (S < 8 ? S : 8); ++jj) feed_start(jj);
     bool abort_run = __syncthreads_or(bad) != 0;
     if (!abort_run && tid == 0) {
         // Planes 0..3 are only queue feed: their stages are free again.
 #pragma unroll
         for (int jj = 0; jj < R; ++jj)
             if (jj + S < nplanes) issue_plane(jj + S);
+    }
+    if (!abort_run) {
+#pragma unroll
+        for (int jj = S; jj < 8; ++jj) feed_start(jj);
     }
 
     for (int i0 = 0; i0 < nint && !abort_run; i0 += 9) {
@@ -606,6 +612,9 @@ const Variant kWave[] = {
     SB200_VARIANT(32, 16, 1, 8, 4, false, "t32x16_r1_s8_a4"),
     SB200_VARIANT(64, 32, 2, 8, 3, false, "t64x32_r2_s8_a3"),
     SB200_VARIANT(32, 64, 2, 8, 3, false, "t32x64_r2_s8_a3"),
+    SB200_VARIANT(64, 32, 2, 6, 2, false, "t64x32_r2_s6_a2"),
+    SB200_VARIANT(128, 16, 2, 6, 2, false, "t128x16_r2_s6_a2"),
+    SB200_VARIANT(128, 32, 2, 7, 2, false, "t128x32_r2_s7_a2"),
 };
 const Variant kHeat[] = {
     SB200_VARIANT(32, 32, 2, 8, 0, true, "t32x32_r2_s8"),
@@ -614,6 +623,7 @@ const Variant kHeat[] = {
     SB200_VARIANT(64, 32, 2, 8, 0, true, "t64x32_r2_s8"),
     SB200_VARIANT(32, 64, 2, 8, 0, true, "t32x64_r2_s8"),
     SB200_VARIANT(128, 16, 2, 8, 0, true, "t128x16_r2_s8"),
+    SB200_VARIANT(128, 32, 2, 8, 0, true, "t128x32_r2_s8"),
 };
 constexpr int kNumWave = sizeof(kWave) / sizeof(kWave[0]);
 constexpr int kNumHeat = sizeof(kHeat) / sizeof(kHeat[0]);
@@ -687,6 +697,7 @@ PencilBoxes pencil_f32_boxes(bool heat, int v) {
     b.halo_y = x.ty + 2 * R;
     b.tile_x = x.tx;
     b.tile_y = x.ty;
+    b.points = b.tile_x * b.tile_y;
     b.aux_tma = !heat && x.aux > 0;
     return b;
 }
