@@ -519,12 +519,34 @@ private:
                                                          std::to_string(rc) + ")");
             }
         }
+        int sms = 148;
+        int dev = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess)
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaGetLastError();
+        const int resident = f16_ ? batch_f16_resident(variant_) : batch_f32_resident(variant_);
+        // Chunks of the chosen length, halved (down to 16 planes) while less than one chunk
+        // per resident CTA is left: with equal chunks the last ones leave most CTAs idle for
+        // a part of a chunk's time, and a 64-plane chunk is a sixth of a step (16 shots of 96
+        // to 320 cells, FP32 375-390 -> 365 us per step, FP16 259 -> 251; from 1.5 or 2.5
+        // chunks per CTA 370 and 391; the choice of the first length then matters little).
+        int64_t left = 0;  // planes of tiles not handed out yet
+        for (int s = 0; s < n; ++s)
+            left += int64_t(tiles_x[s]) * tiles_y[s] * (shots_[s].g.nz - 8);
+        const double slots = double(sms) * resident;
         for (int s : order) {
-            const int inz = static_cast<int>(shots_[s].g.nz - 8);
-            const int zc = (inz + zlen[s] - 1) / zlen[s];
-            for (int z = 0; z < zc; ++z)
+            const int64_t tiles = int64_t(tiles_x[s]) * tiles_y[s];
+            const int end = static_cast<int>(shots_[s].g.nz - 4);
+            for (int z = 4; z < end;) {
+                int len = zlen[s];
+                while (len > 16 && double(left) < slots * len) len = (len + 1) / 2;
+                len = std::min(len, end - z);
                 for (int y = 0; y < tiles_y[s]; ++y)
-                    for (int x = 0; x < tiles_x[s]; ++x) items.push_back(make_int4(s, x, y, z));
+                    for (int x = 0; x < tiles_x[s]; ++x)
+                        items.push_back(make_int4(s, x, y, z | len << 16));
+                left -= tiles * len;
+                z += len;
+            }
         }
         for (int par = 0; par < 2; ++par) {
             const void* src = f16_ ? static_cast<const void*>(tab16[par].data())
@@ -543,12 +565,6 @@ private:
                                           cudaMemcpyHostToDevice, st_)))
             return rc;
         n_items_ = static_cast<int>(items.size());
-        int sms = 148;
-        int dev = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess)
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaGetLastError();
-        const int resident = f16_ ? batch_f16_resident(variant_) : batch_f32_resident(variant_);
         ctas_ = static_cast<unsigned>(std::min<int64_t>(int64_t(sms) * resident, std::max(1, n_items_)));
         // the host copies above read std::vectors that go out of scope here
         return cuda(cudaStreamSynchronize(st_));

@@ -76,7 +76,7 @@ struct alignas(64) ShotF16 {
     F16Args args;
 };
 
-// Work item: x = shot, y = tile x, z = tile y, w = z chunk.
+// Work item: x = shot, y = tile x, z = tile y, w = first plane | planes << 16.
 int batch_f32_variant_count();
 const char* batch_f32_variant_name(int v);
 PencilBoxes batch_f32_boxes(int v);

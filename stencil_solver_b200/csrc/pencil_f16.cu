@@ -211,7 +211,7 @@ struct RingH {
 constexpr int kUpdConvert = 0, kUpdMixedSub = 1, kUpdExactY = 2;
 
 // One tile: columns [tx TX, tx TX + TX) x rows [4 + ty TY, ...) of the interior,
-// marched over z chunk zc.  All threads of the CTA call it; `sm`, `full` and
+// marched over the planes [zb, ze).  All threads of the CTA call it; `sm`, `full` and
 // `auxf` are the CTA's rings.  CARRY false: their mbarriers are freshly
 // initialised (phase 0 on every stage) and the ring positions are compile-time;
 // CARRY true: `ring` gives the positions (advanced on return).  Every copy it
@@ -220,7 +220,7 @@ constexpr int kUpdConvert = 0, kUpdMixedSub = 1, kUpdExactY = 2;
 template <int TX, int TY, int S, int AUX, int PHASE, int UNR, bool CARRY, int UPD>
 __device__ __forceinline__ bool pencil_f16_tile(const CUtensorMap* pmap, const CUtensorMap* qmap,
                                                 const CUtensorMap* kmap, const F16Args& a,
-                                                int tx, int ty, int zc, uint16_t* sm,
+                                                int tx, int ty, int zb, int ze, uint16_t* sm,
                                                 uint64_t* full, uint64_t* auxf, RingH& ring) {
     using P = ShapeH<TX, TY, S, AUX>;
     const uint32_t pb = CARRY ? ring.p : 0u;    // sequence number of plane 0
@@ -232,8 +232,6 @@ __device__ __forceinline__ bool pencil_f16_tile(const CUtensorMap* pmap, const C
     const int ly = tid / P::TPR;
     const int xa = tx * TX;      // first x of the tile (multiple of 8)
     const int y0 = R + ty * TY;  // first interior row of the tile
-    const int zb = R + zc * a.zlen;
-    const int ze = min(zb + a.zlen, a.nz - R);
     const int nint = ze - zb;
     const int nplanes = nint + 2 * R;
 
@@ -527,9 +525,10 @@ __global__ void __launch_bounds__(ShapeH<TX, TY, S, AUX>::NT, ShapeH<TX, TY, S, 
     b /= a.tiles_x;
     const int ty = b % a.tiles_y;
     b /= a.tiles_y;
+    const int zb = R + b * a.zlen;
     RingH ring;
-    (void)pencil_f16_tile<TX, TY, S, AUX, PHASE, UNR, false, UPD>(&pmap, &qmap, &kmap, a, tx, ty,
-                                                                  b, sm, full, auxf, ring);
+    (void)pencil_f16_tile<TX, TY, S, AUX, PHASE, UNR, false, UPD>(
+        &pmap, &qmap, &kmap, a, tx, ty, zb, min(zb + a.zlen, a.nz - R), sm, full, auxf, ring);
 }
 
 // Many grids (shots) in one persistent launch, as batch_f32_kernel: CTAs take
@@ -557,9 +556,9 @@ __global__ void __launch_bounds__(ShapeH<TX, TY, S, AUX>::NT, ShapeH<TX, TY, S, 
         const int4 w = items[it];
         const ShotF16* sh = shots + w.x;
         const F16Args a = sh->args;
-        if (!pencil_f16_tile<TX, TY, S, AUX, PHASE, UNR, true, UPD>(&sh->p, &sh->prev, &sh->k, a,
-                                                                    w.y, w.z, w.w, sm, full, auxf,
-                                                                    ring))
+        const int zb = w.w & 0xffff, ze = zb + (w.w >> 16);
+        if (!pencil_f16_tile<TX, TY, S, AUX, PHASE, UNR, true, UPD>(
+                &sh->p, &sh->prev, &sh->k, a, w.y, w.z, zb, ze, sm, full, auxf, ring))
             break;
     }
     if (threadIdx.x == 0) {

@@ -131,13 +131,13 @@ __device__ __forceinline__ void ordered_lap(const float4 (&q)[9][RPT], const int
 }
 
 // One tile: columns [x0, x0+TX) x [y0, y0+TY) of the interior, marched over the
-// z chunk zc.  All threads of the CTA call it; `sm`, `full` and `auxf` are the
+// planes [zb, ze).  All threads of the CTA call it; `sm`, `full` and `auxf` are the
 // CTA's rings, initialised by the caller.  Returns false when a bounded wait gave
 // up: the error is recorded and every copy in flight has landed.
 template <int TX, int TY, int RPT, int S, int AUX, int MODE>
 __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUtensorMap* qmap,
                                             const CUtensorMap* vmap, const PencilArgs& a,
-                                            int tile_x, int tile_y, int zc, float* sm,
+                                            int tile_x, int tile_y, int zb, int ze, float* sm,
                                             uint64_t* full, uint64_t* auxf, Ring& ring) {
     using P = Shape<TX, TY, RPT, S, AUX>;
     constexpr bool HEAT = MODE == kModeHeat || MODE == kModeHeatExact;
@@ -152,8 +152,6 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
     const int ly = tid / P::TPR;
     const int x0 = R + tile_x * TX;
     const int y0 = R + tile_y * TY;
-    const int zb = R + zc * a.zlen;
-    const int ze = min(zb + a.zlen, a.nz - R);
     const int nint = ze - zb;          // interior planes this tile computes (>= 1)
     const int nplanes = nint + 2 * R;  // planes of p it reads (>= 9)
     const uint32_t pb = ring.p;        // sequence number of plane 0
@@ -490,9 +488,10 @@ __global__ void __launch_bounds__(Shape<TX, TY, RPT, S, AUX>::NT, Shape<TX, TY, 
     b /= a.tiles_x;
     const int ty = b % a.tiles_y;
     b /= a.tiles_y;
+    const int zb = R + b * a.zlen;
     Ring ring;
-    (void)pencil_tile<TX, TY, RPT, S, AUX, MODE>(&pmap, &qmap, &vmap, a, tx, ty, b, sm, full,
-                                                 auxf, ring);
+    (void)pencil_tile<TX, TY, RPT, S, AUX, MODE>(&pmap, &qmap, &vmap, a, tx, ty, zb,
+                                                 min(zb + a.zlen, a.nz - R), sm, full, auxf, ring);
 }
 
 // Many grids (shots) in one persistent launch.  Each CTA takes work items --
@@ -520,8 +519,9 @@ __global__ void __launch_bounds__(Shape<TX, TY, RPT, S, AUX>::NT, Shape<TX, TY, 
         const int4 w = items[it];
         const ShotF32* sh = shots + w.x;
         const PencilArgs a = sh->args;
+        const int zb = w.w & 0xffff, ze = zb + (w.w >> 16);
         if (!pencil_tile<TX, TY, RPT, S, AUX, kModeAcoustic>(&sh->p, &sh->prev, &sh->vel2, a, w.y, w.z,
-                                                     w.w, sm, full, auxf, ring))
+                                                             zb, ze, sm, full, auxf, ring))
             break;
     }
     if (threadIdx.x == 0) {
@@ -813,11 +813,14 @@ struct BatchVariant {
 #define SB200_BATCH_VARIANT(TX, TY, RPT, S, AUX, NAME) \
     BatchVariant { TX, TY, NAME, &launch_batch<TX, TY, RPT, S, AUX>, &resident_batch<TX, TY, RPT, S, AUX> }
 
+// b64x32_r2_s6_a2 (two CTAs, 16 warps per SM): 394 us per step of 16 uneven shots against
+// 401-408 (b32x16_r1_s8_a4) and 416 (b32x32_r2_s8_a4).  Not kept: 64 x 16 and 64 x 32 tiles
+// with 8 warps per SM (416, 428); 32 x 32, 64 x 16, 128 x 16 and 32 x 64 with the short rings
+// (400-410).
 const BatchVariant kBatch[] = {
     SB200_BATCH_VARIANT(32, 32, 2, 8, 4, "b32x32_r2_s8_a4"),
-    SB200_BATCH_VARIANT(64, 16, 2, 8, 3, "b64x16_r2_s8_a3"),
+    SB200_BATCH_VARIANT(64, 32, 2, 6, 2, "b64x32_r2_s6_a2"),
     SB200_BATCH_VARIANT(32, 16, 1, 8, 4, "b32x16_r1_s8_a4"),
-    SB200_BATCH_VARIANT(64, 32, 2, 8, 3, "b64x32_r2_s8_a3"),
 };
 constexpr int kNumBatch = sizeof(kBatch) / sizeof(kBatch[0]);
 
