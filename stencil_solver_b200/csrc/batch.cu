@@ -319,13 +319,10 @@ public:
                 return rc;
             // on the batch's (non-blocking) stream, behind the unpack: a plain
             // cudaMemcpy would not wait for it
-            if (int rc = cuda(cudaMemcpyAsync(out, staging_, static_cast<size_t>(h.g.size()) * 4,
-                                              cudaMemcpyDeviceToHost, st_)))
-                return rc;
-            return cuda(cudaStreamSynchronize(st_));
+            return cuda(download(bounce_, out, staging_, static_cast<size_t>(h.g.size()) * 4, st_));
         }
-        return cuda(cudaMemcpy(out, arena_ + h.off[step_ & 1], static_cast<size_t>(h.g.size()) * 4,
-                               cudaMemcpyDeviceToHost));
+        return cuda(download(bounce_, out, arena_ + h.off[step_ & 1],
+                             static_cast<size_t>(h.g.size()) * 4, st_));
     }
 
     int get_trace(int s, float* out, int64_t n) {
@@ -757,6 +754,7 @@ private:
     int64_t scratch_len_ = 0;
     float* bound_ = nullptr;    // FP16: per-shot source bound per step (max_steps each)
     float* staging_ = nullptr;  // FP16: one shot's FP32 field
+    HostBounce bounce_;
     std::vector<std::vector<float>> wave_host_;
     std::vector<float> vel2_src_;
 

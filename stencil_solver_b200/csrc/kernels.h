@@ -208,6 +208,16 @@ int stats_blocks(const GridDesc& g);
 cudaError_t launch_field_stats(const void* field, bool half, const GridDesc& g, float scale,
                                double* out3, double* scratch, cudaStream_t stream);
 
+// Copies bytes of device memory to the host behind the work on `st` and waits for it
+// (hostcopy.cpp); pageable destinations go through the handle's pinned buffers.
+struct HostBounce {
+    char* buf[2] = {nullptr, nullptr};
+    cudaEvent_t done[2] = {nullptr, nullptr};
+    ~HostBounce();
+    bool ready();
+};
+cudaError_t download(HostBounce& b, void* host, const void* dev, size_t bytes, cudaStream_t st);
+
 // Tensor maps (tmap.cpp).  Encodes (and caches) a 3-D tiled map over a
 // halo-inclusive field of element size esize bytes with the given box and copies
 // it to *out.  Returns 0 or a CUresult / -1 (driver entry point unavailable).

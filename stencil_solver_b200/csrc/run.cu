@@ -240,7 +240,7 @@ public:
     int get_field(float* host) {
         if (!host) return set_error(SB200_ERR_INVALID, "sb200_run_get_field: NULL destination");
         if (int rc = synchronize()) return rc;
-        if (!fp16_) return cuda(cudaMemcpy(host, a_, n_ * 4, cudaMemcpyDeviceToHost));
+        if (!fp16_) return cuda(download(bounce_, host, a_, n_ * 4, st_));
         F16Scale s;
         if (int rc = cuda(cudaMemcpy(&s, scale_dev_, sizeof(s), cudaMemcpyDeviceToHost))) return rc;
         if (int rc = ensure_stage()) return rc;
@@ -248,10 +248,9 @@ public:
             const int64_t m = std::min(kStageFloats, n_ - off);
             if (int rc = sb200_f16_unpack(static_cast<const uint16_t*>(a_) + off, stage_, m, s.a, st_))
                 return rc;
-            if (int rc = cuda(cudaMemcpyAsync(host + off, stage_, m * 4, cudaMemcpyDeviceToHost, st_)))
-                return rc;
+            if (int rc = cuda(download(bounce_, host + off, stage_, m * 4, st_))) return rc;
         }
-        return cuda(cudaStreamSynchronize(st_));
+        return SB200_OK;
     }
 
     // XY plane z (nx * ny floats, x fastest) of the current field in physical
@@ -579,6 +578,7 @@ private:
     int* monitor_dev_ = nullptr;
     F16Scale* scale_dev_ = nullptr;
     float* stage_ = nullptr;
+    HostBounce bounce_;
     cudaGraphExec_t graph_[2] = {nullptr, nullptr};
     void* home_ = nullptr;  // buffer that is current at even parity
     int64_t step_ = 0;
