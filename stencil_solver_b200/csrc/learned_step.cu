@@ -461,71 +461,42 @@ __global__ void __launch_bounds__(LNT, 3)
         }
         const float* pc = plane(i + 4) + soff;
         const float4 c = q[4];
-        // Weights from the kernel parameters (constant bank) each plane, so they
-        // hold no registers through the network epilogues.
-        float2 ax2[R], ay2[R], az2[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            ax2[r] = dup2(a.w.ax[r]);
-            ay2[r] = dup2(a.w.ay[r]);
-            az2[r] = dup2(a.w.az[r]);
-        }
-        const float2 cx2 = dup2(a.w.cx), cy2 = dup2(a.w.cy), cz2 = dup2(a.w.cz),
-                     neg1 = dup2(-1.f), neg2 = dup2(-2.f);
-
-        // Stencil: the FP32 pencil kernel's arithmetic in its order (y per row
-        // from zero, farthest rows first; x and z pair sums; (x + y) + z).
-        // mag: the largest magnitude in the thread's 4 stars.
-        auto absmax4 = [](const float4& v) {
-            return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-        };
-        float mag = absmax4(q[0]);
-#pragma unroll
-        for (int k = 1; k < 9; ++k) mag = fmaxf(mag, absmax4(q[k]));
-        float2 ya[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-        for (int k = -R; k <= R; ++k) {
-            if (k == 0) continue;
-            const float4 row = lds128(pc + k * LSX);
-            mag = fmaxf(mag, absmax4(row));
-            const int d = k > 0 ? k : -k;
-            ya[0] = fma2(ay2[d - 1], pair_of(row, 0), ya[0]);
-            ya[1] = fma2(ay2[d - 1], pair_of(row, 1), ya[1]);
-        }
         const float4 lf = lds128(pc - 4);
         const float4 rt = lds128(pc + 4);
-        mag = fmaxf(mag, fmaxf(absmax4(lf), absmax4(rt)));
-        // Some star of the thread is nonzero and reaches the floor.
-        const bool tact = rin && mag > 0.f && mag >= a.min_scale;
         const float win[12] = {lf.x, lf.y, lf.z, lf.w, c.x, c.y, c.z, c.w, rt.x, rt.y, rt.z, rt.w};
-        float2 lap[2];
+        const float2 neg1 = dup2(-1.f), neg2 = dup2(-2.f);
+
+        // Largest magnitude of each of the thread's 4 stars: the y and z arms lane by lane,
+        // the x arms as the six cells that all four share and the three that are left.
+        float mx[4] = {fabsf(c.x), fabsf(c.y), fabsf(c.z), fabsf(c.w)};
+        auto raise = [&](const float4& u, const float4& v) {
+            mx[0] = fmaxf(mx[0], fmaxf(fabsf(u.x), fabsf(v.x)));
+            mx[1] = fmaxf(mx[1], fmaxf(fabsf(u.y), fabsf(v.y)));
+            mx[2] = fmaxf(mx[2], fmaxf(fabsf(u.z), fabsf(v.z)));
+            mx[3] = fmaxf(mx[3], fmaxf(fabsf(u.w), fabsf(v.w)));
+        };
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const float2 ce = pair_of(c, h);
-            float2 tz = mul2(cz2, ce);
-            float2 tx = mul2(cx2, ce);
-#pragma unroll
-            for (int r = 1; r <= R; ++r) {
-                tz = fma2(az2[r - 1], add2(pair_of(q[4 + r], h), pair_of(q[4 - r], h)), tz);
-                const int e = 4 + 2 * h;
-                const float2 s = make_float2(win[e + r] + win[e - r], win[e + 1 + r] + win[e + 1 - r]);
-                tx = fma2(ax2[r - 1], s, tx);
-            }
-            const float2 tyv = fma2(cy2, ce, ya[h]);
-            lap[h] = add2(add2(tx, tyv), tz);
+        for (int r = 1; r <= R; ++r) {
+            raise(q[4 + r], q[4 - r]);
+            raise(lds128(pc + r * LSX), lds128(pc - r * LSX));
         }
+        {
+            float w[12];
+#pragma unroll
+            for (int k = 0; k < 12; ++k) w[k] = fabsf(win[k]);
+            const float core = fmaxf(fmaxf(w[3], fmaxf(w[4], w[5])), fmaxf(w[6], fmaxf(w[7], w[8])));
+            const float in2 = fmaxf(core, w[2]), in9 = fmaxf(core, w[9]);
+            mx[0] = fmaxf(mx[0], fmaxf(in2, fmaxf(w[0], w[1])));
+            mx[1] = fmaxf(mx[1], fmaxf(in2, fmaxf(w[1], w[9])));
+            mx[2] = fmaxf(mx[2], fmaxf(in9, fmaxf(w[2], w[10])));
+            mx[3] = fmaxf(mx[3], fmaxf(in9, fmaxf(w[10], w[11])));
+        }
+        // Some star of the thread is nonzero and reaches the floor.
+        const float mag = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        const bool tact = rin && mag > 0.f && mag >= a.min_scale;
         if (!mbar_wait(&auxf[i % LAUX], (i / LAUX) & 1)) bad = true;
         const float* st = aux + (i % LAUX) * 2 * LTILE + aoff;
-        const float4 pv = lds128(st);
         const float4 vv = lds128(st + LTILE);
-        float4 o;
-        {
-            const float2 t0 = fma2(neg1, pair_of(pv, 0), add2(pair_of(c, 0), pair_of(c, 0)));
-            const float2 t1 = fma2(neg1, pair_of(pv, 1), add2(pair_of(c, 1), pair_of(c, 1)));
-            const float2 o0 = fma2(pair_of(vv, 0), lap[0], t0);
-            const float2 o1 = fma2(pair_of(vv, 1), lap[1], t1);
-            o = make_float4(o0.x, o0.y, o1.x, o1.y);
-        }
 
         // Features, one pair of points at a time, in the correction kernel's
         // arithmetic: the star's largest magnitude gives s first, then per axis
@@ -548,20 +519,10 @@ __global__ void __launch_bounds__(LNT, 3)
 #pragma unroll
         for (int h = 0; h < 2 && tact; ++h) {
             const float2 ce = pair_of(c, h);
-            float2 mx = make_float2(fabsf(ce.x), fabsf(ce.y));
-#pragma unroll
-            for (int a3 = 0; a3 < 3; ++a3)
-#pragma unroll
-                for (int r = 1; r <= R; ++r) {
-                    const float2 up = arm(a3, r, h);
-                    const float2 dn = arm(a3, -r, h);
-                    mx.x = fmaxf(mx.x, fmaxf(fabsf(up.x), fabsf(dn.x)));
-                    mx.y = fmaxf(mx.y, fmaxf(fabsf(up.y), fabsf(dn.y)));
-                }
             float2 iv;
             float s0, s1;
-            pow2_scale(rin && mx.x >= a.min_scale ? mx.x : 0.f, s0, iv.x);
-            pow2_scale(rin && mx.y >= a.min_scale ? mx.y : 0.f, s1, iv.y);
+            pow2_scale(rin && mx[2 * h] >= a.min_scale ? mx[2 * h] : 0.f, s0, iv.x);
+            pow2_scale(rin && mx[2 * h + 1] >= a.min_scale ? mx[2 * h + 1] : 0.f, s1, iv.y);
             sc[2 * h] = s0 * a.out_scale;
             sc[2 * h + 1] = s1 * a.out_scale;
             act = act || s0 > 0.f || s1 > 0.f;
@@ -594,46 +555,99 @@ __global__ void __launch_bounds__(LNT, 3)
         const bool any = __syncthreads_or(act) != 0;
         tc_fence_after();
         abort_run = s_flag != 0;
-        if (!abort_run && tid == 0) {
-            // The staged plane z and the aux stage of this plane are free now.
-            if (i + 4 + LS < nplanes) issue_plane(i + 4 + LS);
-            if (i + LAUX < nint) issue_aux(i + LAUX);
-            if (any) {
+        if (!abort_run && any && tid == 0) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    tc_mma(tmem + 32 * e, umma_desc(aA + e * kTileA), umma_desc(aW1), 0u);
-                    tc_mma(tmem + 32 * e, umma_desc(aA + e * kTileA + 256), umma_desc(aW1 + 256), 1u);
-                }
-                tc_commit(&mbar);
+            for (int e = 0; e < 4; ++e) {
+                tc_mma(tmem + 32 * e, umma_desc(aA + e * kTileA), umma_desc(aW1), 0u);
+                tc_mma(tmem + 32 * e, umma_desc(aA + e * kTileA + 256), umma_desc(aW1 + 256), 1u);
             }
+            tc_commit(&mbar);
+        }
+        if (!abort_run && any) ++ncommit;
+
+        // Stencil, while layer 1 runs: the FP32 pencil kernel's arithmetic in its order (y
+        // per row from zero, farthest rows first; x and z pair sums; (x + y) + z).  Weights
+        // from the kernel parameters (constant bank) each plane, so they hold no registers
+        // through the network epilogues.
+        float4 o;
+        {
+            float2 ax2[R], ay2[R], az2[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                ax2[r] = dup2(a.w.ax[r]);
+                ay2[r] = dup2(a.w.ay[r]);
+                az2[r] = dup2(a.w.az[r]);
+            }
+            const float2 cx2 = dup2(a.w.cx), cy2 = dup2(a.w.cy), cz2 = dup2(a.w.cz);
+            float2 ya[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+            for (int k = -R; k <= R; ++k) {
+                if (k == 0) continue;
+                const float4 row = lds128(pc + k * LSX);
+                const int d = k > 0 ? k : -k;
+                ya[0] = fma2(ay2[d - 1], pair_of(row, 0), ya[0]);
+                ya[1] = fma2(ay2[d - 1], pair_of(row, 1), ya[1]);
+            }
+            float2 lap[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 ce = pair_of(c, h);
+                float2 tz = mul2(cz2, ce);
+                float2 txv = mul2(cx2, ce);
+#pragma unroll
+                for (int r = 1; r <= R; ++r) {
+                    tz = fma2(az2[r - 1], add2(pair_of(q[4 + r], h), pair_of(q[4 - r], h)), tz);
+                    const int e = 4 + 2 * h;
+                    const float2 sx =
+                        make_float2(win[e + r] + win[e - r], win[e + 1 + r] + win[e + 1 - r]);
+                    txv = fma2(ax2[r - 1], sx, txv);
+                }
+                const float2 tyv = fma2(cy2, ce, ya[h]);
+                lap[h] = add2(add2(txv, tyv), tz);
+            }
+            const float4 pv = lds128(st);
+            const float2 t0 = fma2(neg1, pair_of(pv, 0), add2(pair_of(c, 0), pair_of(c, 0)));
+            const float2 t1 = fma2(neg1, pair_of(pv, 1), add2(pair_of(c, 1), pair_of(c, 1)));
+            const float2 o0 = fma2(pair_of(vv, 0), lap[0], t0);
+            const float2 o1 = fma2(pair_of(vv, 1), lap[1], t1);
+            o = make_float4(o0.x, o0.y, o1.x, o1.y);
         }
         // Warps without an active point skip the epilogues (TMEM loads are
         // warp-wide): their rows' results are discarded.
         const bool wact = __any_sync(0xffffffffu, act);
-        if (!abort_run && any) ++ncommit;
-        if (!abort_run && any && wact) {
+        const bool run = !abort_run && any && wact;
+        uint32_t d[2][4][8];  // accumulator chunks: one at hand, one on its way
+        auto value = [](uint32_t x) { return __uint_as_float(x); };
+        if (run) {
             wait_mma();  // the layer-1 accumulators
-            // Layer 1 epilogue: h1 = relu(acc + b1) as BF16.
+            // Layer 1 epilogue, 8 columns of the 4 tiles at a time: h1 = relu(acc + b1) as
+            // BF16, one 16-byte piece of each row.
+            tc_ld4x8(lane_base, 0, d[0]);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float d[32];
-                tc_ld32(lane_base + 32 * e, d);
-                uint32_t hw[16];
+            for (int k = 0; k < 4; ++k) {
+                tc_wait_ld(d[k & 1]);
+                if (k < 3) tc_ld4x8(lane_base, k + 1, d[(k + 1) & 1]);
 #pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    const float2 t = add2(make_float2(d[2 * k], d[2 * k + 1]),
-                                          make_float2(a.b1[2 * k], a.b1[2 * k + 1]));
-                    hw[k] = relu_bf2(t.x, t.y);
+                for (int e = 0; e < 4; ++e) {
+                    uint32_t hw[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 t = add2(make_float2(value(d[k & 1][e][2 * j]),
+                                                          value(d[k & 1][e][2 * j + 1])),
+                                              make_float2(a.b1[8 * k + 2 * j], a.b1[8 * k + 2 * j + 1]));
+                        hw[j] = relu_bf2(t.x, t.y);
+                    }
+                    *reinterpret_cast<uint4*>(sA + e * kTileA + core_off(tid, 8 * k)) =
+                        make_uint4(hw[0], hw[1], hw[2], hw[3]);
                 }
-                store_row(sA + e * kTileA, tid, hw);
             }
             fence_async_smem();
         }
-        if (!abort_run && any) {
-            tc_fence_before();
-            __syncthreads();
-            tc_fence_after();
-            if (tid == 0) {
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        if (!abort_run && tid == 0) {
+            if (any) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     tc_mma(tmem + 32 * e, umma_desc(aA + e * kTileA), umma_desc(aW2), 0u);
@@ -641,36 +655,43 @@ __global__ void __launch_bounds__(LNT, 3)
                 }
                 tc_commit(&mbar);
             }
-            ++ncommit;
+            // The staged plane z and the aux stage of this plane are free now.
+            if (i + 4 + LS < nplanes) issue_plane(i + 4 + LS);
+            if (i + LAUX < nint) issue_aux(i + LAUX);
         }
-        if (!abort_run && any && wact) {
+        if (!abort_run && any) ++ncommit;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) q[k] = q[k + 1];  // while layer 2 runs
+        if (run) {
             wait_mma();
             // Layer 2 epilogue and the output layer, in the correction kernel's
             // order; then p_next = stencil + s c y.
+            float2 acc[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                float d[32];
-                tc_ld32(lane_base + 32 * e, d);
-                float2 acc = make_float2(0.f, 0.f);
+            for (int e = 0; e < 4; ++e) acc[e] = make_float2(0.f, 0.f);
+            tc_ld4x8(lane_base, 0, d[0]);
 #pragma unroll
-                for (int q4 = 0; q4 < 8; ++q4) {
-                    const float2 uu = add2(make_float2(d[4 * q4], d[4 * q4 + 1]),
-                                           make_float2(a.b2[4 * q4], a.b2[4 * q4 + 1]));
-                    const float2 vw = add2(make_float2(d[4 * q4 + 2], d[4 * q4 + 3]),
-                                           make_float2(a.b2[4 * q4 + 2], a.b2[4 * q4 + 3]));
-                    acc = fma2(make_float2(a.w3[4 * q4], a.w3[4 * q4 + 1]),
-                               make_float2(fmaxf(uu.x, 0.f), fmaxf(uu.y, 0.f)), acc);
-                    acc = fma2(make_float2(a.w3[4 * q4 + 2], a.w3[4 * q4 + 3]),
-                               make_float2(fmaxf(vw.x, 0.f), fmaxf(vw.y, 0.f)), acc);
-                }
-                const float yv = (acc.x + acc.y) + a.b3;
-                if (sc[e] > 0.f) {
-                    if (e == 0) o.x = fmaf(sc[e], yv, o.x);
-                    if (e == 1) o.y = fmaf(sc[e], yv, o.y);
-                    if (e == 2) o.z = fmaf(sc[e], yv, o.z);
-                    if (e == 3) o.w = fmaf(sc[e], yv, o.w);
+            for (int k = 0; k < 4; ++k) {
+                tc_wait_ld(d[k & 1]);
+                if (k < 3) tc_ld4x8(lane_base, k + 1, d[(k + 1) & 1]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int col = 8 * k + 2 * j;
+                    const float2 b = make_float2(a.b2[col], a.b2[col + 1]);
+                    const float2 w = make_float2(a.w3[col], a.w3[col + 1]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 u = add2(make_float2(value(d[k & 1][e][2 * j]),
+                                                          value(d[k & 1][e][2 * j + 1])),
+                                              b);
+                        acc[e] = fma2(w, make_float2(fmaxf(u.x, 0.f), fmaxf(u.y, 0.f)), acc[e]);
+                    }
                 }
             }
+            auto corrected = [&](int e, float x) {
+                return sc[e] > 0.f ? fmaf(sc[e], (acc[e].x + acc[e].y) + a.b3, x) : x;
+            };
+            o = make_float4(corrected(0, o.x), corrected(1, o.y), corrected(2, o.z), corrected(3, o.w));
             tc_fence_before();
         }
         if (!bad && rin) {
@@ -679,8 +700,6 @@ __global__ void __launch_bounds__(LNT, 3)
             if (m > 0.f && m >= a.flag_floor) bits |= face_bits(lx, ly, i, nint);
         }
         goff += a.sz;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) q[k] = q[k + 1];
     }
     {
         const uint32_t out_bits = block_or(bits);

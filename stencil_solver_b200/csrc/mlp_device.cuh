@@ -182,6 +182,28 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Chunk c (8 FP32 columns) of this thread's TMEM lane in each of 4 accumulator tiles of 32
+// columns, without waiting; tc_wait_ld returns when every load issued so far has arrived
+// (the registers pass through it, so no use of them can move ahead of it).
+__device__ __forceinline__ void tc_ld4x8(uint32_t taddr, int c, uint32_t (&r)[4][8]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(r[e][0]), "=r"(r[e][1]), "=r"(r[e][2]), "=r"(r[e][3]), "=r"(r[e][4]),
+              "=r"(r[e][5]), "=r"(r[e][6]), "=r"(r[e][7])
+            : "r"(taddr + 32 * e + 8 * c)
+            : "memory");
+}
+__device__ __forceinline__ void tc_wait_ld(uint32_t (&r)[4][8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        asm volatile(""
+                     : "+r"(r[e][0]), "+r"(r[e][1]), "+r"(r[e][2]), "+r"(r[e][3]), "+r"(r[e][4]),
+                       "+r"(r[e][5]), "+r"(r[e][6]), "+r"(r[e][7])::"memory");
+}
+
 // One feature / activation row (16 words = 32 BF16) into a K-major operand tile.
 __device__ __forceinline__ void store_row(unsigned char* tile, int row, const uint32_t (&w)[16]) {
 #pragma unroll
