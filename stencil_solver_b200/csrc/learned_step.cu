@@ -19,8 +19,8 @@
 //      (4 tiles x 128 rows, K-major BF16), so TMEM lane `tid` of tile e's
 //      accumulator is this thread's own point: the correction lands in the
 //      thread that holds the stencil value and one store writes p_next;
-//   3. one thread issues tcgen05.mma (M = 128, N = 32, K = 16: 2 per tile and
-//      layer) into TMEM columns 32 e, commits to an mbarrier that every thread
+//   3. a thread of warp e issues tile e's tcgen05.mma (M = 128, N = 32, K = 16: 2 per
+//      layer) into TMEM columns 32 e and commits to an mbarrier that every thread
 //      waits on (two CTA barriers per plane in all); the epilogue of
 //      layer 1 (bias, ReLU, BF16) writes layer 2's A tiles over the
 //      features, layer 2 overwrites the accumulators, its epilogue (bias, ReLU,
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(LNT, 3)
     float* sm = reinterpret_cast<float*>(base + kOffP);
     float* aux = reinterpret_cast<float*>(base + kOffAux);
 
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int lx = tid % LTPR, ly = tid / LTPR;
     int b = blockIdx.x;
     const int tx = b % a.tiles_x;
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(LNT, 3)
         for (int s = 0; s < LS; ++s) mbar_init(&full[s], 1);
 #pragma unroll
         for (int s = 0; s < LAUX; ++s) mbar_init(&auxf[s], 1);
-        mbar_init(&mbar, 1);
+        mbar_init(&mbar, LNT / 32);  // one commit per warp and layer
         fence_barrier_init();
         s_flag = 0;
     }
@@ -388,7 +388,13 @@ __global__ void __launch_bounds__(LNT, 3)
     tc_fence_after();
     const uint32_t tmem = s_tmem;
     const uint32_t lane_base = tmem + (uint32_t(32 * warp) << 16);
-    const uint32_t aA = smem_u32(sA), aW1 = smem_u32(sW1), aW2 = smem_u32(sW2);
+    // Warp e issues tile e's MMAs: its accumulator and its operands' descriptors (the K = 16
+    // steps start 256 bytes, 16 units of the address field, apart).  One thread issuing all 8
+    // of a layer, with their descriptors built each time, kept its warp's other lanes and the
+    // block's barrier waiting (260^3, active everywhere: 315 -> 300 us).
+    const uint32_t tacc = tmem + 32 * warp;
+    const uint64_t dA0 = umma_desc(smem_u32(sA) + warp * kTileA), dA1 = dA0 + 16,
+                   dW1 = umma_desc(smem_u32(sW1)), dW2 = umma_desc(smem_u32(sW2));
 
     int issued_hi = -1, aux_issued_hi = -1;
     auto plane = [&](int j) -> const float* { return sm + (j % LS) * LPLANE; };
@@ -555,12 +561,9 @@ __global__ void __launch_bounds__(LNT, 3)
         const bool any = __syncthreads_or(act) != 0;
         tc_fence_after();
         abort_run = s_flag != 0;
-        if (!abort_run && any && tid == 0) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                tc_mma(tmem + 32 * e, umma_desc(aA + e * kTileA), umma_desc(aW1), 0u);
-                tc_mma(tmem + 32 * e, umma_desc(aA + e * kTileA + 256), umma_desc(aW1 + 256), 1u);
-            }
+        if (!abort_run && any && lane == 0) {  // warp e: tile e
+            tc_mma(tacc, dA0, dW1, 0u);
+            tc_mma(tacc, dA1, dW1 + 16, 1u);
             tc_commit(&mbar);
         }
         if (!abort_run && any) ++ncommit;
@@ -646,18 +649,15 @@ __global__ void __launch_bounds__(LNT, 3)
         tc_fence_before();
         __syncthreads();
         tc_fence_after();
-        if (!abort_run && tid == 0) {
+        if (!abort_run && lane == 0) {
             if (any) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    tc_mma(tmem + 32 * e, umma_desc(aA + e * kTileA), umma_desc(aW2), 0u);
-                    tc_mma(tmem + 32 * e, umma_desc(aA + e * kTileA + 256), umma_desc(aW2 + 256), 1u);
-                }
+                tc_mma(tacc, dA0, dW2, 0u);
+                tc_mma(tacc, dA1, dW2 + 16, 1u);
                 tc_commit(&mbar);
             }
             // The staged plane z and the aux stage of this plane are free now.
-            if (i + 4 + LS < nplanes) issue_plane(i + 4 + LS);
-            if (i + LAUX < nint) issue_aux(i + LAUX);
+            if (warp == 0 && i + 4 + LS < nplanes) issue_plane(i + 4 + LS);
+            if (warp == 0 && i + LAUX < nint) issue_aux(i + LAUX);
         }
         if (!abort_run && any) ++ncommit;
 #pragma unroll
