@@ -149,6 +149,12 @@ std::vector<std::pair<double, int>> rank_splits(int64_t tiles, int inz, int resi
 //     staged words a point instead of 1.41);
 //   * small grids: as many short CTAs as there are slots (acoustic 64^3 4.9 -> 3.2 us,
 //     320^3 96 -> 84 us; heat 160^3 10.5 -> 8.1 us; FP16 96^3 6.0 -> 5.2 us).
+//   * reference order: 59 separately rounded operations a point, bound by issue and power;
+//     the one-row tile covers odd extents best, two-row tiles spend fewer instructions a
+//     point (acoustic 384^3 178 us with t32x16_r1_s8_a4, 174 / 174 / 170 with the other
+//     three in the table's order; 512^3 438 against 410 / 408 / 415; 160 x 150 x 170 14.1
+//     against 17.7 / 19.1 / 21.2; heat 512^3 301 against 288, 160 x 150 x 170 12.1 against
+//     13.7).
 struct Candidate {
     const char* name;
     double in_l2, beyond;
@@ -158,6 +164,10 @@ struct Family {
     int step_bytes;  // per cell: the fields a step keeps in use
     Candidate tiles[4];
 };
+// Kinds of choice beyond the public ones: the reference order on the pencil tiles, and the
+// ragged kernels.
+enum Internal : int { kExactWave = 4, kExactHeat, kRaggedWave, kRaggedHeat };
+
 const Family kFamilies[] = {
     // SB200_KIND_WAVE_F32
     {2.1, 12,
@@ -167,6 +177,13 @@ const Family kFamilies[] = {
     {6.7, 8, {{"t32x32_r2_s8", 1.05, 0}, {"t64x16_r2_s8", 1.0, 1.114}, {"t128x16_r2_s8", 0, 1.0}}},
     // SB200_KIND_WAVE_F16
     {4.3, 6, {{"h64x16_s8_a4", 0, 1.02}, {"h64x32_s8_a2", 1.1, 0}, {"h128x16_s8_a2", 1.0, 1.0}}},
+    {},  // SB200_KIND_WAVE2_F32: one tile
+    // kExactWave
+    {2.1, 12,
+     {{"t32x16_r1_s8_a4", 1.0, 1.0}, {"t64x32_r2_s6_a2", 0.95, 0.95},
+      {"t128x16_r2_s6_a2", 0.94, 0.94}, {"t128x32_r2_s7_a2", 0.92, 0.92}}},
+    // kExactHeat
+    {2.1, 8, {{"t32x16_r1_s8", 1.0, 1.0}, {"t64x16_r2_s8", 0.96, 0.96}}},
 };
 constexpr double kL2Bytes = 126e6;
 
@@ -188,8 +205,11 @@ int resident_ctas(int kind, int v) {
                                          : pencil_f32_resident(kind == SB200_KIND_HEAT_F32, v);
 }
 
-PencilConfig cheapest(int kind, const GridDesc& g) {
-    const Family& f = kFamilies[kind];
+// The cheapest tile and split of a family (a public kind's or a reference-order one).
+PencilConfig cheapest(int family, const GridDesc& g) {
+    const Family& f = kFamilies[family];
+    const bool exact = family >= kExactWave;
+    const int kind = !exact ? family : family == kExactHeat ? SB200_KIND_HEAT_F32 : SB200_KIND_WAVE_F32;
     const bool beyond = double(g.size()) * f.step_bytes > kL2Bytes;
     PencilConfig best;
     double cost = 0;
@@ -200,7 +220,8 @@ PencilConfig cheapest(int kind, const GridDesc& g) {
         const PencilBoxes b = kind == SB200_KIND_WAVE_F16
                                   ? pencil_f16_boxes(v)
                                   : pencil_f32_boxes(kind == SB200_KIND_HEAT_F32, v);
-        const int resident = resident_ctas(kind, v);
+        const int resident = exact ? pencil_f32_resident(kind == SB200_KIND_HEAT_F32, v, true)
+                                   : resident_ctas(kind, v);
         const auto s =
             rank_splits(column_tiles(kind, v, g), static_cast<int>(g.nz - 8), resident, f.start)
                 .front();
@@ -213,18 +234,6 @@ PencilConfig cheapest(int kind, const GridDesc& g) {
     }
     return best;
 }
-
-// Tile of the reference-order steps: 59 separately rounded operations a point leave them
-// short of warps rather than of bytes, and the one-row tile runs 4 CTAs per SM (384^3
-// acoustic: 162 us against 170-175 for the two-row tiles).
-int exact_variant(bool heat) {
-    return heat ? variant_by_name(SB200_KIND_HEAT_F32, "t32x16_r1_s8")
-                : variant_by_name(SB200_KIND_WAVE_F32, "t32x16_r1_s8_a4");
-}
-
-// Family of steps with a choice of their own beyond the public kinds: the reference
-// order on the pencil tiles, and the ragged kernels.
-enum Internal : int { kExactWave = 4, kExactHeat, kRaggedWave, kRaggedHeat };
 
 PencilConfig choose(int kind, const GridDesc& g) {
     {
@@ -257,13 +266,6 @@ PencilConfig choose(int kind, const GridDesc& g) {
     const double start = kFamilies[SB200_KIND_WAVE_F32].start;
     if (kind >= kRaggedWave) {
         c.zchunks = rank_splits(ragged_ctas(g, 1), inz, ragged_resident(kind == kRaggedHeat, g), start)
-                        .front()
-                        .second;
-    } else if (kind >= kExactWave) {
-        const bool heat = kind == kExactHeat;
-        c.variant = exact_variant(heat);
-        c.zchunks = rank_splits(pencil_f32_ctas(heat, c.variant, g, 1), inz,
-                                pencil_f32_resident(heat, c.variant, true), start)
                         .front()
                         .second;
     } else if (kind == SB200_KIND_WAVE2_F32) {

@@ -13,8 +13,13 @@
 //     second AUX-stage ring, AUX-1 planes ahead of their use (AUX = 0 instead loads
 //     them with 128-bit global loads at the start of the plane).
 //   * Each thread owns a float4 of x (4 points) in RPT consecutive rows.  Its z
-//     neighbours (z-4..z+4) live in a 9-deep register queue; the loop is unrolled
-//     by 9 so queue slots are compile-time registers and nothing is shifted.
+//     neighbours (z-4..z+4) live in a register queue of Q planes and the loop is unrolled
+//     by Q, so queue slots are compile-time registers.  Q = 9 shifts nothing.  The
+//     reference-order modes have Q = 8 (the pair z-4, z+4 is added as plane z+4 takes
+//     plane z-4's slot): the stages of an 8-stage ring are then compile-time too, which
+//     takes their t32x16_r1_s8_a4 from 57 to 53 instructions a point, 384^3 from 193 to
+//     179 us.  The other modes gain nothing by it (heat 23.9 -> 25.2 instructions: the
+//     slot's new plane needs a move; the acoustic rings have 6 or 7 stages).
 //   * x and y neighbours come from the staged plane with 128-bit shared loads (a
 //     quarter-warp reads 128 contiguous bytes, so no bank conflicts).
 //   * p_next is written with 128-bit streaming stores and may alias p_prev (in-place
@@ -68,13 +73,31 @@ struct Shape {
     static constexpr int MINB = (512 / NT) > 0 ? (512 / NT) : 1;  // caps registers at 128
 };
 
-// Ring position a CTA carries from one tile to the next: the sequence numbers of
-// the next p plane and the next aux iteration.  Stage = seq % ring size, phase
-// parity = (seq / ring size) & 1, so the mbarriers are initialised once per CTA
-// and their phases simply continue across the tiles a persistent CTA processes.
+// Ring state a CTA carries from one tile to the next, so that the mbarriers are
+// initialised once and their phases continue across the tiles a persistent CTA
+// processes.  A ring whose size divides the unroll starts every tile at stage 0 (its
+// stages are then compile-time) and carries one bit per stage, the parity of its next
+// phase; another ring carries the sequence number of its next plane: stage = seq % size,
+// parity = (seq / size) & 1.
 struct Ring {
     uint32_t p = 0;
     uint32_t aux = 0;
+};
+template <int S, int Q>
+struct RingOf {
+    static constexpr bool kBits = Q % S == 0;
+    // Stage and phase parity of a tile's j-th fill, from the carried state.
+    static __device__ __forceinline__ uint32_t stage(uint32_t at, uint32_t j) {
+        return kBits ? j % S : (at + j) % S;
+    }
+    static __device__ __forceinline__ uint32_t parity(uint32_t at, uint32_t j) {
+        return (kBits ? (at >> (j % S)) ^ (j / S) : (at + j) / S) & 1u;
+    }
+    // The state after a tile of n fills.
+    static __device__ __forceinline__ uint32_t after(uint32_t at, uint32_t n) {
+        if (!kBits) return at + n;
+        return at ^ ((n / S) & 1u ? (1u << S) - 1u : 0u) ^ ((1u << (n % S)) - 1u);
+    }
 };
 
 // Laplacian of the thread's RPT x 4 points in the reference's operation order
@@ -84,12 +107,12 @@ struct Ring {
 // the kernel's arguments: the same rounding as an add, and nothing that the
 // compiler can contract (it does contract mul.rn.f32x2 into add.rn.f32x2).
 template <int RPT, int SX>
-__device__ __forceinline__ void ordered_lap(const float4 (&q)[9][RPT], const int u, const float* pc,
-                                            const PencilArgs& a, const float2 one,
-                                            float2 (&lap)[RPT][2]) {
+__device__ __forceinline__ void ordered_lap(const float4 (&q)[8][RPT], const float2 (&z4)[RPT][2],
+                                            const int u, const float* pc, const PencilArgs& a,
+                                            const float2 one, float2 (&lap)[RPT][2]) {
     const float2 c2[R + 1] = {dup2(C0), dup2(C1), dup2(C2), dup2(C3), dup2(C4)};
     const float2 ix2 = dup2(a.inv_dx2), iy2 = dup2(a.inv_dy2), iz2 = dup2(a.inv_dz2);
-    const int cs = (u + 4) % 9;
+    const int cs = (u + 4) % 8;
 #pragma unroll
     for (int j = 0; j < RPT; ++j) {
         const float4 c = q[cs][j];
@@ -109,8 +132,9 @@ __device__ __forceinline__ void ordered_lap(const float4 (&q)[9][RPT], const int
             for (int h = 0; h < 2; ++h) {
                 const float2 sy = add2(pair_of(yu, h), pair_of(yd, h));
                 ly[h] = fma2(mul2(mul2(c2[r], sy), iy2), one, ly[h]);
-                const float2 sz = add2(pair_of(q[(u + 4 + r) % 9][j], h),
-                                       pair_of(q[(u + 4 - r + 9) % 9][j], h));
+                const float2 sz = r == R ? z4[j][h]
+                                         : add2(pair_of(q[(u + 4 + r) % 8][j], h),
+                                                pair_of(q[(u + 4 - r) % 8][j], h));
                 lz[h] = fma2(mul2(mul2(c2[r], sz), iz2), one, lz[h]);
             }
         }
@@ -154,32 +178,34 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
     const int y0 = R + tile_y * TY;
     const int nint = ze - zb;          // interior planes this tile computes (>= 1)
     const int nplanes = nint + 2 * R;  // planes of p it reads (>= 9)
-    const uint32_t pb = ring.p;        // sequence number of plane 0
-    const uint32_t ab = ring.aux;      // sequence number of aux iteration 0
+    constexpr int Q = EXACT ? 8 : 9;  // register queue, and unroll of the plane loop
+    using RP = RingOf<S, Q>;
+    using RA = RingOf<NAUX, Q>;
+    const uint32_t pb = ring.p, ab = ring.aux;
 
     int issued_hi = -1;      // thread 0: highest p plane handed to TMA
     int aux_issued_hi = -1;  // thread 0: highest aux iteration handed to TMA
     auto issue_plane = [&](int j) {  // thread 0 only
-        const uint32_t s = (pb + j) % S;
+        const uint32_t s = RP::stage(pb, j);
         mbar_arrive_expect_tx(&full[s], P::PLANE_BYTES);
         tma_load_3d(sm + s * P::PLANE, pmap, &full[s], x0 - R, y0 - R, zb - R + j);
         issued_hi = j;
     };
     auto issue_aux = [&](int it) {  // thread 0 only
-        const uint32_t s = (ab + it) % NAUX;
+        const uint32_t s = RA::stage(ab, it);
         float* st = aux + s * 2 * P::TILE;
         mbar_arrive_expect_tx(&auxf[s], 2 * P::TILE_BYTES);
         tma_load_3d(st, qmap, &auxf[s], x0, y0, zb + it);
         tma_load_3d(st + P::TILE, vmap, &auxf[s], x0, y0, zb + it);
         aux_issued_hi = it;
     };
-    auto wait_plane = [&](int j) {
-        return mbar_wait(&full[(pb + j) % S], ((pb + j) / S) & 1);
+    auto wait_plane = [&](uint32_t j) {
+        return mbar_wait(&full[RP::stage(pb, j)], RP::parity(pb, j));
     };
-    auto wait_aux = [&](int it) {
-        return mbar_wait(&auxf[(ab + it) % NAUX], ((ab + it) / NAUX) & 1);
+    auto wait_aux = [&](uint32_t it) {
+        return mbar_wait(&auxf[RA::stage(ab, it)], RA::parity(ab, it));
     };
-    auto plane = [&](int j) -> const float* { return sm + ((pb + j) % S) * P::PLANE; };
+    auto plane = [&](uint32_t j) -> const float* { return sm + RP::stage(pb, j) * P::PLANE; };
 
     if (tid == 0) {
         prefetch_tmap(pmap);
@@ -220,7 +246,7 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
     const float2 cx2 = dup2(a.w.cx), cy2 = dup2(a.w.cy), cz2 = dup2(a.w.cz), neg1 = dup2(-1.f);
     const float2 one = dup2(a.one);  // EXACT: see ordered_lap
 
-    float4 q[9][RPT];
+    float4 q[Q][RPT];  // plane j in slot j % Q
     bool bad = false;
     // Start-up: planes 0..7 (z = zb-4 .. zb+3) fill queue slots 0..7; a ring shorter than
     // that takes the last of them into the stages that planes 0 and 1 leave.
@@ -244,12 +270,12 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
         for (int jj = S; jj < 8; ++jj) feed_start(jj);
     }
 
-    for (int i0 = 0; i0 < nint && !abort_run; i0 += 9) {
+    for (int i0 = 0; i0 < nint && !abort_run; i0 += Q) {
 #pragma unroll
-        for (int u = 0; u < 9; ++u) {
+        for (int u = 0; u < Q; ++u) {
             const int i = i0 + u;
             if (i < nint && !abort_run) {
-                const int cs = (u + 4) % 9;  // centre slot (plane z)
+                const int cs = (u + 4) % Q;  // centre slot (plane z)
                 // p_prev / vel2 of this plane (global-load variant).
                 float4 pv[RPT], vv[RPT];
                 if (!HEAT && !kAuxTma) {
@@ -261,19 +287,26 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
                         }
                     }
                 }
-                // Queue feed: plane z+4.
+                // Queue feed: plane z+4 (Q = 8: it meets plane z-4 and takes its slot).
+                float2 z4[RPT][2];
                 {
                     const int jf = i + 8;
                     if (!wait_plane(jf)) bad = true;
                     const float* pf = plane(jf) + soff;
 #pragma unroll
-                    for (int j = 0; j < RPT; ++j) q[(u + 8) % 9][j] = lds128(pf + j * P::SX);
+                    for (int j = 0; j < RPT; ++j) {
+                        const float4 f = lds128(pf + j * P::SX);
+                        if (Q == 8) {
+                            z4[j][0] = add2(pair_of(f, 0), pair_of(q[u][j], 0));
+                            z4[j][1] = add2(pair_of(f, 1), pair_of(q[u][j], 1));
+                        }
+                        q[(u + 8) % Q][j] = f;
+                    }
                 }
                 const float* pc = plane(i + 4) + soff;
-
                 float2 lap[RPT][2];
                 if constexpr (EXACT) {
-                    ordered_lap<RPT, P::SX>(q, u, pc, a, one, lap);
+                    ordered_lap<RPT, P::SX>(q, z4, u, pc, a, one, lap);
                 } else {
                     // y: neighbour rows outside the own block from shared memory, own
                     // rows from the queue centre, accumulated from zero in row order
@@ -346,7 +379,7 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
                 }
                 if (kAuxTma) {
                     if (!wait_aux(i)) bad = true;
-                    const float* st = aux + ((ab + i) % NAUX) * 2 * P::TILE + aoff;
+                    const float* st = aux + RA::stage(ab, i) * 2 * P::TILE + aoff;
 #pragma unroll
                     for (int j = 0; j < RPT; ++j) {
                         pv[j] = lds128(st + j * TX);
@@ -448,8 +481,8 @@ __device__ __forceinline__ bool pencil_tile(const CUtensorMap* pmap, const CUten
         }
         return false;
     }
-    ring.p = pb + nplanes;
-    if (kAuxTma) ring.aux = ab + nint;
+    ring.p = RP::after(pb, nplanes);
+    if (kAuxTma) ring.aux = RA::after(ab, nint);
     return true;
 }
 

@@ -19,16 +19,17 @@
 // are compile-time, and the 4 rows above and below serve 4 points.  Planes of p fill an
 // 8-stage ring, p_prev and vel2 tiles a 4-stage ring; plane z + 4 and the tiles of z are
 // one group on one mbarrier, 4 groups in flight, warp k issuing residue k.  The z
-// neighbours live in a 9-deep register queue (plane loop unrolled by 9); one CTA
-// barrier per plane.
+// neighbours live in an 8-deep register queue (the pair z - 4, z + 4 is added as plane
+// z + 4 takes plane z - 4's slot; plane loop unrolled by 8, so every stage and phase is
+// compile-time); one CTA barrier per plane.
 //
 // Why lanes are columns: a float4 of x per thread, as in the pencil kernel, would need
 // 16-byte aligned rows in shared memory; rows copied by 4-byte cp.async instead cost 97
 // instructions per point, half of them copies and addresses (245 us at 401 x 357 x 301).
-// Here 78 instructions and 13 words of shared memory per point.  Acoustic step measured,
-// against the one-thread-per-point kernel that ran before: 401 x 357 x 301 150 against
-// 318 us (its bytes at the copy rate: 98 us), 511^3 452 against 983 us; heat 401 x 357 x
-// 301 119 against 289 us.
+// Here 73 instructions and 14 words of shared memory per point (79 with a 9-deep queue
+// and stages computed from the plane's number).  Acoustic step measured, against the
+// one-thread-per-point kernel that ran before: 401 x 357 x 301 152 (9-deep queue: 161)
+// against 328 us (its bytes at the copy rate: 98 us).  Bound by issue and power.
 #include <algorithm>
 
 #include "kernels.h"
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(RaggedShape<TX, TY>::NT, 512 / RaggedShape<TX,
     };
     const uint32_t sh_step = uint32_t((((a.ny & 3) * (a.nx & 3)) & 3) * 4) * 0x01010101u;
 
-    float2 q[9][RPT / 2];
+    float2 q[8][RPT / 2];  // plane j of the chunk in slot j % 8
     bool bad = !mbar_wait(&start, 0);
     uint32_t sh = shifts(zb - R);
 #pragma unroll
@@ -208,48 +209,54 @@ __global__ void __launch_bounds__(RaggedShape<TX, TY>::NT, 512 / RaggedShape<TX,
     const float2 ix2 = dup2(a.inv_dx2), iy2 = dup2(a.inv_dy2), iz2 = dup2(a.inv_dz2);
     const float2 k2 = dup2(a.k), one = dup2(a.one), neg1 = dup2(-1.f);
     float* dst = a.next + int64_t(zb) * a.sz + int64_t(gy) * a.sy + gx;
-    for (int i0 = 0; i0 < nint && !abort_run; i0 += 9) {
+    const char* const pbase = reinterpret_cast<const char*>(sm) + poff;
+    const char* const abase = reinterpret_cast<const char*>(aux) + aoff;
+    for (int i0 = 0; i0 < nint && !abort_run; i0 += 8) {
 #pragma unroll
-        for (int u = 0; u < 9; ++u) {
+        for (int u = 0; u < 8; ++u) {
             const int i = i0 + u;
             if (i < nint && !abort_run) {
-                // This lane's column by residue: centre plane, own row group.
-                const char* cen = reinterpret_cast<const char*>(sm + ((i + 4) % RS) * PPLANE) + poff;
-                const int fed = i & 4 ? PPLANE * 16 : -PPLANE * 16;  // plane i + 8: stage i % 8
-                const char* st =
-                    reinterpret_cast<const char*>(aux + (i % RG) * 2 * ATILE) + aoff;
+                // This lane's column by residue.  The stages of the centre plane i + 4, of the
+                // fed plane i + 8 and of the aux tiles are compile-time offsets.
+                constexpr int kBytes = 4 * PPLANE;
+                const int cen = (u + 4) % RS * kBytes, fed = u * kBytes;
                 uint32_t s[4];
                 const char* pc[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     s[k] = __byte_perm(sh, 0, 0x4440 + k);
-                    pc[k] = cen + s[k];
+                    pc[k] = pbase + s[k];
                 }
                 sh = (sh + sh_step) & 0x0c0c0c0cu;
-                if (!mbar_wait(&full[i % RG], (i / RG) & 1)) bad = true;
+                if (!mbar_wait(&full[u % RG], u / RG)) bad = true;
+                // Plane z + 4 meets plane z - 4 and takes its slot.
+                float2 z4[RPT / 2];
 #pragma unroll
-                for (int h = 0; h < RPT / 2; ++h)
-                    q[(u + 8) % 9][h] =
-                        make_float2(lds_at(pc[2 * h] + fed, 4 * (2 * h) * PBLOCK),
-                                    lds_at(pc[2 * h + 1] + fed, 4 * (2 * h + 1) * PBLOCK));
+                for (int h = 0; h < RPT / 2; ++h) {
+                    const float2 f =
+                        make_float2(lds_at(pc[2 * h], fed + 4 * (2 * h) * PBLOCK),
+                                    lds_at(pc[2 * h + 1], fed + 4 * (2 * h + 1) * PBLOCK));
+                    z4[h] = add2(f, q[u][h]);
+                    q[u][h] = f;
+                }
                 // Row pairs (-4, -3) .. (6, 7): the own ones are the queue's centre.
                 float2 row[6];
 #pragma unroll
                 for (int m = 0; m < 6; ++m)
                     row[m] = m == 2 || m == 3
-                                 ? q[(u + 4) % 9][m - 2]
+                                 ? q[(u + 4) % 8][m - 2]
                                  : make_float2(lds_at(pc[2 * (m & 1)],
-                                                      4 * (2 * (m & 1) * PBLOCK + (m / 2 - 1) * PW)),
+                                                      cen + 4 * (2 * (m & 1) * PBLOCK + (m / 2 - 1) * PW)),
                                                lds_at(pc[2 * (m & 1) + 1],
-                                                      4 * ((2 * (m & 1) + 1) * PBLOCK +
-                                                           (m / 2 - 1) * PW)));
+                                                      cen + 4 * ((2 * (m & 1) + 1) * PBLOCK +
+                                                                 (m / 2 - 1) * PW)));
                 auto row_at = [&](int e) { return e & 1 ? row[e / 2].y : row[e / 2].x; };
                 float2 o[RPT / 2], kv[RPT / 2];
 #pragma unroll
                 for (int h = 0; h < RPT / 2; ++h) {
-                    const float2 c = q[(u + 4) % 9][h];
+                    const float2 c = q[(u + 4) % 8][h];
                     const int e = R + 2 * h;  // the pair's first row in row_at
-                    const int o0 = 4 * 2 * h * PBLOCK, o1 = 4 * (2 * h + 1) * PBLOCK;
+                    const int o0 = cen + 4 * 2 * h * PBLOCK, o1 = cen + 4 * (2 * h + 1) * PBLOCK;
                     auto x_at = [&](int d) {
                         return make_float2(lds_at(pc[2 * h], o0 + 4 * d),
                                            lds_at(pc[2 * h + 1], o1 + 4 * d));
@@ -263,7 +270,8 @@ __global__ void __launch_bounds__(RaggedShape<TX, TY>::NT, 512 / RaggedShape<TX,
                                                               row_at(e + 1 + r) + row_at(e + 1 - r))
                                                 : add2(row[(e + r) / 2], row[(e - r) / 2]);
                         l_y = fma2(mul2(mul2(c2[r], sy), iy2), one, l_y);
-                        const float2 sz = add2(q[(u + 4 + r) % 9][h], q[(u + 4 - r + 9) % 9][h]);
+                        const float2 sz =
+                            r == R ? z4[h] : add2(q[(u + 4 + r) % 8][h], q[(u + 4 - r) % 8][h]);
                         l_z = fma2(mul2(mul2(c2[r], sz), iz2), one, l_z);
                     }
                     const float2 lap = add2(add2(l_x, l_y), l_z);
@@ -271,9 +279,10 @@ __global__ void __launch_bounds__(RaggedShape<TX, TY>::NT, 512 / RaggedShape<TX,
                         // 2u - u is exact: the reference's heat arithmetic is u + k*lap
                         o[h] = fma2(mul2(k2, lap), one, c);
                     } else {
-                        const char* a0 = st + s[2 * h];
-                        const char* a1 = st + s[2 * h + 1];
-                        const int b0 = 4 * 2 * h * ABLOCK, b1 = 4 * (2 * h + 1) * ABLOCK;
+                        const char* a0 = abase + s[2 * h];
+                        const char* a1 = abase + s[2 * h + 1];
+                        const int st = u % RG * 2 * ATILE * 4;
+                        const int b0 = st + 4 * 2 * h * ABLOCK, b1 = st + 4 * (2 * h + 1) * ABLOCK;
                         kv[h] = mul2(k2, make_float2(lds_at(a0, b0 + 4 * ATILE),
                                                      lds_at(a1, b1 + 4 * ATILE)));
                         // 2c - p_prev in one rounding (2c is exact)

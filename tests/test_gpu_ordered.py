@@ -57,3 +57,34 @@ def test_steps_bit_for_bit(torch_cuda, shape):
         step(dev[0], out, g, 900.0)
         assert np.array_equal(out.cpu().numpy(), heat)
     assert sb.device_error() == 0
+
+
+@pytest.mark.parametrize("heat", [False, True], ids=["acoustic", "heat"])
+def test_every_tile_and_split_bit_for_bit(torch_cuda, heat):
+    """Each tile of the table in the reference order, over chunks of 67, 23, 9, 8 and 1
+    planes (a whole unroll of 8, one more, remainders, and less than the rings hold)."""
+    shape = (75, 90, 108)
+    nz, ny, nx = shape
+    d, dt = (10.0, 7.5, 12.0), np.float32(1e-3)
+    g = sb.Grid(nx, ny, nz, *d, float(dt))
+    cur, prev, vel2 = case(shape, 5)
+    dev = [torch_cuda.from_numpy(a).cuda() for a in (cur, prev, vel2)]
+    if heat:
+        k = np.full(shape, np.float32(900.0) * dt, np.float32)
+        ref = oracle.wave_step(cur, cur, k, *d, np.float32(1.0), out=prev.copy())
+    else:
+        ref = oracle.wave_step(cur, prev, vel2, *d, dt, out=prev.copy())
+    kind = sb.KIND_HEAT_F32 if heat else sb.KIND_WAVE_F32
+    try:
+        for v in range(len(sb.variant_names(kind))):
+            for zchunks in (1, 3, 8, 9, 67):
+                sb.set_pencil_override(kind, v, zchunks)
+                out = dev[1].clone()
+                if heat:
+                    sb.heat_step_exact(dev[0], out, g, 900.0)
+                else:
+                    sb.wave_step_exact(dev[0], out, dev[2], out, g)
+                assert np.array_equal(out.cpu().numpy(), ref), (v, zchunks)
+    finally:
+        sb.set_pencil_override(kind, -1, 1)
+    assert sb.device_error() == 0
