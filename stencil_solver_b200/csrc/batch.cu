@@ -319,9 +319,9 @@ public:
                 return rc;
             // on the batch's (non-blocking) stream, behind the unpack: a plain
             // cudaMemcpy would not wait for it
-            return cuda(download(bounce_, out, staging_, static_cast<size_t>(h.g.size()) * 4, st_));
+            return cuda(download(out, staging_, static_cast<size_t>(h.g.size()) * 4, st_));
         }
-        return cuda(download(bounce_, out, arena_ + h.off[step_ & 1],
+        return cuda(download(out, arena_ + h.off[step_ & 1],
                              static_cast<size_t>(h.g.size()) * 4, st_));
     }
 
@@ -754,7 +754,6 @@ private:
     int64_t scratch_len_ = 0;
     float* bound_ = nullptr;    // FP16: per-shot source bound per step (max_steps each)
     float* staging_ = nullptr;  // FP16: one shot's FP32 field
-    HostBounce bounce_;
     std::vector<std::vector<float>> wave_host_;
     std::vector<float> vel2_src_;
 

@@ -157,7 +157,7 @@ cudaError_t launch_leap2_f32(const PencilMaps& maps, float* out1, float* out2, c
 int pencil_f32_resident(bool heat, int v, bool exact = false);
 // Sets up every variant on the current device (before a stream capture, whose
 // launches must not be the first ones).
-void pencil_f32_prepare();
+void pencil_f32_prepare(bool heat, bool exact);
 void pencil_f16_prepare();
 // Number of CTAs a launch uses (for occupancy/wave reasoning in the tuner).
 int64_t pencil_f32_ctas(bool heat, int v, const GridDesc& g, int zchunks);
@@ -209,14 +209,8 @@ cudaError_t launch_field_stats(const void* field, bool half, const GridDesc& g, 
                                double* out3, double* scratch, cudaStream_t stream);
 
 // Copies bytes of device memory to the host behind the work on `st` and waits for it
-// (hostcopy.cpp); pageable destinations go through the handle's pinned buffers.
-struct HostBounce {
-    char* buf[2] = {nullptr, nullptr};
-    cudaEvent_t done[2] = {nullptr, nullptr};
-    ~HostBounce();
-    bool ready();
-};
-cudaError_t download(HostBounce& b, void* host, const void* dev, size_t bytes, cudaStream_t st);
+// (hostcopy.cpp); several threads take the page faults of a pageable destination.
+cudaError_t download(void* host, const void* dev, size_t bytes, cudaStream_t st);
 
 // Tensor maps (tmap.cpp).  Encodes (and caches) a 3-D tiled map over a
 // halo-inclusive field of element size esize bytes with the given box and copies

@@ -740,9 +740,8 @@ int pencil_f32_resident(bool heat, int v, bool exact) {
     return exact ? x.resident_exact() : x.resident();
 }
 
-void pencil_f32_prepare() {
-    for (const Variant& v : kWave) v.resident(), v.resident_exact();
-    for (const Variant& v : kHeat) v.resident(), v.resident_exact();
+void pencil_f32_prepare(bool heat, bool exact) {
+    for (int v = 0; v < (heat ? kNumHeat : kNumWave); ++v) pencil_f32_resident(heat, v, exact);
 }
 
 int64_t pencil_f32_ctas(bool heat, int v, const GridDesc& g, int zchunks) {
@@ -846,14 +845,16 @@ struct BatchVariant {
 #define SB200_BATCH_VARIANT(TX, TY, RPT, S, AUX, NAME) \
     BatchVariant { TX, TY, NAME, &launch_batch<TX, TY, RPT, S, AUX>, &resident_batch<TX, TY, RPT, S, AUX> }
 
-// b64x32_r2_s6_a2 (two CTAs, 16 warps per SM): 394 us per step of 16 uneven shots against
-// 401-408 (b32x16_r1_s8_a4) and 416 (b32x32_r2_s8_a4).  Not kept: 64 x 16 and 64 x 32 tiles
-// with 8 warps per SM (416, 428); 32 x 32, 64 x 16, 128 x 16 and 32 x 64 with the short rings
-// (400-410).
+// Short rings (6 planes, 2 aux stages) give the 64-wide tiles 16 warps per SM: per step of 16
+// uneven shots, before chunks shorten at the end, 394 us (b64x32_r2_s6_a2, two CTAs) and 410
+// (b64x16_r2_s6_a2) against 428 and 416 for the same tiles with 8-plane rings and 8 warps;
+// b32x16_r1_s8_a4 401-408, b32x32_r2_s8_a4 416.  Not kept: 32 x 32, 128 x 16 and 32 x 64 with
+// the short rings (400-404).
 const BatchVariant kBatch[] = {
     SB200_BATCH_VARIANT(32, 32, 2, 8, 4, "b32x32_r2_s8_a4"),
-    SB200_BATCH_VARIANT(64, 32, 2, 6, 2, "b64x32_r2_s6_a2"),
+    SB200_BATCH_VARIANT(64, 16, 2, 6, 2, "b64x16_r2_s6_a2"),
     SB200_BATCH_VARIANT(32, 16, 1, 8, 4, "b32x16_r1_s8_a4"),
+    SB200_BATCH_VARIANT(64, 32, 2, 6, 2, "b64x32_r2_s6_a2"),
 };
 constexpr int kNumBatch = sizeof(kBatch) / sizeof(kBatch[0]);
 

@@ -240,7 +240,7 @@ public:
     int get_field(float* host) {
         if (!host) return set_error(SB200_ERR_INVALID, "sb200_run_get_field: NULL destination");
         if (int rc = synchronize()) return rc;
-        if (!fp16_) return cuda(download(bounce_, host, a_, n_ * 4, st_));
+        if (!fp16_) return cuda(download(host, a_, n_ * 4, st_));
         F16Scale s;
         if (int rc = cuda(cudaMemcpy(&s, scale_dev_, sizeof(s), cudaMemcpyDeviceToHost))) return rc;
         if (int rc = ensure_stage()) return rc;
@@ -248,7 +248,7 @@ public:
             const int64_t m = std::min(kStageFloats, n_ - off);
             if (int rc = sb200_f16_unpack(static_cast<const uint16_t*>(a_) + off, stage_, m, s.a, st_))
                 return rc;
-            if (int rc = cuda(download(bounce_, host + off, stage_, m * 4, st_))) return rc;
+            if (int rc = cuda(download(host + off, stage_, m * 4, st_))) return rc;
         }
         return SB200_OK;
     }
@@ -528,10 +528,14 @@ private:
     int capture(cudaGraphExec_t* out) {
         const int C = c_.graph_chunk;
         // Everything a launch sets up on first use (kernel attributes, occupancy
-        // queries, the kernel choice, tensor maps) happens before the capture.
-        pencil_f32_prepare();
-        pencil_f16_prepare();
-        ragged_prepare();
+        // queries, the kernel choice, tensor maps) happens before the capture.  Only of the
+        // kernels this run can take: a kernel's first query also loads its code.
+        if (fp16_)
+            pencil_f16_prepare();
+        else if (c_.grid.nx % 4 == 0)
+            pencil_f32_prepare(heat_, c_.exact != 0);
+        else
+            ragged_prepare();
         int v = 0, z = 0;
         sb200_pencil_choice(heat_ ? SB200_KIND_HEAT_F32
                                   : (fp16_ ? SB200_KIND_WAVE_F16 : SB200_KIND_WAVE_F32),
@@ -578,7 +582,6 @@ private:
     int* monitor_dev_ = nullptr;
     F16Scale* scale_dev_ = nullptr;
     float* stage_ = nullptr;
-    HostBounce bounce_;
     cudaGraphExec_t graph_[2] = {nullptr, nullptr};
     void* home_ = nullptr;  // buffer that is current at even parity
     int64_t step_ = 0;

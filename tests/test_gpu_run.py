@@ -191,3 +191,21 @@ def test_fp16_initial_scale_from_the_fields(torch_cuda, shape, at, in_prev):
             with np.errstate(invalid="ignore"):
                 want = (p * np.float32(a)).astype(np.float16).astype(np.float32) / np.float32(a)
             assert np.array_equal(r.field(), want, equal_nan=True)
+
+
+@pytest.mark.parametrize("precision", [sb.PRECISION_F32, sb.PRECISION_F16], ids=["f32", "f16"])
+@pytest.mark.parametrize("shape", [(16, 256, 256), (17, 256, 256), (131, 139, 136)], ids=str)
+def test_fields_of_several_megabytes_to_any_memory(torch_cuda, shape, precision):
+    """4 MB (one direct copy), a little more, and several chunks with a remainder; into new
+    pages, into memory that starts inside a page, and into pinned memory."""
+    nz, ny, nx = shape
+    p = np.random.default_rng(3).integers(-9, 10, shape).astype(np.float32)  # exact in FP16
+    with sb.Run(sb.Grid(nx, ny, nz, 10, 10, 10, 1e-3), precision=precision) as r:
+        r.set_fields(p, p, np.full(shape, 2.25e6, np.float32))
+        assert np.array_equal(r.field(), p)
+        room = np.full(p.size + 12, 77.0, np.float32)
+        r.field(room[5:5 + p.size])
+        assert np.array_equal(room[5:5 + p.size].reshape(shape), p)
+        assert (room[:5] == 77).all() and (room[5 + p.size:] == 77).all()
+        pinned = torch_cuda.empty(shape).pin_memory()
+        assert np.array_equal(r.field(pinned).numpy(), p)
