@@ -98,7 +98,8 @@ cudaError_t launch_flags_compose(const uint8_t* in, uint8_t* out, const GridDesc
 // flags_in: per chunk, whether p may hold a value at or above the floor (NULL:
 // all may); box (x0, x1, y0, y1, z0, z1 cells, or NULL) counts as flagged;
 // flags_out receives the flags of p_next (NULL: none).
-cudaError_t launch_learned_step(const PencilMaps& maps, float* next, const GridDesc& g,
+cudaError_t launch_learned_step(const PencilMaps& maps, const float* p, float* next,
+                                const GridDesc& g,
                                 const LearnedNet& net, int sms, int* err, cudaStream_t stream,
                                 const uint8_t* flags_in = nullptr, uint8_t* flags_out = nullptr,
                                 const int64_t* box = nullptr);

@@ -5,11 +5,14 @@
 // correction kernel (sb200_wave_step_f32, then sb200_mlp_correct).  No
 // reference counterpart: the correction is this project's learned layer.
 //
-// Work unit: a CTA owns a 32 x 16 tile of interior columns and marches z, as the
-// FP32 pencil kernel does: planes of p (with the 4-cell halo) arrive by TMA in
-// a 6-stage ring, the p_prev / vel2 tiles in a 3-stage ring, z neighbours come
-// from a 9-deep register queue (shifted one slot per plane).  Each thread owns 4
-// consecutive x of one row.  Per plane:
+// Work unit: a CTA owns a 32 x 16 tile of interior columns and marches z.  The plane at
+// hand (with the 4-cell halo) arrives by TMA in a 3-stage ring, the p_prev / vel2 tiles in
+// a 2-stage ring.  Each thread owns 4 consecutive x of one row; its z neighbours are a
+// 9-deep register queue (shifted one slot per plane) that it feeds from global memory: a
+// ring that held planes z .. z+4 as the FP32 pencil kernel's does would take the shared
+// memory of the fourth CTA per SM (57 KB each), and a plane's chain of barriers, MMAs and
+// epilogues wants every warp it can get (260^3, active everywhere: 300 us with 3 CTAs and
+// 149 registers, 264 with 4 and 128; 388^3 918 and 866).  Per plane:
 //   1. the stencil (the pencil kernel's arithmetic and order) and the 26
 //      features of each of the thread's 4 points, in the correction kernel's
 //      arithmetic: the star's largest magnitude first, then the differences
@@ -33,7 +36,7 @@
 // chunk of p may hold a value at or above half the floor; the kernel writes the
 // same for p_next.  A CTA with no flagged chunk among its 26 neighbours can have no
 // active star and takes a plain path: the same stencil with the queue in
-// compile-time slots (unrolled by 9), 12-stage rings in the shared memory the
+// compile-time slots (unrolled by 9), 10-stage rings in the shared memory the
 // network would use, no TMEM -- after giving up the TMEM allocation permit, which
 // the SM otherwise waits on before it starts another CTA of this kernel.
 //
@@ -56,8 +59,7 @@ using namespace mlp;
 constexpr int LTX = 32, LTY = 16;  // tile of columns
 constexpr int LTPR = LTX / 4;      // threads per row (4 x each)
 constexpr int LNT = LTPR * LTY;    // 128 threads: one per A-tile row
-constexpr int LS = 6, LAUX = 3;    // staged planes of p; p_prev / vel2 stages
-static_assert(LS >= 6 && LS <= 8, "planes z..z+4 staged, plus one in flight");
+constexpr int LS = 3, LAUX = 2;    // staged centre planes of p; p_prev / vel2 stages
 constexpr int LSX = LTX + 2 * R, LSY = LTY + 2 * R;
 constexpr uint32_t LPLANE_BYTES = LSX * LSY * 4u;
 constexpr int LPLANE = int(((LPLANE_BYTES + 127u) / 128u) * 32u);  // stride, floats
@@ -65,19 +67,23 @@ constexpr uint32_t LTILE_BYTES = LTX * LTY * 4u;
 constexpr int LTILE = int(LTILE_BYTES / 4u);
 constexpr uint32_t kLCols = 128;  // TMEM: tile e's 32 accumulator columns at 32 e
 constexpr int kTileA = 128 * 64;  // one A tile: 128 rows x 32 BF16
-// Shared memory from a 1024-byte aligned base: A tiles, W1, W2, staged planes, aux.
+// Shared memory from a 128-byte aligned base: A tiles, W1, W2, staged planes, aux.
 constexpr int kOffW1 = 4 * kTileA, kOffW2 = kOffW1 + H * F * 2, kOffP = kOffW2 + H * H * 2;
 constexpr int kOffAux = kOffP + LS * LPLANE * 4;
-constexpr int kLSmem = kOffAux + LAUX * 2 * LTILE * 4 + 1024;
+constexpr int kLSmem = kOffAux + LAUX * 2 * LTILE * 4 + 128;
+static_assert(4 * (kLSmem + 1024 + 512) <= 228 * 1024, "4 CTAs per SM");
+static_assert(4 * kLCols <= 512, "and their TMEM columns");
 // The plain path of an idle chunk has no network: its rings take the whole
 // dynamic shared memory (PS staged planes, PAUX p_prev / vel2 stages), so the
 // short plain iterations still have PS - 4 planes of copy lead.
-constexpr int PS = 12, PAUX = 4;
+constexpr int PS = 10, PAUX = 4;
 constexpr int kOffPAux = PS * LPLANE * 4;
-static_assert(kOffPAux + PAUX * 2 * LTILE * 4 + 1024 <= kLSmem, "plain rings fit");
+static_assert(kOffPAux + PAUX * 2 * LTILE * 4 + 128 <= kLSmem, "plain rings fit");
 static_assert(LNT == 128, "one thread per TMEM lane of an M = 128 tile");
 
 struct LearnedArgs {
+    const float* p;
+    const float* p5;  // p, 5 planes on
     float* next;  // p_next, in place over p_prev (read through qmap)
     int nx, ny, nz;
     int64_t sy, sz;
@@ -315,7 +321,7 @@ __device__ __forceinline__ void plain_chunk(const CUtensorMap& pmap, const CUten
         a.flags_out[(int64_t(zc) * a.tiles_y + ty) * a.tiles_x + tx] = uint8_t(out_bits);
 }
 
-__global__ void __launch_bounds__(LNT, 3)
+__global__ void __launch_bounds__(LNT, 4)
     learned_step_kernel(const __grid_constant__ CUtensorMap pmap,
                         const __grid_constant__ CUtensorMap qmap,
                         const __grid_constant__ CUtensorMap vmap, const LearnedArgs a) {
@@ -327,7 +333,7 @@ __global__ void __launch_bounds__(LNT, 3)
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t s_tmem;
     __shared__ int s_flag;  // a bounded wait gave up
-    unsigned char* base = smem_align<1024>(dyn);
+    unsigned char* base = smem_align<128>(dyn);
     unsigned char* sA = base;
     unsigned char* sW1 = base + kOffW1;
     unsigned char* sW2 = base + kOffW2;
@@ -344,7 +350,7 @@ __global__ void __launch_bounds__(LNT, 3)
     const int x0 = R + tx * LTX, y0 = R + ty * LTY;
     const int zb = R + b * a.zlen;
     const int ze = min(zb + a.zlen, a.nz - R);
-    const int nint = ze - zb, nplanes = nint + 2 * R;
+    const int nint = ze - zb;
 
     // No star of this chunk can reach the floor when neither the chunk nor the
     // facing slab of a face neighbour is flagged: then the plain step is the
@@ -363,6 +369,11 @@ __global__ void __launch_bounds__(LNT, 3)
         *reinterpret_cast<uint16_t*>(sW1 + core_off(i / F, i % F)) = a.w1b[i];
         *reinterpret_cast<uint16_t*>(sW2 + core_off(i / H, i % H)) = a.w2b[i];
     }
+    // A tiles start zeroed: rows of points that never become active are read by
+    // the MMAs (their results are discarded) and must hold finite values.  Before the
+    // barrier below: a thread zeroes pieces of others' rows.
+    for (int i = tid; i < 4 * kTileA / 16; i += LNT)
+        reinterpret_cast<uint4*>(sA)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (tid == 0) {
         prefetch_tmap(&pmap);
         prefetch_tmap(&qmap);
@@ -397,11 +408,10 @@ __global__ void __launch_bounds__(LNT, 3)
                    dW1 = umma_desc(smem_u32(sW1)), dW2 = umma_desc(smem_u32(sW2));
 
     int issued_hi = -1, aux_issued_hi = -1;
-    auto plane = [&](int j) -> const float* { return sm + (j % LS) * LPLANE; };
-    auto issue_plane = [&](int j) {  // thread 0 only
-        mbar_arrive_expect_tx(&full[j % LS], LPLANE_BYTES);
-        tma_load_3d(sm + (j % LS) * LPLANE, &pmap, &full[j % LS], x0 - R, y0 - R, zb - R + j);
-        issued_hi = j;
+    auto issue_plane = [&](int it) {  // thread 0 only: the plane of iteration it, with halo
+        mbar_arrive_expect_tx(&full[it % LS], LPLANE_BYTES);
+        tma_load_3d(sm + (it % LS) * LPLANE, &pmap, &full[it % LS], x0 - R, y0 - R, zb + it);
+        issued_hi = it;
     };
     auto issue_aux = [&](int it) {  // thread 0 only
         float* st = aux + (it % LAUX) * 2 * LTILE;
@@ -411,7 +421,7 @@ __global__ void __launch_bounds__(LNT, 3)
         aux_issued_hi = it;
     };
     if (tid == 0) {
-        for (int s = 0; s < LS && s < nplanes; ++s) issue_plane(s);
+        for (int it = 0; it < LS && it < nint; ++it) issue_plane(it);
         for (int it = 0; it < LAUX && it < nint; ++it) issue_aux(it);
     }
 
@@ -419,34 +429,17 @@ __global__ void __launch_bounds__(LNT, 3)
     const bool rin = gx < a.nx - R && gy < a.ny - R;
     const int soff = (ly + R) * LSX + 4 * lx + R;
     const int aoff = ly * LTX + 4 * lx;
-    int64_t goff = static_cast<int64_t>(zb) * a.sz + static_cast<int64_t>(gy) * a.sy + gx;
+    // This thread's 4 points of plane z.  A column outside the grid reads its last one;
+    // nothing uses the values.
+    int64_t goff = static_cast<int64_t>(zb) * a.sz +
+                   static_cast<int64_t>(min(gy, a.ny - 1)) * a.sy + min(gx, a.nx - 4);
 
-
-    float4 q[9];  // planes z-4 .. z+4: slot k holds plane z - 4 + k
-    bool bad = false;
-    // Start-up: planes 0..5 are staged; 0..3 only feed the queue, so their stages
-    // take planes 6..9 at once; 4..7 stay staged as the first centre planes.
+    // z neighbours: planes z-4 .. z+4 (slot k: plane z - 4 + k), read from global memory.
+    // The staged planes are centre planes only, read 4 planes later and from L2.
+    float4 q[9];
 #pragma unroll
-    for (int jj = 0; jj < LS; ++jj) {
-        if (!mbar_wait(&full[jj], 0)) bad = true;
-        q[jj] = lds128(plane(jj) + soff);
-    }
-    bool abort_run = __syncthreads_or(bad) != 0;
-    if (!abort_run && tid == 0) {
-#pragma unroll
-        for (int jj = 0; jj < R; ++jj)
-            if (jj + LS < nplanes) issue_plane(jj + LS);
-    }
-#pragma unroll
-    for (int jj = LS; jj < 8; ++jj) {
-        if (!mbar_wait(&full[jj % LS], (jj / LS) & 1)) bad = true;
-        q[jj] = lds128(plane(jj) + soff);
-    }
-    // A tiles start zeroed: rows of points that never become active are read by
-    // the MMAs (their results are discarded) and must hold finite values.
-    for (int i = tid; i < 4 * kTileA / 16; i += LNT)
-        reinterpret_cast<uint4*>(sA)[i] = make_uint4(0u, 0u, 0u, 0u);
-    fence_async_smem();
+    for (int k = 0; k < 9; ++k) q[k] = ldg_stream(a.p + goff + (k - R) * a.sz);
+    bool bad = false, abort_run = false;
     uint32_t ncommit = 0;  // MMA commits issued (uniform): the mbarrier's phases
     uint32_t waited = 0;   // commits this thread has seen complete (phases complete in order)
     auto wait_mma = [&]() {  // the latest commit
@@ -460,12 +453,8 @@ __global__ void __launch_bounds__(LNT, 3)
     // One plane per iteration; the queue shifts by one slot at the end (the body
     // is too large to unroll 9 times and still fit the instruction cache).
     for (int i = 0; i < nint && !abort_run; ++i) {
-        {
-            const int jf = i + 8;  // queue feed: plane z + 4
-            if (!mbar_wait(&full[jf % LS], (jf / LS) & 1)) bad = true;
-            q[8] = lds128(plane(jf) + soff);
-        }
-        const float* pc = plane(i + 4) + soff;
+        if (!mbar_wait(&full[i % LS], (i / LS) & 1)) bad = true;
+        const float* pc = sm + (i % LS) * LPLANE + soff;
         const float4 c = q[4];
         const float4 lf = lds128(pc - 4);
         const float4 rt = lds128(pc + 4);
@@ -655,13 +644,14 @@ __global__ void __launch_bounds__(LNT, 3)
                 tc_mma(tacc, dA1, dW2 + 16, 1u);
                 tc_commit(&mbar);
             }
-            // The staged plane z and the aux stage of this plane are free now.
-            if (warp == 0 && i + 4 + LS < nplanes) issue_plane(i + 4 + LS);
+            // The stages of this plane are free now.
+            if (warp == 0 && i + LS < nint) issue_plane(i + LS);
             if (warp == 0 && i + LAUX < nint) issue_aux(i + LAUX);
         }
         if (!abort_run && any) ++ncommit;
 #pragma unroll
         for (int k = 0; k < 8; ++k) q[k] = q[k + 1];  // while layer 2 runs
+        if (i + 1 < nint) q[8] = ldg_stream(a.p5 + goff);
         if (run) {
             wait_mma();
             // Layer 2 epilogue and the output layer, in the correction kernel's
@@ -734,7 +724,7 @@ int learned_step_resident() {
     cudaGetDevice(&dev);
     if (cached[dev & 63] > 0) return cached[dev & 63];
     // From the kernel's registers and shared memory and the SM's budgets (the
-    // occupancy query answers 1 for this kernel, while 3 CTAs run per SM).
+    // occupancy query answers 1 for this kernel, while 4 CTAs run per SM).
     cudaFuncAttributes fa{};
     int regs_sm = 0, smem_sm = 0, reserved = 0;
     if (cudaFuncSetAttribute(learned_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -820,6 +810,10 @@ LearnedChunks learned_step_chunks(const GridDesc& g, int sms, bool flagged) {
     // 64 planes keep the network path near the activity (on the learned solve at
     // 516^3: 127 planes 107 ms, 64 planes 96 ms, 32 planes 99 ms, 16 planes 119
     // ms for 200 steps; shorter chunks re-read more halo planes).
+    // A grid that fits one wave takes as many chunks as there are slots, 3 planes or more
+    // each (128^3 45.8 us with 16 chunks, 42.1 with 18; 100^3 24.8 and 23.8 with 31; 64^3
+    // 13.5 and 12.8 with 19).
+    if (!flagged) zc = static_cast<int>(std::max<int64_t>(zc, std::min<int64_t>(slots / tiles, inz / 3)));
     if (flagged) zc = std::max(zc, (inz + 63) / 64);
     zc = std::min(zc, inz);
     c.zlen = (inz + zc - 1) / zc;
@@ -827,12 +821,15 @@ LearnedChunks learned_step_chunks(const GridDesc& g, int sms, bool flagged) {
     return c;
 }
 
-cudaError_t launch_learned_step(const PencilMaps& maps, float* next, const GridDesc& g,
+cudaError_t launch_learned_step(const PencilMaps& maps, const float* p, float* next,
+                                const GridDesc& g,
                                 const LearnedNet& net, int sms, int* err, cudaStream_t stream,
                                 const uint8_t* flags_in, uint8_t* flags_out, const int64_t* box) {
     if (!g.has_interior()) return cudaSuccess;
     const LearnedChunks ch = learned_step_chunks(g, sms, flags_in != nullptr || flags_out != nullptr);
     LearnedArgs a{};
+    a.p = p;
+    a.p5 = p + 5 * g.nx * g.ny;
     a.next = next;
     a.nx = static_cast<int>(g.nx);
     a.ny = static_cast<int>(g.ny);

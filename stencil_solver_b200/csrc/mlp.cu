@@ -1076,7 +1076,7 @@ int learned_step_impl(void* h, const float* p, float* p_prev_next, const float* 
     net.b3 = m->host[OFF_B3];
     net.out_scale = m->out_scale;
     net.min_scale = m->min_scale;
-    return cuda_err(launch_learned_step(maps, p_prev_next, g, net, m->sms, err, st, flags_in,
+    return cuda_err(launch_learned_step(maps, p, p_prev_next, g, net, m->sms, err, st, flags_in,
                                         flags_out, box),
                     where);
 }

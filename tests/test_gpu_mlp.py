@@ -462,3 +462,29 @@ def test_composed_flags_keep_the_bits(torch_cuda):
             assert torch.equal(a, b), float((a - b).abs().max())
         assert idle > 0
         assert sb.device_error() == 0
+
+
+@pytest.mark.parametrize("shape", [(72, 260, 260), (40, 68, 388), (13, 132, 132)], ids=str)
+def test_learned_step_bits_with_the_device_full(torch_cuda, shape):
+    """Several blocks per SM, chunks of a few planes (their first planes meet the start-up),
+    active everywhere, repeated: each run has the bits of step and correction."""
+    torch = torch_cuda
+    nz, ny, nx = shape
+    g = sb.Grid(nx, ny, nz, 10, 10, 10, 8e-4)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(11)
+    p, q = (torch.randn(shape, generator=gen, device="cuda") for _ in range(2))
+    v = torch.rand(shape, generator=gen, device="cuda") * 1.3e7 + 2.25e6
+    w, _, _ = net_and_rows(14, 1)
+    with sb.Mlp() as m:
+        m.set_params(w)
+        m.output_scale = 0.05
+        m.set_kernel("tcgen05")
+        ref = q.clone()
+        sb.wave_step(p, ref, v, ref, g)
+        m.correct(p, v, ref, g)
+        for _ in range(20):
+            out = q.clone()
+            m.learned_step(p, out, v, g)
+            assert torch.equal(out, ref)
+    assert sb.device_error() == 0
