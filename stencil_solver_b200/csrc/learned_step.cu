@@ -340,7 +340,9 @@ __global__ void __launch_bounds__(LNT, 4)
     float* sm = reinterpret_cast<float*>(base + kOffP);
     float* aux = reinterpret_cast<float*>(base + kOffAux);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // uniform to the compiler too: TMEM addresses
+                                                             // stay in uniform registers (267 -> 263 us)
     const int lx = tid % LTPR, ly = tid / LTPR;
     int b = blockIdx.x;
     const int tx = b % a.tiles_x;
