@@ -6,8 +6,9 @@
 // (each rounded up to 256 bytes); per parity, a table of shot descriptors
 // (TMA maps + sweep arguments) tells the kernel which level is current.  The
 // work list is every shot's (tile x, tile y, z chunk) triple, shots in order of
-// decreasing size so the largest pieces are handed out first; CTAs pull items
-// from a device counter until the list is empty (batch_f32_kernel).  The
+// decreasing size so the largest pieces are handed out first, and chunks that
+// shorten towards the end of the list; CTAs pull items from a device counter
+// until the list is empty (batch_f32_kernel).  The
 // kernel's last CTA resets the counter and advances the shared step index that
 // selects each shot's source sample and trace slot, so chunks of steps replay
 // from captured CUDA graphs with no host work between steps.
