@@ -956,7 +956,12 @@ int sb200_mlp_train_step(void* h, const uint16_t* X, const float* t, int64_t n, 
     if (!(lr > 0.f)) return set_error(SB200_ERR_INVALID, std::string(where) + ": lr must be positive");
     if (!X || !t || n <= 0) return set_error(SB200_ERR_INVALID, std::string(where) + ": bad arguments");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!m->grad_zero)
+    // A captured step runs later, any number of times and between any others: it brings its
+    // own zeroing, and what it leaves is not known here.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (int rc = cuda_err(cudaStreamIsCapturing(st, &capture), where)) return rc;
+    const bool captured = capture != cudaStreamCaptureStatusNone;
+    if (captured || !m->grad_zero)
         if (int rc = cuda_err(cudaMemsetAsync(m->grad, 0, NSLOT * 4, st), where)) return rc;
     m->grad_zero = false;  // until the update that zeroes it again is on its way
     if (int rc = launch_grad(*m, X, t, n, m->grad, st, where)) return rc;
@@ -968,7 +973,7 @@ int sb200_mlp_train_step(void* h, const uint16_t* X, const float* t, int64_t n, 
                                          m->m2, m->grad, lr, b1, b2, 1e-8f, c1, c2, m->w1b, m->w2b,
                                          m->w2tb, loss),
                             where);
-    m->grad_zero = !rc;
+    m->grad_zero = !rc && !captured;
     return rc;
 }
 

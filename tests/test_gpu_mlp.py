@@ -488,3 +488,28 @@ def test_learned_step_bits_with_the_device_full(torch_cuda, shape):
             m.learned_step(p, out, v, g)
             assert torch.equal(out, ref)
     assert sb.device_error() == 0
+
+
+def test_a_captured_training_step_zeroes_its_own_gradient(torch_cuda):
+    """Capture a handle's first step, take an eager one before any replay, replay twice:
+    every loss is the oracle's at the parameters the step started from (tolerance:
+    test_gradients_match_oracle's)."""
+    torch = torch_cuda
+    w, X, t = net_and_rows(8, 1000)
+    Xd, td = dev(torch, X.view(np.int16)), dev(torch, t)
+    loss = torch.zeros(1, device="cuda")
+    with sb.Mlp() as m:
+        m.set_params(w)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            m.train_step(Xd, td, 1e-3, loss, stream=torch.cuda.current_stream().cuda_stream)
+        eager = lambda: m.train_step(Xd, td, 1e-3, loss)
+        for step in (eager, graph.replay, graph.replay, eager, eager):
+            before = m.params()
+            torch.cuda.synchronize()
+            step()
+            torch.cuda.synchronize()
+            want, _ = oracle.mlp_grad(before, X, t, round_bf16=True)
+            assert abs(float(loss) - want) <= 1e-4 * want
+            assert np.any(m.params() != before)
