@@ -278,10 +278,12 @@ PencilConfig choose(int kind, const GridDesc& g) {
     return c;
 }
 
-// Grids whose reference-order steps stay on the one-thread-per-point kernel: a staged
-// sweep first fills its rings (64^3 acoustic: 5.2 us against 6.2 aligned and 6.6 ragged;
-// 88^3 8.2 against 8.2; 96^3 9.7 against 8.2; 128^3 17.3 against 12.3).
-constexpr int64_t kNaivePoints = int64_t(1) << 19;
+// Interior points from which reference-order steps run on staged planes; below, the
+// one-thread-per-point kernel, which fills no rings first.  Acoustic step in a graph, one
+// thread per point against staged, us: aligned 64^3 3.1 and 3.8, 72^3 3.5 and 4.0, 80^3 5.5
+// and 4.7, 88^3 6.3 and 4.8; ragged 72^3 4.6 and 4.5, 80^3 5.4 and 5.8, 88^3 6.3 and 5.8
+// (heat crosses at the same sizes).
+constexpr int64_t kPencilPoints = int64_t(5) << 16, kRaggedPoints = int64_t(7) << 16;
 
 bool pencil_ok(const GridDesc& g, std::initializer_list<const void*> ptrs) {
     if (g.nx % 4 != 0) return false;
@@ -345,8 +347,7 @@ int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_n
         return fail(SB200_ERR_INVALID, std::string(where) + ": source index outside the grid");
     if (!g.has_interior()) return SB200_OK;  // no interior point: nothing to update
     auto st = static_cast<cudaStream_t>(stream);
-    const bool staged = g.interior() >= kNaivePoints;
-    if ((staged || !exact) && pencil_ok(g, {p, p_prev, vel2, p_next})) {
+    if ((g.interior() >= kPencilPoints || !exact) && pencil_ok(g, {p, p_prev, vel2, p_next})) {
         const PencilConfig cfg = choose(exact ? int(kExactWave) : int(SB200_KIND_WAVE_F32), g);
         PencilMaps maps;
         if (int rc = pencil_maps(false, cfg.variant, g, p, p_prev, vel2, &maps, where)) return rc;
@@ -354,7 +355,7 @@ int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_n
                                                     device_error_ptr(), st, exact),
                              where);
     }
-    if (staged && ragged_ok(g) && aligned16(p) && aligned16(p_prev) && aligned16(vel2)) {
+    if (g.interior() >= kRaggedPoints && ragged_ok(g) && aligned16(p) && aligned16(p_prev) && aligned16(vel2)) {
         PencilMaps maps;
         if (int rc = ragged_maps(false, g, p, p_prev, vel2, &maps, where)) return rc;
         return finish_launch(launch_wave_ragged_f32(maps, p_next, g, src,
@@ -369,15 +370,14 @@ int heat_step(const float* u, float* u_next, const GridDesc& g, float alpha_dt, 
               bool exact, const char* where) {
     auto st = static_cast<cudaStream_t>(stream);
     PencilMaps maps;
-    const bool staged = g.interior() >= kNaivePoints;
-    if ((staged || !exact) && pencil_ok(g, {u, u_next})) {
+    if ((g.interior() >= kPencilPoints || !exact) && pencil_ok(g, {u, u_next})) {
         const PencilConfig cfg = choose(exact ? int(kExactHeat) : int(SB200_KIND_HEAT_F32), g);
         if (int rc = pencil_maps(true, cfg.variant, g, u, nullptr, nullptr, &maps, where)) return rc;
         return finish_launch(launch_heat_pencil_f32(maps, u_next, g, alpha_dt, cfg,
                                                     device_error_ptr(), st, exact),
                              where);
     }
-    if (staged && ragged_ok(g) && aligned16(u)) {
+    if (g.interior() >= kRaggedPoints && ragged_ok(g) && aligned16(u)) {
         if (int rc = ragged_maps(true, g, u, nullptr, nullptr, &maps, where)) return rc;
         return finish_launch(launch_heat_ragged_f32(maps, u_next, g, alpha_dt,
                                                     choose(kRaggedHeat, g).zchunks,

@@ -4,8 +4,8 @@
 // in exactly the order of its CPU branch (stencil_naive.cu:151-169): every product and sum
 // goes through __fmul_rn / __fadd_rn, so nvcc cannot contract them into FMAs and the
 // result is bit-identical to the oracle's FP32 restatement built with -ffp-contract=off.
-// They serve the reference-order steps of grids below 2^19 interior points and of fields
-// whose base is not 16-byte aligned (larger grids: pencil_f32.cu in that order, and
+// They serve the reference-order steps of grids below 5 (nx % 4 != 0: 7) times 2^16
+// interior points and of fields whose base is not 16-byte aligned (larger grids: pencil_f32.cu in that order, and
 // ragged_f32.cu where nx % 4 != 0).
 #include "kernels.h"
 #include "sb200_common.cuh"

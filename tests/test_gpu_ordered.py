@@ -1,6 +1,6 @@
-"""Reference-order steps on the kernels that stage planes by TMA (2^19 interior points
-and more): grids of any row length (rows as lines of four), and the pencil tiles in
-that order on aligned grids; below, the one-thread-per-point kernel.  Bit for bit the
+"""Reference-order steps on the kernels that stage planes by TMA (5 x 2^16 interior points
+and more, 7 x 2^16 where rows are ragged): grids of any row length (rows as lines of
+four), and the pencil tiles in that order on aligned grids; below, the one-thread-per-point kernel.  Bit for bit the
 oracle, halos (and everything outside the interior) untouched."""
 from __future__ import annotations
 
@@ -14,12 +14,13 @@ pytestmark = pytest.mark.gpu
 
 # (nz, ny, nx): one interior plane and column-thin grids; rows of every residue modulo
 # 4 words and planes of every residue; one below, at and above both ragged tiles
-# (64 x 16, 32 x 32); the last size of the one-thread-per-point kernel and the first
-# staged one
+# (64 x 16, 32 x 32); the last sizes of the one-thread-per-point kernel and the first
+# staged ones
 RAGGED = [(9, 733, 741), (10, 520, 521), (2060, 9, 265), (900, 603, 9), (137, 72, 71),
           (133, 72, 73), (71, 137, 74), (75, 90, 105), (41, 250, 73), (12, 23, 41),
-          (9, 9, 9), (88, 88, 89), (89, 89, 89)]
-ALIGNED = [(9, 733, 740), (133, 72, 72), (75, 90, 108), (12, 24, 40), (2060, 9, 264)]
+          (9, 9, 9), (88, 88, 89), (89, 89, 89), (85, 85, 85), (85, 85, 86)]
+ALIGNED = [(9, 733, 740), (133, 72, 72), (75, 90, 108), (12, 24, 40), (2060, 9, 264), (76, 76, 76),
+           (76, 76, 80)]
 
 
 def case(shape, seed):
