@@ -147,14 +147,16 @@ struct Leap2Math {
         const float2 o1 = fma2(pair_of(vv, 1), lap[1], t1);
         return make_float4(o0.x, o0.y, o1.x, o1.y);
     }
-    // element e of o += (dt2 vel2[e]) * w, rounded as the one-step kernel rounds it
+    // element e of o += (dt2 vel2[e]) * w in the one-step kernel's roundings: the product
+    // joins the sum in one explicit fma (o + kv * w is contracted or not as the compiler
+    // likes, lane by lane)
     __device__ __forceinline__ static void add_source(float4& o, const float4& vv, float dt2,
                                                       float w, int e) {
-        const float add = (dt2 * f4get(vv, e)) * w;
-        if (e == 0) o.x = o.x + add;
-        if (e == 1) o.y = o.y + add;
-        if (e == 2) o.z = o.z + add;
-        if (e == 3) o.w = o.w + add;
+        const float kv = dt2 * f4get(vv, e);
+        if (e == 0) o.x = fmaf(kv, w, o.x);
+        if (e == 1) o.y = fmaf(kv, w, o.y);
+        if (e == 2) o.z = fmaf(kv, w, o.z);
+        if (e == 3) o.w = fmaf(kv, w, o.w);
     }
 };
 

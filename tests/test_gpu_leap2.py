@@ -118,3 +118,26 @@ def test_argument_checks(torch_cuda):
     with pytest.raises(sb.StencilError) as e:
         sb.wave_step2(*z, g2)
     assert e.value.status == sb.SB200_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("lane", range(4))
+@pytest.mark.parametrize("variant", range(len(sb.variant_names(sb.KIND_WAVE2_F32))))
+def test_source_rounds_alike_at_every_column(torch_cuda, variant, lane):
+    """The source's product meets the update in one rounding, in both steps, whichever
+    of a thread's four columns holds it: eight cells and sample pairs per column (two
+    roundings differ from one in about half of them)."""
+    g = sb.Grid(76, 45, 37, 10.0, 10.0, 10.0, 7e-4)
+    p, q, v = fields(torch_cuda, g, 40 + lane)
+    rng = np.random.default_rng(lane)
+    sb.set_pencil_override(sb.KIND_WAVE2_F32, variant, 2)
+    try:
+        for k in range(8):
+            # the tile's inside, its ring beside a neighbour, and beyond the first tile
+            src = g.index(4 + lane + 8 * k, 5 + 4 * k, 6 + 3 * k)
+            w0, w1 = (float(w) for w in rng.uniform(-1.0, 1.0, 2).astype(np.float32))
+            o1, o2 = torch_cuda.zeros_like(p), torch_cuda.zeros_like(p)
+            sb.wave_step2(p, q, v, o1, o2, g, src, w0, w1)
+            r1, r2 = one_step_pair(torch_cuda, p, q, v, g, src, w0, w1)
+            assert torch_cuda.equal(o1, r1) and torch_cuda.equal(o2, r2), (k, src)
+    finally:
+        sb.set_pencil_override(sb.KIND_WAVE2_F32, -1, 1)
