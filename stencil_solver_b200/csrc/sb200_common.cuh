@@ -70,7 +70,10 @@ cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+    // the caller reports e: nothing is left for a later launch's check to find
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

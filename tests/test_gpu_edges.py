@@ -125,3 +125,16 @@ def test_two_step_thin_grids(torch_cuda, shape, variant, zchunks):
     sb.wave_step(a, b, v, b, g, src, -0.25)
     torch_cuda.cuda.synchronize()
     assert torch_cuda.equal(o1, a) and torch_cuda.equal(o2, b)
+
+
+def test_a_refused_launch_leaves_no_error_behind(torch_cuda):
+    """A grid taller than a launch may be (z blocks of two planes, at most 65535 of them)
+    is refused on the host; the calls after it do not report that error again."""
+    g = sb.Grid(9, 9, 2 * 65535 + 9 + 8, 10.0, 10.0, 10.0, 1e-3)
+    p, q, v = (torch_cuda.zeros(g.shape, device="cuda") for _ in range(3))
+    with pytest.raises(sb.StencilError) as e:
+        sb.wave_step_exact(p, q, v, q, g)
+    assert e.value.status == sb.SB200_ERR_CUDA
+    h = torch_cuda.zeros(64, dtype=torch_cuda.int16, device="cuda")
+    sb.f16_pack(torch_cuda.ones(64, device="cuda"), h, 64, 2.0)
+    assert (h.view(torch_cuda.float16).cpu() == 2).all()
