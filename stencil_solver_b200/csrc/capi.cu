@@ -285,6 +285,23 @@ PencilConfig choose(int kind, const GridDesc& g) {
 // (heat crosses at the same sizes).
 constexpr int64_t kPencilPoints = int64_t(5) << 16, kRaggedPoints = int64_t(7) << 16;
 
+// Whether reference-order steps of a grid are worth staging: enough points, and not too few
+// rows for the tiles.  The staged kernels compute whole tiles of at least 16 rows, the
+// one-thread-per-point kernel rows of 32 columns; a point of the latter costs about 3
+// (ragged rows; from 3.0 on) or 3.5 of the former.  Acoustic step, one thread per point
+// against staged, us: 264 columns of 3000 - 8 planes with 4 rows (4 tile points to one) 26.7
+// and 35.2, 5 rows (3.2) 36.9 and 35.3, 6 rows 42.4 and 35.4; 265 columns (ragged; 3.6 and
+// 3.0 to one) with 5 rows 41.0 and 45.8, with 6 47.1 and 45.9.  A single row took up to 4.6
+// times as long staged (73 x 9 x 20000: 24.7 and 114).  Grids too tall for a launch of the
+// one-thread-per-point kernel are staged all the same.
+bool staged_pays(const GridDesc& g, bool ragged) {
+    if (g.interior() < (ragged ? kRaggedPoints : kPencilPoints)) return false;
+    if (!naive_fits(g)) return true;
+    const int64_t lanes = (g.nx - 8 + 31) / 32 * 32, rows = g.ny - 8;
+    return ragged ? ragged_covered(g) <= 3 * lanes * rows
+                  : 2 * ((rows + 15) / 16 * 16) <= 7 * rows;
+}
+
 bool pencil_ok(const GridDesc& g, std::initializer_list<const void*> ptrs) {
     if (g.nx % 4 != 0) return false;
     for (const void* p : ptrs)
@@ -347,7 +364,7 @@ int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_n
         return fail(SB200_ERR_INVALID, std::string(where) + ": source index outside the grid");
     if (!g.has_interior()) return SB200_OK;  // no interior point: nothing to update
     auto st = static_cast<cudaStream_t>(stream);
-    if ((g.interior() >= kPencilPoints || !exact) && pencil_ok(g, {p, p_prev, vel2, p_next})) {
+    if ((!exact || staged_pays(g, false)) && pencil_ok(g, {p, p_prev, vel2, p_next})) {
         const PencilConfig cfg = choose(exact ? int(kExactWave) : int(SB200_KIND_WAVE_F32), g);
         PencilMaps maps;
         if (int rc = pencil_maps(false, cfg.variant, g, p, p_prev, vel2, &maps, where)) return rc;
@@ -355,7 +372,7 @@ int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_n
                                                     device_error_ptr(), st, exact),
                              where);
     }
-    if (g.interior() >= kRaggedPoints && ragged_ok(g) && aligned16(p) && aligned16(p_prev) && aligned16(vel2)) {
+    if (staged_pays(g, true) && ragged_ok(g) && aligned16(p) && aligned16(p_prev) && aligned16(vel2)) {
         PencilMaps maps;
         if (int rc = ragged_maps(false, g, p, p_prev, vel2, &maps, where)) return rc;
         return finish_launch(launch_wave_ragged_f32(maps, p_next, g, src,
@@ -370,14 +387,14 @@ int heat_step(const float* u, float* u_next, const GridDesc& g, float alpha_dt, 
               bool exact, const char* where) {
     auto st = static_cast<cudaStream_t>(stream);
     PencilMaps maps;
-    if ((g.interior() >= kPencilPoints || !exact) && pencil_ok(g, {u, u_next})) {
+    if ((!exact || staged_pays(g, false)) && pencil_ok(g, {u, u_next})) {
         const PencilConfig cfg = choose(exact ? int(kExactHeat) : int(SB200_KIND_HEAT_F32), g);
         if (int rc = pencil_maps(true, cfg.variant, g, u, nullptr, nullptr, &maps, where)) return rc;
         return finish_launch(launch_heat_pencil_f32(maps, u_next, g, alpha_dt, cfg,
                                                     device_error_ptr(), st, exact),
                              where);
     }
-    if (g.interior() >= kRaggedPoints && ragged_ok(g) && aligned16(u)) {
+    if (staged_pays(g, true) && ragged_ok(g) && aligned16(u)) {
         if (int rc = ragged_maps(true, g, u, nullptr, nullptr, &maps, where)) return rc;
         return finish_launch(launch_heat_ragged_f32(maps, u_next, g, alpha_dt,
                                                     choose(kRaggedHeat, g).zchunks,

@@ -42,6 +42,8 @@ struct SourceDesc {
     float* trace = nullptr;
 };
 
+// Whether a grid's blocks fit a launch of the one-thread-per-point kernel.
+bool naive_fits(const GridDesc& g);
 cudaError_t launch_wave_naive(const float* cur, const float* prev, const float* vel2,
                               float* next, const GridDesc& g, const SourceDesc& src,
                               cudaStream_t stream);
@@ -127,6 +129,8 @@ cudaError_t launch_prepass_pencil_f32(const PencilMaps& maps, float* prev, const
 // ragged_ok(g), 16-byte aligned p (u), p_prev and vel2 (maps: tensor_map_rows4 with
 // ragged_boxes), has_interior().  next may alias p_prev.
 bool ragged_ok(const GridDesc& g);
+// Points of a plane that the kernel's tiles cover.
+int64_t ragged_covered(const GridDesc& g);
 PencilBoxes ragged_boxes(bool heat, const GridDesc& g);
 int ragged_resident(bool heat, const GridDesc& g);
 void ragged_prepare();

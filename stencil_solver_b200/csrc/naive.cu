@@ -5,8 +5,8 @@
 // goes through __fmul_rn / __fadd_rn, so nvcc cannot contract them into FMAs and the
 // result is bit-identical to the oracle's FP32 restatement built with -ffp-contract=off.
 // They serve the reference-order steps of grids below 5 (nx % 4 != 0: 7) times 2^16
-// interior points and of fields whose base is not 16-byte aligned (larger grids: pencil_f32.cu in that order, and
-// ragged_f32.cu where nx % 4 != 0).
+// interior points, of grids with few rows, and of fields whose base is not 16-byte aligned
+// (the others: pencil_f32.cu in that order, and ragged_f32.cu where nx % 4 != 0).
 #include "kernels.h"
 #include "sb200_common.cuh"
 
@@ -101,14 +101,21 @@ dim3 naive_grid(const GridDesc& g, dim3 block) {
                 static_cast<unsigned>((iz + block.z - 1) / block.z));
 }
 
+constexpr unsigned kBlockX = 32, kBlockY = 4, kBlockZ = 2;
+
 }  // namespace
+
+bool naive_fits(const GridDesc& g) {
+    const dim3 n = naive_grid(g, dim3(kBlockX, kBlockY, kBlockZ));
+    return n.y <= 65535 && n.z <= 65535;
+}
 
 cudaError_t launch_wave_naive(const float* cur, const float* prev, const float* vel2,
                               float* next, const GridDesc& g, const SourceDesc& src,
                               cudaStream_t stream) {
     if (!g.has_interior()) return cudaSuccess;
     const float dt2 = g.dt * g.dt;
-    const dim3 block(32, 4, 2);
+    const dim3 block(kBlockX, kBlockY, kBlockZ);
     NaiveArgs a = make_args(cur, prev, vel2, next, g, dt2, src.idx, src.w);
     a.wavelet = src.wavelet;
     a.step = src.step;
@@ -131,7 +138,7 @@ cudaError_t launch_set_int(int* dst, int value, cudaStream_t stream) {
 cudaError_t launch_heat_naive(const float* u, float* u_next, const GridDesc& g, float alpha_dt,
                               cudaStream_t stream) {
     if (!g.has_interior()) return cudaSuccess;
-    const dim3 block(32, 4, 2);
+    const dim3 block(kBlockX, kBlockY, kBlockZ);
     return launch_after(naive_kernel<true>, naive_grid(g, block), block, 0, stream,
                         make_args(u, nullptr, nullptr, u_next, g, alpha_dt, -1, 0.0f));
 }

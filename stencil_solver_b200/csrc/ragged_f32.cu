@@ -371,15 +371,17 @@ constexpr Shape shape_of() {
 
 const Shape kShapes[] = {shape_of<64, 16>(), shape_of<32, 32>()};
 
+// Points of a plane that a shape's tiles cover.
+int64_t covered(const Shape& s, const GridDesc& g) {
+    const int64_t x = (g.nx - 2 * R + s.tx - 1) / s.tx, y = (g.ny - 2 * R + s.ty - 1) / s.ty;
+    return x * s.tx * y * s.ty;
+}
+
 // The shape whose tiles cover fewer points outside the interior; where they cover the
 // same, the wider one (acoustic: 401 x 357 x 301 covers 448 or 416 columns and runs 156
 // or 150 us; 383^3 covers the same points and runs 195 or 198 us).
 const Shape& shape_for(const GridDesc& g) {
-    auto covered = [&](const Shape& s) {
-        const int64_t x = (g.nx - 2 * R + s.tx - 1) / s.tx, y = (g.ny - 2 * R + s.ty - 1) / s.ty;
-        return x * s.tx * y * s.ty;
-    };
-    return covered(kShapes[1]) < covered(kShapes[0]) ? kShapes[1] : kShapes[0];
+    return covered(kShapes[1], g) < covered(kShapes[0], g) ? kShapes[1] : kShapes[0];
 }
 
 RaggedArgs make_args(float* next, const GridDesc& g, float k, int zchunks, int* err) {
@@ -420,6 +422,8 @@ unsigned ctas_of(const RaggedArgs& a, const GridDesc& g) {
 bool ragged_ok(const GridDesc& g) {
     return g.nx < (int64_t(1) << 28) && g.ny * g.nz < (int64_t(1) << 30) && g.ny * g.nz >= 4;
 }
+
+int64_t ragged_covered(const GridDesc& g) { return covered(shape_for(g), g); }
 
 PencilBoxes ragged_boxes(bool heat, const GridDesc& g) {
     const Shape& s = shape_for(g);

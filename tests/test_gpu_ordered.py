@@ -89,3 +89,41 @@ def test_every_tile_and_split_bit_for_bit(torch_cuda, heat):
     finally:
         sb.set_pencil_override(kind, -1, 1)
     assert sb.device_error() == 0
+
+
+# rows on both sides of the line between one thread per point and staged planes (aligned:
+# 4 and 5 rows; ragged, by covered columns: 5 and 6 rows of 257, 7 and 8 of 65), a single
+# row, and the grids too tall for the former's launch
+THIN = [(2060, 12, 264), (2060, 13, 264), (2060, 13, 265), (2060, 14, 265), (1900, 15, 73),
+        (1900, 16, 73), (5000, 9, 265), (131090, 9, 40), (131090, 9, 41)]
+
+
+@pytest.mark.parametrize("shape", THIN, ids=str)
+def test_grids_of_few_rows_bit_for_bit(torch_cuda, shape):
+    test_steps_bit_for_bit(torch_cuda, shape)
+
+
+@pytest.mark.parametrize("shape", [(5000, 9, 264), (5000, 9, 265), (12000, 12, 73)], ids=str)
+def test_few_rows_take_no_longer_than_one_thread_per_point(torch_cuda, shape):
+    """Fields off a 16-byte boundary always run one thread per point: steps of the same
+    grid from aligned fields (which tiles of 16 rows would make 1.8 to 4.6 times as
+    long) take no more than 1.4 times theirs."""
+    nz, ny, nx = shape
+    g = sb.Grid(nx, ny, nz, 10.0, 7.5, 12.0, 1e-3)
+    n = nx * ny * nz
+
+    def step_us(offset):
+        p, q, v = (torch_cuda.zeros(n + 4, device="cuda")[offset:offset + n].view(shape)
+                   for _ in range(3))
+        e0, e1 = (torch_cuda.cuda.Event(enable_timing=True) for _ in range(2))
+        best = float("inf")
+        for _ in range(6):
+            e0.record()
+            for _ in range(50):
+                sb.wave_step_exact(p, q, v, q, g)
+            e1.record()
+            e1.synchronize()
+            best = min(best, e0.elapsed_time(e1) * 20.0)
+        return best
+
+    assert step_us(0) <= 1.4 * step_us(1)
