@@ -6,12 +6,15 @@
 // Here several threads touch the destination a chunk ahead of the copy: 5.2 ms and 12.5 ms
 // with chunks of 16 MB (4 MB: 5.5 and 20).  Nothing outlives the call; pinned buffers of
 // the library's own and as many copying threads took 3.5 ms, but pinning them first took
-// 2 to 9 ms.
+// 2 to 9 ms.  A destination whose pages are in place is copied to in one call: starting
+// the threads for it cost 0.2 ms and the chunks 1 to 10 % (5.6 MB 0.53 instead of 0.37 ms).
 #include <cuda_runtime.h>
 #include <sched.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <atomic>
+#include <cstdint>
 #include <memory>
 #include <thread>
 #include <vector>
@@ -33,6 +36,19 @@ bool pageable(const void* p) {
         return false;
     }
     return a.type == cudaMemoryTypeUnregistered;
+}
+
+// Whether the pages of [p, p + n) are in place, judged by 16 of them.  (A new page
+// among the others costs its fault, nothing else.)
+bool in_place(const char* p, size_t n) {
+    const uintptr_t first = reinterpret_cast<uintptr_t>(p) & ~(kPage - 1);
+    const size_t last = (reinterpret_cast<uintptr_t>(p) + n - 1 - first) / kPage;
+    for (size_t k = 0; k < 16; ++k) {
+        unsigned char in = 0;
+        if (mincore(reinterpret_cast<void*>(first + last * k / 15 * kPage), kPage, &in) != 0 || !(in & 1))
+            return false;
+    }
+    return true;
 }
 
 // Threads that touch pages: the process' CPUs less the copying one, at most 8.
@@ -85,7 +101,7 @@ private:
 }  // namespace
 
 cudaError_t download(void* host, const void* dev, size_t bytes, cudaStream_t st) {
-    if (bytes <= kDirect || !pageable(host)) {
+    if (bytes <= kDirect || !pageable(host) || in_place(static_cast<const char*>(host), bytes)) {
         const cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
         return e != cudaSuccess ? e : cudaStreamSynchronize(st);
     }

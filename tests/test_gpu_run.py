@@ -209,3 +209,64 @@ def test_fields_of_several_megabytes_to_any_memory(torch_cuda, shape, precision)
         assert (room[:5] == 77).all() and (room[5 + p.size:] == 77).all()
         pinned = torch_cuda.empty(shape).pin_memory()
         assert np.array_equal(r.field(pinned).numpy(), p)
+
+
+@pytest.mark.parametrize("precision", [sb.PRECISION_F32, sb.PRECISION_F16], ids=["f32", "f16"])
+def test_fields_to_new_and_half_new_pages_from_two_threads(torch_cuda, precision):
+    """Two handles' fields land beside each other in one mapping, downloaded by two host
+    threads at once: pages in place, new ones, the first half in place and every other
+    MB in place, starting inside a page."""
+    import mmap
+    import threading
+
+    shape = (67, 176, 184)  # 8.7 MB
+    nz, ny, nx = shape
+    n = nx * ny * nz
+    p = np.random.default_rng(5).integers(-9, 10, shape).astype(np.float32)  # exact in FP16
+    runs = [sb.Run(sb.Grid(nx, ny, nz, 10, 10, 10, 1e-3), precision=precision) for _ in range(2)]
+    for k, r in enumerate(runs):
+        r.set_fields(p + k, p + k, np.full(shape, 2.25e6, np.float32))
+    for touched in ("all", "none", "half", "odd"):
+        m = mmap.mmap(-1, 8 * n + 8192)
+        room = np.frombuffer(m, np.float32)
+        for i in range(0, 8 * n, 4096):
+            if touched == "all" or (touched == "half" and i < 4 * n) or (touched == "odd" and i >> 20 & 1):
+                room[i // 4] = 3
+        outs = [room[5 + k * n:5 + (k + 1) * n] for k in range(2)]
+        ts = [threading.Thread(target=r.field, args=(o,)) for r, o in zip(runs, outs)]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+        for k, o in enumerate(outs):
+            assert np.array_equal(o.reshape(shape), p + k), touched
+        assert (room[5 + 2 * n:] == 0).all() and not room[1:5].any()
+        del room, outs, ts, o
+        m.close()
+    for r in runs:
+        r.close()
+
+
+def test_a_field_to_pages_in_place_costs_one_copy(torch_cuda):
+    """5.6 MB to an array that is in use: within a third of the runtime's own copy of the
+    field (starting threads for its pages made it 1.6 times as long)."""
+    import time
+
+    shape = (112, 112, 112)
+    src = torch_cuda.zeros(shape, device="cuda")
+    out = torch_cuda.ones(shape)
+
+    def best(f):
+        ts = []
+        for _ in range(30):
+            t0 = time.perf_counter()
+            f()
+            ts.append(time.perf_counter() - t0)
+        return min(ts)
+
+    with sb.Run(sb.Grid(112, 112, 112, 10, 10, 10, 1e-3)) as r:
+        r.set_fields(np.zeros(shape, np.float32), None, np.full(shape, 2.25e6, np.float32))
+        torch_cuda.cuda.synchronize()
+        copy, field = best(lambda: out.copy_(src)), best(lambda: r.field(out))
+    print(copy, field)
+    assert field <= copy * 4 / 3 + 40e-6  # and the checks before it
