@@ -528,16 +528,26 @@ private:
         // a part of a chunk's time, and a 64-plane chunk is a sixth of a step (16 shots of 96
         // to 320 cells, FP32 375-390 -> 365 us per step, FP16 259 -> 251; from 1.5 or 2.5
         // chunks per CTA 370 and 391; the choice of the first length then matters little).
+        // A list that fills most of one wave as it is would only gain the planes that every
+        // chunk reads before its first.  Kept and halved, us: FP32, 256 chunks on 296 CTAs,
+        // one shot of 256^3 52.0 and 57.3, 8 of 128^3 50.7 and 57.5, 224 (7 of 128^3) 49.4 and
+        // 52.9; FP16, whose CTAs start sooner, 576 on 592 (18 of 128^3) 73.2 and 78.3, but 512
+        // (16 of 128^3) 72.5 and 70.4, (2 of 256^3) 70.3 and 66.4.
         int64_t left = 0;  // planes of tiles not handed out yet
-        for (int s = 0; s < n; ++s)
-            left += int64_t(tiles_x[s]) * tiles_y[s] * (shots_[s].g.nz - 8);
-        const double slots = double(sms) * resident;
+        int64_t chunks = 0;
+        for (int s = 0; s < n; ++s) {
+            const int64_t tiles = int64_t(tiles_x[s]) * tiles_y[s], inz = shots_[s].g.nz - 8;
+            left += tiles * inz;
+            chunks += tiles * ((inz + zlen[s] - 1) / zlen[s]);
+        }
+        const int64_t slots = int64_t(sms) * resident;
+        const bool one_wave = chunks <= slots && 10 * chunks > (f16_ ? 9 : 7) * slots;
         for (int s : order) {
             const int64_t tiles = int64_t(tiles_x[s]) * tiles_y[s];
             const int end = static_cast<int>(shots_[s].g.nz - 4);
             for (int z = 4; z < end;) {
                 int len = zlen[s];
-                while (len > 16 && double(left) < slots * len) len = (len + 1) / 2;
+                while (!one_wave && len > 16 && left < slots * len) len = (len + 1) / 2;
                 len = std::min(len, end - z);
                 for (int y = 0; y < tiles_y[s]; ++y)
                     for (int x = 0; x < tiles_x[s]; ++x)

@@ -254,3 +254,19 @@ def test_batch_thin_shots_match_single_grid_runs(precision):
             for (p, tr), (rp, rtr) in zip(got, refs):
                 assert np.array_equal(p, rp), (v, zlen)
                 assert np.array_equal(tr, rtr), (v, zlen)
+
+
+# (shots, items of 32 x 32 columns and 64 planes): each fits the 296 CTAs that a B200 holds
+@pytest.mark.parametrize("shots, equal", [([256], 8 * 8 * 4), ([128] * 8, 8 * 4 * 4 * 2),
+                                          ([64] * 64, 64 * 2 * 2)], ids=["1x256", "8x128", "64x64"])
+def test_a_work_list_of_one_wave_keeps_its_chunks(shots, equal):
+    def items(extents):
+        with sb.Batch([(sb.Grid(n, n, n, 10.0, 10.0, 10.0, 7e-4), -1) for n in extents],
+                      max_steps=4, graph_chunk=0) as b:
+            b.set_choice(0, 64)
+            return b.choice()["items"]
+
+    assert sb.lib().sb200_batch_variant_name(0).decode().startswith("b32x32")
+    assert items(shots) == equal
+    # many waves of the same: the last chunks are cut
+    assert items(shots * 20) > 20 * equal
