@@ -11,6 +11,7 @@
 #include <string>
 #include <tuple>
 
+#include "dispatch.h"
 #include "kernels.h"
 #include "stencil_b200.h"
 
@@ -119,17 +120,25 @@ double split_cost(int64_t tiles, int inz, int zlen, int resident, int sms, doubl
     return waves * (zlen + start);
 }
 
+// What a step costs beside other runs (Sharing, dispatch.h): its part of the sweeping, at
+// least its latency over the steps that overlap it, and a tenth of its latency on top.
+constexpr double kOverlap[] = {1.0, 1.25, 3.0};
+
 // (cost, z chunks) of every distinct chunk length, cheapest first.
-std::vector<std::pair<double, int>> rank_splits(int64_t tiles, int inz, int resident, double start) {
+std::vector<std::pair<double, int>> rank_splits(int64_t tiles, int inz, int resident, double start,
+                                                int sharing) {
     const int sms = std::max(1, sm_count());
     resident = std::max(1, resident);
     std::vector<std::pair<double, int>> out;
     int last = 0;
-    for (int zc = 1; zc <= std::min(inz, 512); ++zc) {
-        const int zlen = (inz + zc - 1) / zc;
+    for (int n = 1; n <= std::min(inz, 512); ++n) {
+        const int zlen = (inz + n - 1) / n;
         if (zlen == last) continue;
         last = zlen;
-        out.emplace_back(split_cost(tiles, inz, zlen, resident, sms, start), (inz + zlen - 1) / zlen);
+        const int zc = (inz + zlen - 1) / zlen;
+        const double alone = split_cost(tiles, inz, zlen, resident, sms, start);
+        const double work = double(tiles) * zc / (double(sms) * resident) * (zlen + start);
+        out.emplace_back(sharing ? std::max(work, alone / kOverlap[sharing]) + 0.1 * alone : alone, zc);
     }
     std::stable_sort(out.begin(), out.end());
     if (out.empty()) out.emplace_back(1.0, 1);
@@ -155,6 +164,12 @@ std::vector<std::pair<double, int>> rank_splits(int64_t tiles, int inz, int resi
 //     three in the table's order; 512^3 438 against 410 / 408 / 415; 160 x 150 x 170 14.1
 //     against 17.7 / 19.1 / 21.2; heat 512^3 301 against 288, 160 x 150 x 170 12.1 against
 //     13.7).
+//   * runs at once, each on its stream, all take one tile: CTAs of unlike kernels do not
+//     share the SMs well, and short chunks that fill an idle device only add planes on a full
+//     one.  48 runs of 96 to 192 cells, us per step of all: each its own choice 652, the
+//     same splits on t64x32_r2_s6_a2 418, with 8 chunks 386 (t128x16_r2_s6_a2 420,
+//     t32x32_r2_s8_a4 421); FP16 339, h64x16_s8_a4 265 (h64x32_s8_a2 278); heat 298,
+//     t64x16_r2_s8 274; reference order 499, t32x16_r1_s8_a4 403-416 (t64x32_r2_s6_a2 439).
 struct Candidate {
     const char* name;
     double in_l2, beyond;
@@ -163,6 +178,8 @@ struct Family {
     double start;
     int step_bytes;  // per cell: the fields a step keeps in use
     Candidate tiles[4];
+    const char* shared;       // the tile of runs that share the device
+    const char* many_beyond;  // and that of many, beyond L2
 };
 // Kinds of choice beyond the public ones: the reference order on the pencil tiles, and the
 // ragged kernels.
@@ -172,18 +189,23 @@ const Family kFamilies[] = {
     // SB200_KIND_WAVE_F32
     {2.1, 12,
      {{"t32x32_r2_s8_a4", 1.38, 0}, {"t64x32_r2_s6_a2", 1.04, 1.074}, {"t128x16_r2_s6_a2", 1.0, 0},
-      {"t128x32_r2_s7_a2", 0, 1.0}}},
+      {"t128x32_r2_s7_a2", 0, 1.0}},
+     "t64x32_r2_s6_a2", "t64x32_r2_s6_a2"},
     // SB200_KIND_HEAT_F32
-    {6.7, 8, {{"t32x32_r2_s8", 1.05, 0}, {"t64x16_r2_s8", 1.0, 1.114}, {"t128x16_r2_s8", 0, 1.0}}},
+    {6.7, 8, {{"t32x32_r2_s8", 1.05, 0}, {"t64x16_r2_s8", 1.0, 1.114}, {"t128x16_r2_s8", 0, 1.0}},
+     "t64x16_r2_s8", "t128x16_r2_s8"},
     // SB200_KIND_WAVE_F16
-    {4.3, 6, {{"h64x16_s8_a4", 0, 1.02}, {"h64x32_s8_a2", 1.1, 0}, {"h128x16_s8_a2", 1.0, 1.0}}},
+    {4.3, 6, {{"h64x16_s8_a4", 0, 1.02}, {"h64x32_s8_a2", 1.1, 0}, {"h128x16_s8_a2", 1.0, 1.0}},
+     "h64x16_s8_a4", "h64x16_s8_a4"},
     {},  // SB200_KIND_WAVE2_F32: one tile
     // kExactWave
     {2.1, 12,
      {{"t32x16_r1_s8_a4", 1.0, 1.0}, {"t64x32_r2_s6_a2", 0.95, 0.95},
-      {"t128x16_r2_s6_a2", 0.94, 0.94}, {"t128x32_r2_s7_a2", 0.92, 0.92}}},
+      {"t128x16_r2_s6_a2", 0.94, 0.94}, {"t128x32_r2_s7_a2", 0.92, 0.92}},
+     "t32x16_r1_s8_a4", "t32x16_r1_s8_a4"},
     // kExactHeat
-    {2.1, 8, {{"t32x16_r1_s8", 1.0, 1.0}, {"t64x16_r2_s8", 0.96, 0.96}}},
+    {2.1, 8, {{"t32x16_r1_s8", 1.0, 1.0}, {"t64x16_r2_s8", 0.96, 0.96}}, "t32x16_r1_s8",
+     "t32x16_r1_s8"},
 };
 constexpr double kL2Bytes = 126e6;
 
@@ -206,7 +228,7 @@ int resident_ctas(int kind, int v) {
 }
 
 // The cheapest tile and split of a family (a public kind's or a reference-order one).
-PencilConfig cheapest(int family, const GridDesc& g) {
+PencilConfig cheapest(int family, const GridDesc& g, int sharing) {
     const Family& f = kFamilies[family];
     const bool exact = family >= kExactWave;
     const int kind = !exact ? family : family == kExactHeat ? SB200_KIND_HEAT_F32 : SB200_KIND_WAVE_F32;
@@ -214,7 +236,9 @@ PencilConfig cheapest(int family, const GridDesc& g) {
     PencilConfig best;
     double cost = 0;
     for (const Candidate& c : f.tiles) {
-        const double weight = beyond ? c.beyond : c.in_l2;
+        double weight = beyond ? c.beyond : c.in_l2;
+        if (sharing && c.name)
+            weight = std::strcmp(c.name, sharing == kMany && beyond ? f.many_beyond : f.shared) == 0;
         const int v = c.name && weight > 0 ? variant_by_name(kind, c.name) : -1;
         if (v < 0) continue;
         const PencilBoxes b = kind == SB200_KIND_WAVE_F16
@@ -223,7 +247,7 @@ PencilConfig cheapest(int family, const GridDesc& g) {
         const int resident = exact ? pencil_f32_resident(kind == SB200_KIND_HEAT_F32, v, true)
                                    : resident_ctas(kind, v);
         const auto s =
-            rank_splits(column_tiles(kind, v, g), static_cast<int>(g.nz - 8), resident, f.start)
+            rank_splits(column_tiles(kind, v, g), static_cast<int>(g.nz - 8), resident, f.start, sharing)
                 .front();
         const double t = s.first * weight * b.points * resident;
         if (cost == 0 || t < cost) {
@@ -235,7 +259,7 @@ PencilConfig cheapest(int family, const GridDesc& g) {
     return best;
 }
 
-PencilConfig choose(int kind, const GridDesc& g) {
+PencilConfig choose(int kind, const GridDesc& g, int sharing = kAlone) {
     {
         std::lock_guard<std::mutex> lock(g_cfg_mu);
         // the reference order runs the same tiles: an override of the kind holds for it too
@@ -252,27 +276,28 @@ PencilConfig choose(int kind, const GridDesc& g) {
     }
     PencilConfig c;
     if (kind < 4 && tuned_choice(kind, g, &c)) return c;
-    // Heuristic pick, memoised per (kind, extents, device): launches stay cheap
+    // Heuristic pick, memoised per (kind, extents, device, sharing): launches stay cheap
     // on the host.
     static std::mutex memo_mu;
-    static std::map<std::tuple<int, int64_t, int64_t, int64_t, int>, PencilConfig> memo;
+    static std::map<std::tuple<int, int64_t, int64_t, int64_t, int, int>, PencilConfig> memo;
     int dev = 0;
     cudaGetDevice(&dev);
-    const auto key = std::make_tuple(kind, g.nx, g.ny, g.nz, dev);
+    const auto key = std::make_tuple(kind, g.nx, g.ny, g.nz, dev, sharing);
     std::lock_guard<std::mutex> lock(memo_mu);
     auto it = memo.find(key);
     if (it != memo.end()) return it->second;
     const int inz = static_cast<int>(g.nz - 8);
     const double start = kFamilies[SB200_KIND_WAVE_F32].start;
     if (kind >= kRaggedWave) {
-        c.zchunks = rank_splits(ragged_ctas(g, 1), inz, ragged_resident(kind == kRaggedHeat, g), start)
+        c.zchunks = rank_splits(ragged_ctas(g, 1), inz, ragged_resident(kind == kRaggedHeat, g), start,
+                                sharing)
                         .front()
                         .second;
     } else if (kind == SB200_KIND_WAVE2_F32) {
         c.variant = std::max(0, variant_by_name(kind, "l32x32_r1_s8"));
         c.zchunks = zchunk_ranking(kind, c.variant, g, 1).front();
     } else {
-        c = cheapest(kind, g);
+        c = cheapest(kind, g, sharing);
     }
     memo[key] = c;
     return c;
@@ -352,7 +377,7 @@ int ragged_maps(bool heat, const GridDesc& g, const void* field, const void* pre
 
 int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_next,
               const sb200_grid* grid, const SourceDesc& src, void* stream, bool exact,
-              const char* where) {
+              const char* where, int sharing = kAlone) {
     const int64_t src_index = src.idx;
     GridDesc g;
     if (int rc = to_desc(grid, &g)) return rc;
@@ -365,7 +390,7 @@ int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_n
     if (!g.has_interior()) return SB200_OK;  // no interior point: nothing to update
     auto st = static_cast<cudaStream_t>(stream);
     if ((!exact || staged_pays(g, false)) && pencil_ok(g, {p, p_prev, vel2, p_next})) {
-        const PencilConfig cfg = choose(exact ? int(kExactWave) : int(SB200_KIND_WAVE_F32), g);
+        const PencilConfig cfg = choose(exact ? int(kExactWave) : int(SB200_KIND_WAVE_F32), g, sharing);
         PencilMaps maps;
         if (int rc = pencil_maps(false, cfg.variant, g, p, p_prev, vel2, &maps, where)) return rc;
         return finish_launch(launch_wave_pencil_f32(maps, p_prev, vel2, p_next, g, src, cfg,
@@ -376,19 +401,28 @@ int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_n
         PencilMaps maps;
         if (int rc = ragged_maps(false, g, p, p_prev, vel2, &maps, where)) return rc;
         return finish_launch(launch_wave_ragged_f32(maps, p_next, g, src,
-                                                    choose(kRaggedWave, g).zchunks,
+                                                    choose(kRaggedWave, g, sharing).zchunks,
                                                     device_error_ptr(), st),
                              where);
     }
     return finish_launch(launch_wave_naive(p, p_prev, vel2, p_next, g, src, st), where);
 }
 
-int heat_step(const float* u, float* u_next, const GridDesc& g, float alpha_dt, void* stream,
-              bool exact, const char* where) {
+int heat_step(const float* u, float* u_next, const sb200_grid* grid, float alpha, void* stream,
+              bool exact, const char* where, int sharing = kAlone) {
+    GridDesc g;
+    if (int rc = to_desc(grid, &g)) return rc;
+    if (!u || !u_next) return fail(SB200_ERR_INVALID, std::string(where) + ": NULL field pointer");
+    if (u == u_next)
+        return fail(SB200_ERR_INVALID, std::string(where) + ": u_next must not alias u");
+    if (!std::isfinite(alpha))
+        return fail(SB200_ERR_INVALID, std::string(where) + ": alpha must be finite");
+    if (!g.has_interior()) return SB200_OK;
+    const float alpha_dt = alpha * g.dt;
     auto st = static_cast<cudaStream_t>(stream);
     PencilMaps maps;
     if ((!exact || staged_pays(g, false)) && pencil_ok(g, {u, u_next})) {
-        const PencilConfig cfg = choose(exact ? int(kExactHeat) : int(SB200_KIND_HEAT_F32), g);
+        const PencilConfig cfg = choose(exact ? int(kExactHeat) : int(SB200_KIND_HEAT_F32), g, sharing);
         if (int rc = pencil_maps(true, cfg.variant, g, u, nullptr, nullptr, &maps, where)) return rc;
         return finish_launch(launch_heat_pencil_f32(maps, u_next, g, alpha_dt, cfg,
                                                     device_error_ptr(), st, exact),
@@ -397,7 +431,7 @@ int heat_step(const float* u, float* u_next, const GridDesc& g, float alpha_dt, 
     if (staged_pays(g, true) && ragged_ok(g) && aligned16(u)) {
         if (int rc = ragged_maps(true, g, u, nullptr, nullptr, &maps, where)) return rc;
         return finish_launch(launch_heat_ragged_f32(maps, u_next, g, alpha_dt,
-                                                    choose(kRaggedHeat, g).zchunks,
+                                                    choose(kRaggedHeat, g, sharing).zchunks,
                                                     device_error_ptr(), st),
                              where);
     }
@@ -448,7 +482,7 @@ SourceDesc host_source(int64_t idx, float amp) {
 
 int wave_step_f16(const uint16_t* p, uint16_t* p_prev_next, const uint16_t* k,
                   const sb200_grid* grid, const SourceDesc& src, const sb200_f16_scale* scale,
-                  int phase, void* stream) {
+                  int phase, void* stream, int sharing = kAlone) {
     const char* where = "sb200_wave_step_f16";
     GridDesc g;
     if (int rc = to_desc(grid, &g)) return rc;
@@ -465,7 +499,7 @@ int wave_step_f16(const uint16_t* p, uint16_t* p_prev_next, const uint16_t* k,
     if (g.nx % 8 != 0 || !aligned16(p) || !aligned16(p_prev_next) || !aligned16(k))
         return fail(SB200_ERR_UNSUPPORTED,
                     std::string(where) + ": needs nx % 8 == 0 and 16-byte aligned fields");
-    const PencilConfig cfg = choose(SB200_KIND_WAVE_F16, g);
+    const PencilConfig cfg = choose(SB200_KIND_WAVE_F16, g, sharing);
     const PencilBoxes b = pencil_f16_boxes(cfg.variant);
     PencilMaps maps;
     int rc = tensor_map_3d(&maps.p, p, g.nx, g.ny, g.nz, 2, b.halo_x, b.halo_y);
@@ -485,9 +519,16 @@ int wave_step_f16(const uint16_t* p, uint16_t* p_prev_next, const uint16_t* k,
 // Step dispatch with a full source descriptor (trace included), for the run
 // engine; the public entry points wrap these.
 int dispatch_wave_f32(const float* p, const float* p_prev, const float* vel2, float* p_next,
-                      const sb200_grid* grid, const SourceDesc& src, void* stream, bool exact) {
+                      const sb200_grid* grid, const SourceDesc& src, void* stream, bool exact,
+                      int sharing) {
     return wave_step(p, p_prev, vel2, p_next, grid, src, stream, exact,
-                     exact ? "sb200_wave_step_exact_f32" : "sb200_wave_step_f32");
+                     exact ? "sb200_wave_step_exact_f32" : "sb200_wave_step_f32", sharing);
+}
+
+int dispatch_heat_f32(const float* u, float* u_next, const sb200_grid* grid, float alpha,
+                      void* stream, bool exact, int sharing) {
+    return heat_step(u, u_next, grid, alpha, stream, exact,
+                     exact ? "sb200_heat_step_exact_f32" : "sb200_heat_step_f32", sharing);
 }
 
 int dispatch_wave2_f32(const float* p, const float* p_prev, const float* vel2, float* out1,
@@ -499,8 +540,8 @@ int dispatch_wave2_f32(const float* p, const float* p_prev, const float* vel2, f
 
 int dispatch_wave_f16(const uint16_t* p, uint16_t* p_prev_next, const uint16_t* k,
                       const sb200_grid* grid, const SourceDesc& src, const sb200_f16_scale* scale,
-                      int phase, void* stream) {
-    return wave_step_f16(p, p_prev_next, k, grid, src, scale, phase, stream);
+                      int phase, void* stream, int sharing) {
+    return wave_step_f16(p, p_prev_next, k, grid, src, scale, phase, stream, sharing);
 }
 
 int set_error(int code, const std::string& msg) { return fail(code, msg); }
@@ -511,7 +552,7 @@ std::vector<int> zchunk_ranking(int kind, int v, const GridDesc& g, int max_n) {
     // (two steps per sweep: a chunk reads 16 halo planes)
     const auto ranked =
         rank_splits(column_tiles(kind, v, g), static_cast<int>(g.nz - 8), resident_ctas(kind, v),
-                    kind == SB200_KIND_WAVE2_F32 ? 6.0 : kFamilies[kind].start);
+                    kind == SB200_KIND_WAVE2_F32 ? 6.0 : kFamilies[kind].start, kAlone);
     std::vector<int> out;
     for (const auto& s : ranked)
         if (static_cast<int>(out.size()) < max_n) out.push_back(s.second);
@@ -628,29 +669,12 @@ int sb200_set_device_int(int* dst, int value, void* stream) {
 
 int sb200_heat_step_exact_f32(const float* u, float* u_next, const sb200_grid* grid,
                               float alpha, void* stream) {
-    GridDesc g;
-    if (int rc = to_desc(grid, &g)) return rc;
-    if (!u || !u_next)
-        return fail(SB200_ERR_INVALID, "sb200_heat_step_exact_f32: NULL field pointer");
-    if (u == u_next)
-        return fail(SB200_ERR_INVALID, "sb200_heat_step_exact_f32: u_next must not alias u");
-    if (!std::isfinite(alpha))
-        return fail(SB200_ERR_INVALID, "sb200_heat_step_exact_f32: alpha must be finite");
-    if (!g.has_interior()) return SB200_OK;
-    return heat_step(u, u_next, g, alpha * g.dt, stream, true, "sb200_heat_step_exact_f32");
+    return heat_step(u, u_next, grid, alpha, stream, true, "sb200_heat_step_exact_f32");
 }
 
 int sb200_heat_step_f32(const float* u, float* u_next, const sb200_grid* grid, float alpha,
                         void* stream) {
-    GridDesc g;
-    if (int rc = to_desc(grid, &g)) return rc;
-    if (!u || !u_next) return fail(SB200_ERR_INVALID, "sb200_heat_step_f32: NULL field pointer");
-    if (u == u_next)
-        return fail(SB200_ERR_INVALID, "sb200_heat_step_f32: u_next must not alias u");
-    if (!std::isfinite(alpha))
-        return fail(SB200_ERR_INVALID, "sb200_heat_step_f32: alpha must be finite");
-    if (!g.has_interior()) return SB200_OK;
-    return heat_step(u, u_next, g, alpha * g.dt, stream, false, "sb200_heat_step_f32");
+    return heat_step(u, u_next, grid, alpha, stream, false, "sb200_heat_step_f32");
 }
 
 int sb200_wave_prepass_f32(const float* p, float* p_prev, const float* vel2, float* r,

@@ -10,8 +10,15 @@
 
 namespace sb200 {
 
+// Beside how many other runs an untuned step is made: at most one, two or three, four and
+// more.  Its tile and z split follow that, its bits do not.
+enum Sharing : int { kAlone = 0, kFew, kMany };
+
 int dispatch_wave_f32(const float* p, const float* p_prev, const float* vel2, float* p_next,
-                      const sb200_grid* grid, const SourceDesc& src, void* stream, bool exact);
+                      const sb200_grid* grid, const SourceDesc& src, void* stream, bool exact,
+                      int sharing);
+int dispatch_heat_f32(const float* u, float* u_next, const sb200_grid* grid, float alpha,
+                      void* stream, bool exact, int sharing);
 // Two acoustic steps in one sweep (out1 = t+dt, out2 = t+2dt; w1 = the host
 // sample of the second step).  outputs_may_alias: out1 == out2 is accepted
 // (timing trials only: the values are then unusable).
@@ -20,7 +27,7 @@ int dispatch_wave2_f32(const float* p, const float* p_prev, const float* vel2, f
                        void* stream, bool outputs_may_alias);
 int dispatch_wave_f16(const uint16_t* p, uint16_t* p_prev_next, const uint16_t* k,
                       const sb200_grid* grid, const SourceDesc& src, const sb200_f16_scale* scale,
-                      int phase, void* stream);
+                      int phase, void* stream, int sharing);
 // Records msg as the calling thread's last error and returns code.
 int set_error(int code, const std::string& msg);
 // Address of the library's device error word on the current device (the word

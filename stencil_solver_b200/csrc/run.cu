@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -38,6 +39,9 @@ __global__ void monitor_kernel(const double* stats3, int* flag, double limit) {
     launch_order();
     if (!(stats3[2] == 0.0) || !(stats3[1] <= limit)) atomicExch(flag, 1);
 }
+
+// Per device: runs with steps queued that nobody has waited for.
+std::atomic<int> g_busy[64] = {};
 
 constexpr int64_t kStageFloats = int64_t(1) << 24;  // host <-> device staging: up to 64 MB
 
@@ -74,6 +78,7 @@ public:
         if (c_.src_index >= n_) return set_error(SB200_ERR_INVALID, "sb200_run_create: bad source");
         if (fp16_) c_.graph_chunk = c_.graph_chunk ? c_.renorm_every : 0;
 
+        if (int rc = cuda(cudaGetDevice(&dev_))) return rc;
         if (int rc = cuda(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking))) return rc;
         const size_t es = fp16_ ? 2 : 4;
         if (int rc = alloc(&a_, n_ * es)) return rc;
@@ -109,6 +114,7 @@ public:
 
     ~Run() {
         if (st_) cudaStreamSynchronize(st_);
+        set_busy(false);
         drop_graphs();
         for (void* p : {a_, b_, static_cast<void*>(vel2_), static_cast<void*>(k_),
                         static_cast<void*>(wavelet_dev_), static_cast<void*>(trace_dev_),
@@ -140,7 +146,7 @@ public:
                     return rc;
                 vel2_host_src_ = c_.src_index >= 0 ? vel2[c_.src_index] : 0.f;
             }
-            return cuda(cudaStreamSynchronize(st_));
+            return wait();
         }
         // FP16: initial scale from the fields' largest magnitude, taken on the device as
         // their chunks pass through the staging buffer, and the first window's source.
@@ -175,7 +181,7 @@ public:
         if (same)
             if (int rc = cuda(cudaMemcpyAsync(b_, a_, n_ * 2, cudaMemcpyDeviceToDevice, st_))) return rc;
         if (int rc = stage_in(vel2, k_, 1.f, true)) return rc;
-        return cuda(cudaStreamSynchronize(st_));
+        return wait();
     }
 
     // generated: the samples are the run's own Ricker, which steps() extends on
@@ -200,18 +206,22 @@ public:
                 return set_error(SB200_ERR_INVALID, "sb200_run_steps: wavelet shorter than the run");
             }
         }
+        const int beside = std::max(others(), seen_);
+        share_ = beside < 2 ? kAlone : beside < 4 ? kFew : kMany;
+        if (n > 0) set_busy(true);
         const int C = c_.graph_chunk;
         int64_t done = 0;
         while (done < n) {
             const bool aligned = !fp16_ || step_ % c_.renorm_every == 0;
             if (C > 0 && aligned && n - done >= C) {
-                // a graph bakes in which buffer is current: one per parity
-                const int par = a_ == home_ ? 0 : 1;
-                if (!graph_[par]) {
-                    if (int rc = capture(&graph_[par])) return rc;
+                // a graph bakes in which buffer is current, and the launches' tiles and
+                // splits: one per parity and sharing
+                cudaGraphExec_t& graph = graph_[share_][a_ == home_ ? 0 : 1];
+                if (!graph) {
+                    if (int rc = capture(&graph)) return rc;
                 }
                 if (int rc = sb200_set_device_int(step_dev_, static_cast<int>(step_), st_)) return rc;
-                if (int rc = cuda(cudaGraphLaunch(graph_[par], st_))) return rc;
+                if (int rc = cuda(cudaGraphLaunch(graph, st_))) return rc;
                 step_ += C;
                 done += C;
                 continue;
@@ -223,7 +233,7 @@ public:
     }
 
     int synchronize() {
-        if (int rc = cuda(cudaStreamSynchronize(st_))) return rc;
+        if (int rc = wait()) return rc;
         int flag = 0;
         if (int rc = cuda(cudaMemcpy(&flag, monitor_dev_, sizeof(int), cudaMemcpyDeviceToHost)))
             return rc;
@@ -290,7 +300,7 @@ public:
     int stats(double* out3) {
         if (!out3) return set_error(SB200_ERR_INVALID, "sb200_run_stats: NULL destination");
         if (int rc = enqueue_stats()) return rc;
-        if (int rc = cuda(cudaStreamSynchronize(st_))) return rc;
+        if (int rc = wait()) return rc;
         if (int rc = cuda(cudaMemcpy(out3, stats_dev_, 3 * sizeof(double), cudaMemcpyDeviceToHost)))
             return rc;
         if (fp16_) {  // stats of the stored field: bring them to physical units
@@ -311,6 +321,20 @@ private:
         return set_error(SB200_ERR_CUDA, std::string("run: ") + cudaGetErrorString(e));
     }
     int alloc(void** p, size_t bytes) { return cuda(cudaMalloc(p, bytes)); }
+
+    void set_busy(bool busy) {
+        if (busy != busy_) g_busy[dev_ & 63] += busy ? 1 : -1;
+        busy_ = busy;
+    }
+    int others() const { return g_busy[dev_ & 63].load() - (busy_ ? 1 : 0); }
+    // Waits for the run's stream.  The first of several runs to be stepped meets the others
+    // here: it takes its steps for shared from the next time on.
+    int wait() {
+        if (busy_) seen_ = others();
+        const int rc = cuda(cudaStreamSynchronize(st_));
+        set_busy(false);
+        return rc;
+    }
 
     // Staging: one chunk of kStageFloats values, or two whole fields where they are no
     // longer than a chunk.
@@ -466,19 +490,16 @@ private:
         }
         int rc;
         if (heat_) {
-            rc = c_.exact ? sb200_heat_step_exact_f32(static_cast<const float*>(a_),
-                                                      static_cast<float*>(b_), &c_.grid,
-                                                      c_.diffusivity, st_)
-                          : sb200_heat_step_f32(static_cast<const float*>(a_),
-                                                static_cast<float*>(b_), &c_.grid, c_.diffusivity,
-                                                st_);
+            rc = dispatch_heat_f32(static_cast<const float*>(a_), static_cast<float*>(b_), &c_.grid,
+                                   c_.diffusivity, st_, c_.exact != 0, share_);
         } else if (fp16_) {
             rc = dispatch_wave_f16(static_cast<const uint16_t*>(a_), static_cast<uint16_t*>(b_), k_,
                                    &c_.grid, src, reinterpret_cast<const sb200_f16_scale*>(scale_dev_),
-                                   phase, st_);
+                                   phase, st_, share_);
         } else {
             rc = dispatch_wave_f32(static_cast<const float*>(a_), static_cast<const float*>(b_),
-                                   vel2_, static_cast<float*>(b_), &c_.grid, src, st_, c_.exact != 0);
+                                   vel2_, static_cast<float*>(b_), &c_.grid, src, st_, c_.exact != 0,
+                                   share_);
         }
         std::swap(a_, b_);
         return rc;
@@ -518,11 +539,12 @@ private:
     }
 
     void drop_graphs() {
-        for (auto& g : graph_)
-            if (g) {
-                cudaGraphExecDestroy(g);
-                g = nullptr;
-            }
+        for (auto& pair : graph_)
+            for (auto& g : pair)
+                if (g) {
+                    cudaGraphExecDestroy(g);
+                    g = nullptr;
+                }
     }
 
     int capture(cudaGraphExec_t* out) {
@@ -582,7 +604,11 @@ private:
     int* monitor_dev_ = nullptr;
     F16Scale* scale_dev_ = nullptr;
     float* stage_ = nullptr;
-    cudaGraphExec_t graph_[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph_[3][2] = {};  // [sharing][parity]
+    int dev_ = 0;
+    bool busy_ = false;  // steps queued since the last wait
+    int seen_ = 0;        // other busy runs at that wait
+    int share_ = kAlone;  // as found by the latest steps()
     void* home_ = nullptr;  // buffer that is current at even parity
     int64_t step_ = 0;
 };

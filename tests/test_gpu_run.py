@@ -270,3 +270,79 @@ def test_a_field_to_pages_in_place_costs_one_copy(torch_cuda):
         copy, field = best(lambda: out.copy_(src)), best(lambda: r.field(out))
     print(copy, field)
     assert field <= copy * 4 / 3 + 40e-6  # and the checks before it
+
+
+@pytest.mark.parametrize("opts", [{}, {"exact": 1}, {"precision": sb.PRECISION_F16},
+                                  {"physics": sb.PHYSICS_HEAT, "diffusivity": 1.0}],
+                         ids=["f32", "exact", "f16", "heat"])
+def test_runs_at_once_give_the_same_bits(opts):
+    """Eight runs of unlike grids queued before the first is waited for (they take other
+    tiles and splits than a run alone), in passes that cross the graphs' parity, against
+    each run by itself."""
+    shapes = [(72, 64, 60), (96, 88, 80), (40, 41, 44), (64, 128, 100), (128, 33, 49),
+              (64, 64, 64), (88, 72, 101), (56, 90, 38)]
+    heat = "physics" in opts
+
+    def make(shape, seed):
+        nx, ny, nz = shape
+        g = sb.Grid(nx, ny, nz, 10.0, 10.0, 10.0, 7e-4)
+        r = sb.Run(g, graph_chunk=4, renorm_every=4, **opts,
+                   **({} if heat else {"src_index": g.index(nx // 2, ny // 2, nz // 2)}))
+        rng = np.random.default_rng(seed)
+        p = np.where(np.pad(np.ones([n - 8 for n in g.shape], bool), 4),
+                     rng.standard_normal(g.shape), 0).astype(np.float32)
+        r.set_fields(p, p, np.full(g.shape, 2000.0 ** 2, np.float32))
+        return r
+
+    alone = []
+    for k, s in enumerate(shapes):
+        with make(s, k) as r:
+            for n in (9, 8, 12):
+                r.steps(n)
+                r.synchronize()
+            alone.append(r.field())
+    runs = [make(s, k) for k, s in enumerate(shapes)]
+    for n in (9, 8, 12):
+        for r in runs:
+            r.steps(n)
+        for r in runs[::3]:
+            r.synchronize()
+    for r, want in zip(runs, alone):
+        assert np.array_equal(r.field(), want)
+        r.close()
+
+
+def test_runs_at_once_take_no_longer_than_their_steps_alone(torch_cuda):
+    """24 uneven runs at once, each on its stream: less than the sum of their times one
+    after the other (with tiles and splits chosen for an idle device it was more)."""
+    import time
+
+    rng = np.random.default_rng(0)
+    runs = []
+    for _ in range(24):
+        nx, ny, nz = (int(rng.choice([96, 128, 160, 192])) for _ in range(3))
+        g = sb.Grid(nx, ny, nz, 10.0, 10.0, 10.0, 7e-4)
+        r = sb.Run(g, src_index=g.index(nx // 2, ny // 2, nz // 2), graph_chunk=100)
+        z = np.zeros(g.shape, np.float32)
+        r.set_fields(z, z, np.full(g.shape, 2000.0 ** 2, np.float32))
+        runs.append(r)
+
+    def wall(at_once):
+        best = float("inf")
+        for _ in range(4):
+            torch_cuda.cuda.synchronize()
+            t0 = time.perf_counter()
+            for r in runs:
+                r.steps(100)
+                if not at_once:
+                    r.synchronize()
+            for r in runs:
+                r.synchronize()
+            best = min(best, time.perf_counter() - t0)
+        return best
+
+    alone, together = wall(False), wall(True)
+    print(alone, together)
+    for r in runs:
+        r.close()
+    assert together < 0.95 * alone
