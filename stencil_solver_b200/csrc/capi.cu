@@ -181,9 +181,16 @@ struct Family {
     const char* shared;       // the tile of runs that share the device
     const char* many_beyond;  // and that of many, beyond L2
 };
-// Kinds of choice beyond the public ones: the reference order on the pencil tiles, and the
-// ragged kernels.
-enum Internal : int { kExactWave = 4, kExactHeat, kRaggedWave, kRaggedHeat };
+// Kinds of choice beyond the public ones: the reference order on the pencil tiles, the
+// composition pre-pass, and the ragged kernels.
+enum Internal : int { kExactWave = 4, kExactHeat, kPrepass, kRaggedWave, kRaggedHeat };
+bool reference_order(int kind) { return kind == kExactWave || kind == kExactHeat; }
+// The public kind whose tiles a kind runs on.
+int tiles_of(int kind) {
+    return kind == kExactHeat ? SB200_KIND_HEAT_F32
+           : kind == kExactWave || kind == kPrepass ? SB200_KIND_WAVE_F32
+                                                    : kind;
+}
 
 const Family kFamilies[] = {
     // SB200_KIND_WAVE_F32
@@ -206,6 +213,11 @@ const Family kFamilies[] = {
     // kExactHeat
     {2.1, 8, {{"t32x16_r1_s8", 1.0, 1.0}, {"t64x16_r2_s8", 0.96, 0.96}}, "t32x16_r1_s8",
      "t32x16_r1_s8"},
+    // kPrepass beyond L2 (smaller grids: as the acoustic step).  It writes two fields and pays
+    // more for a chunk's start; the acoustic step's choice took 10 to 14 % longer than the one
+    // 64 x 32 CTA per SM before it on some grids (192 x 1024 x 1024 805 and 715 us, 440^3 310
+    // and 283).  Over 22 grids now at most 4 % longer than the better of the two, 715 and 281.
+    {10, 12, {{"t64x32_r2_s8_a3", 0, 1.02}, {"t128x32_r2_s7_a2", 0, 0.96}}, "", ""},
 };
 constexpr double kL2Bytes = 126e6;
 
@@ -229,10 +241,11 @@ int resident_ctas(int kind, int v) {
 
 // The cheapest tile and split of a family (a public kind's or a reference-order one).
 PencilConfig cheapest(int family, const GridDesc& g, int sharing) {
+    const bool beyond = double(g.size()) * kFamilies[family].step_bytes > kL2Bytes;
+    if (family == kPrepass && !beyond) family = SB200_KIND_WAVE_F32;
     const Family& f = kFamilies[family];
-    const bool exact = family >= kExactWave;
-    const int kind = !exact ? family : family == kExactHeat ? SB200_KIND_HEAT_F32 : SB200_KIND_WAVE_F32;
-    const bool beyond = double(g.size()) * f.step_bytes > kL2Bytes;
+    const bool exact = reference_order(family);
+    const int kind = tiles_of(family);
     PencilConfig best;
     double cost = 0;
     for (const Candidate& c : f.tiles) {
@@ -262,11 +275,8 @@ PencilConfig cheapest(int family, const GridDesc& g, int sharing) {
 PencilConfig choose(int kind, const GridDesc& g, int sharing = kAlone) {
     {
         std::lock_guard<std::mutex> lock(g_cfg_mu);
-        // the reference order runs the same tiles: an override of the kind holds for it too
-        const int of = kind == kExactWave   ? SB200_KIND_WAVE_F32
-                       : kind == kExactHeat ? SB200_KIND_HEAT_F32
-                                            : kind;
-        const Override o = of < 4 ? g_override[of] : Override();
+        // an override of a kind holds for all that run on its tiles
+        const Override o = tiles_of(kind) < 4 ? g_override[tiles_of(kind)] : Override();
         if (o.variant >= 0) {
             PencilConfig c;
             c.variant = o.variant;
@@ -275,7 +285,7 @@ PencilConfig choose(int kind, const GridDesc& g, int sharing = kAlone) {
         }
     }
     PencilConfig c;
-    if (kind < 4 && tuned_choice(kind, g, &c)) return c;
+    if ((kind < 4 || kind == kPrepass) && tuned_choice(tiles_of(kind), g, &c)) return c;
     // Heuristic pick, memoised per (kind, extents, device, sharing): launches stay cheap
     // on the host.
     static std::mutex memo_mu;
@@ -692,7 +702,7 @@ int sb200_wave_prepass_f32(const float* p, float* p_prev, const float* vel2, flo
     if (!pencil_ok(g, {p, p_prev, vel2, r}))
         return fail(SB200_ERR_UNSUPPORTED,
                     std::string(where) + ": needs nx % 4 == 0 and 16-byte aligned fields");
-    const PencilConfig cfg = choose(SB200_KIND_WAVE_F32, g);
+    const PencilConfig cfg = choose(kPrepass, g);
     PencilMaps maps;
     if (int rc = pencil_maps(false, cfg.variant, g, p, p_prev, vel2, &maps, where)) return rc;
     return finish_launch(launch_prepass_pencil_f32(maps, p_prev, vel2, r, g, beta, cfg,

@@ -77,3 +77,31 @@ def test_prepass_rejects_bad_arguments(torch_cuda):
     with pytest.raises(sb.StencilError) as e:
         sb.wave_prepass(x, x.clone(), x.clone(), x.clone(), odd)
     assert e.value.status == sb.SB200_ERR_UNSUPPORTED
+
+
+def test_untuned_choice_beyond_l2(torch_cuda):
+    """192 x 1024 x 1024: the untuned pre-pass is no slower than one 64 x 32 tile per SM in
+    three chunks (the acoustic step's choice took 1.13 times as long)."""
+    g = sb.Grid(192, 1024, 1024, 10.0, 10.0, 10.0, 7e-4)
+    p, q, r = (torch_cuda.zeros(g.shape, device="cuda") for _ in range(3))
+    p.normal_()
+    v = torch_cuda.full(g.shape, 4e6, device="cuda")
+    tile = sb.variant_names(sb.KIND_WAVE_F32).index("t64x32_r2_s8_a3")
+
+    def ms(variant):
+        sb.set_pencil_override(sb.KIND_WAVE_F32, variant, 3)
+        e0, e1 = (torch_cuda.cuda.Event(enable_timing=True) for _ in range(2))
+        sb.wave_prepass(p, q, v, r, g)
+        e0.record()
+        for _ in range(10):
+            sb.wave_prepass(p, q, v, r, g)
+        e1.record()
+        e1.synchronize()
+        return e0.elapsed_time(e1) / 10
+
+    try:
+        pairs = [(ms(-1), ms(tile)) for _ in range(5)]
+    finally:
+        sb.set_pencil_override(sb.KIND_WAVE_F32, -1, 1)
+    print(pairs)
+    assert min(a for a, _ in pairs) <= 1.05 * min(b for _, b in pairs)
