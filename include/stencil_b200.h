@@ -464,6 +464,10 @@ int sb200_mlp_set_min_scale(void* handle, float floor);
 float sb200_mlp_min_scale(void* handle);
 /* Correction kernel of the handle: 0 = tcgen05 (default), 1 = mma.sync. */
 int sb200_mlp_set_kernel(void* handle, int kernel);
+/* For tests of the error path: on != 0 makes every active chunk of the handle's fused steps end
+ * as if its last wait for the tensor cores had run out of time.  sb200_device_error then
+ * reports it, and flags_out is not written. */
+int sb200_mlp_give_up_wait(void* handle, int on);
 /* Training rows at n cells (device int64 flat indices, interior only):
  * X[r] = features of p at cells[r], t[r] = (p_true - p_plain)[cell] / s. */
 int sb200_mlp_samples(const float* p, const float* vel2, const float* p_true, const float* p_plain,

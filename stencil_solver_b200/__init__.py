@@ -194,6 +194,7 @@ _SIGNATURES = {
     "sb200_mlp_set_params": ([C.c_void_p, C.c_void_p], C.c_int),
     "sb200_mlp_set_output_scale": ([C.c_void_p, C.c_float], C.c_int),
     "sb200_mlp_set_kernel": ([C.c_void_p, C.c_int], C.c_int),
+    "sb200_mlp_give_up_wait": ([C.c_void_p, C.c_int], C.c_int),
     "sb200_mlp_output_scale": ([C.c_void_p], C.c_float),
     "sb200_mlp_forward": ([C.c_void_p] * 3 + [C.c_int64, C.c_void_p], C.c_int),
     "sb200_mlp_gradients": ([C.c_void_p] * 3 + [C.c_int64, C.c_void_p, C.c_void_p], C.c_int),

@@ -82,6 +82,7 @@ struct LearnedNet {
     float b3 = 0.f;
     float out_scale = 1.f;
     float min_scale = 0.f;  // correction floor (stars below it: no correction)
+    bool give_up = false;   // sb200_mlp_give_up_wait
 };
 // Boxes of its tensor maps, resident CTAs per SM, and the launch: p_next =
 // acoustic step of p + learned correction, in place over p_prev.

@@ -102,6 +102,7 @@ struct LearnedArgs {
     float b1[H], b2[H], w3[H];
     float b3;
     int* err;
+    bool give_up;  // tests: as if the last plane's layer-2 wait had given up
     // Activity flags (one byte per tile and z chunk; zchunks chunks of zlen):
     // flags_in[c] != 0 when chunk c of p may hold a value at or above half the floor
     // (NULL: every chunk may), box [x0, x1) x [y0, y1) x [z0, z1) cells counts as
@@ -333,6 +334,7 @@ __global__ void __launch_bounds__(LNT, 4)
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t s_tmem;
     __shared__ int s_flag;  // a bounded wait gave up
+    __shared__ int s_late;  // one did by the end of a plane (read after the last only)
     unsigned char* base = smem_align<128>(dyn);
     unsigned char* sA = base;
     unsigned char* sW1 = base + kOffW1;
@@ -387,6 +389,7 @@ __global__ void __launch_bounds__(LNT, 4)
         mbar_init(&mbar, LNT / 32);  // one commit per warp and layer
         fence_barrier_init();
         s_flag = 0;
+        s_late = 0;
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -691,23 +694,29 @@ __global__ void __launch_bounds__(LNT, 4)
             const float m = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(o.w)));
             if (m > 0.f && m >= a.flag_floor) bits |= face_bits(lx, ly, i, nint);
         }
+        if (bad) s_late = 1;
         goff += a.sz;
     }
     {
         const uint32_t out_bits = block_or(bits);
-        if (a.flags_out && tid == 0 && !abort_run)
+        if (a.flags_out && tid == 0 && !abort_run && !(s_late || a.give_up))
             a.flags_out[(int64_t(b) * a.tiles_y + ty) * a.tiles_x + tx] = uint8_t(out_bits);
     }
 
     if (abort_run && tid == 0) {
-        record_error(a.err, kDevWaitTimeout);
-        // Let every copy and MMA still in flight land before shared memory and
-        // TMEM are released.
+        // Let every copy still in flight land before shared memory is released.
         for (int jj = max(0, issued_hi - LS + 1); jj <= issued_hi; ++jj)
             (void)mbar_wait(&full[jj % LS], (jj / LS) & 1);
         for (int it = max(0, aux_issued_hi - LAUX + 1); it <= aux_issued_hi; ++it)
             (void)mbar_wait(&auxf[it % LAUX], (it / LAUX) & 1);
-        if (waited < ncommit) (void)mbar_wait(&mbar, (ncommit - 1u) & 1u);
+    }
+    // A wait for the tensor cores that gave up in the last plane stopped no next plane: it is
+    // reported here.  Their commits still in flight, at most a plane's two, land as well (one
+    // that this thread has not seen complete may cost the wait's limit).
+    if (tid == 0 && (abort_run || s_late || a.give_up)) {
+        record_error(a.err, kDevWaitTimeout);
+        for (uint32_t k = max(waited, ncommit > 2 ? ncommit - 2 : 0u); k < ncommit; ++k)
+            (void)mbar_wait(&mbar, k & 1u);
     }
     tc_fence_before();
     __syncthreads();
@@ -866,6 +875,7 @@ cudaError_t launch_learned_step(const PencilMaps& maps, const float* p, float* n
     }
     a.b3 = net.b3;
     a.err = err;
+    a.give_up = net.give_up;
     return launch_after(learned_step_kernel, ctas, LNT, kLSmem, stream, maps.p, maps.prev, maps.vel2,
                         a);
 }

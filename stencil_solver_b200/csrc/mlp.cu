@@ -785,6 +785,7 @@ struct Mlp {
     float out_scale = 1.f;  // the correction is s * out_scale * y
     float min_scale = 0.f;  // correction floor: stars below it get no correction
     int kernel = 0;         // correction kernel: 0 = tcgen05, 1 = mma.sync
+    bool give_up = false;   // sb200_mlp_give_up_wait
     // Host copy of the FP32 parameters for the fused step, which takes biases
     // and w3 by value; stale after a device-side update (train_step).
     std::vector<float> host;
@@ -1081,6 +1082,7 @@ int learned_step_impl(void* h, const float* p, float* p_prev_next, const float* 
     net.b3 = m->host[OFF_B3];
     net.out_scale = m->out_scale;
     net.min_scale = m->min_scale;
+    net.give_up = m->give_up;
     return cuda_err(launch_learned_step(maps, p, p_prev_next, g, net, m->sms, err, st, flags_in,
                                         flags_out, box),
                     where);
@@ -1118,6 +1120,12 @@ int sb200_mlp_flags_compose(void* h, const sb200_grid* grid, const uint8_t* flag
     return cuda_err(launch_flags_compose(flags_p, flags_r, grid_desc(*grid), m->sms,
                                          static_cast<cudaStream_t>(stream)),
                     "sb200_mlp_flags_compose");
+}
+
+int sb200_mlp_give_up_wait(void* h, int on) {
+    if (!h) return set_error(SB200_ERR_INVALID, "sb200_mlp_give_up_wait: NULL handle");
+    static_cast<Mlp*>(h)->give_up = on != 0;
+    return SB200_OK;
 }
 
 int sb200_mlp_set_kernel(void* h, int kernel) {

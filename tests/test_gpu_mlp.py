@@ -513,3 +513,39 @@ def test_a_captured_training_step_zeroes_its_own_gradient(torch_cuda):
             want, _ = oracle.mlp_grad(before, X, t, round_bf16=True)
             assert abs(float(loss) - want) <= 1e-4 * want
             assert np.any(m.params() != before)
+
+
+@pytest.mark.parametrize("flagged", [False, True], ids=["unflagged", "flagged"])
+@pytest.mark.parametrize("shape", [(9, 44, 72), (20, 44, 72), (72, 260, 260)], ids=str)
+def test_learned_step_reports_a_wait_of_the_last_plane(torch_cuda, shape, flagged):
+    """A wait for the tensor cores that gives up in a chunk's last plane (chunks of one
+    plane, of a few, of many): the error is reported, flags_out stays unwritten, and the
+    next launch is sound."""
+    nz, ny, nx = shape
+    g = sb.Grid(nx, ny, nz, 10.0, 10.0, 10.0, 7e-4)
+    gen = torch_cuda.Generator(device="cuda")
+    gen.manual_seed(nz)
+    p, q = (torch_cuda.randn(shape, generator=gen, device="cuda") for _ in range(2))
+    v = torch_cuda.full(shape, 2.25e6, device="cuda")
+    with sb.Mlp(seed=4) as m:
+        n = m.flags_bytes(g)
+        ones = torch_cuda.full((n,), 255, dtype=torch_cuda.uint8, device="cuda")
+
+        def step(flags_out):
+            out = q.clone()
+            m.learned_step(p, out, v, g, flags=(ones, flags_out) if flagged else None)
+            torch_cuda.cuda.synchronize()
+            return out
+
+        want = step(torch_cuda.zeros_like(ones))
+        assert sb.device_error() == 0
+        for _ in range(2):
+            left = torch_cuda.full_like(ones, 0x55)
+            assert sb.lib().sb200_mlp_give_up_wait(m.handle, 1) == 0
+            step(left)
+            assert sb.device_error() > 0  # (cleared by this call)
+            assert (left == 0x55).all()
+            assert sb.lib().sb200_mlp_give_up_wait(m.handle, 0) == 0
+            out = torch_cuda.zeros_like(ones)
+            assert torch_cuda.equal(step(out), want) and sb.device_error() == 0
+            assert not flagged or bool(out.any())
