@@ -541,6 +541,25 @@ int dispatch_heat_f32(const float* u, float* u_next, const sb200_grid* grid, flo
                      exact ? "sb200_heat_step_exact_f32" : "sb200_heat_step_f32", sharing);
 }
 
+int prepare_step(const sb200_grid* grid, bool heat, bool half, bool exact, int sharing) {
+    GridDesc g;
+    if (int rc = to_desc(grid, &g)) return rc;
+    if (!g.has_interior()) return SB200_OK;
+    if (!device_error_ptr())
+        return fail(SB200_ERR_CUDA, "device error word unavailable");
+    if (half) {
+        pencil_f16_resident(choose(SB200_KIND_WAVE_F16, g, sharing).variant);
+    } else if (g.nx % 4 == 0 && (!exact || staged_pays(g, false))) {
+        const int kind = heat ? (exact ? int(kExactHeat) : int(SB200_KIND_HEAT_F32))
+                              : (exact ? int(kExactWave) : int(SB200_KIND_WAVE_F32));
+        pencil_f32_resident(heat, choose(kind, g, sharing).variant, exact);
+    } else if (staged_pays(g, true) && ragged_ok(g)) {
+        choose(heat ? kRaggedHeat : kRaggedWave, g, sharing);
+        ragged_resident(heat, g);
+    }
+    return SB200_OK;
+}
+
 int dispatch_wave2_f32(const float* p, const float* p_prev, const float* vel2, float* out1,
                        float* out2, const sb200_grid* grid, const SourceDesc& src, float w1,
                        void* stream, bool outputs_may_alias) {

@@ -19,6 +19,10 @@ int dispatch_wave_f32(const float* p, const float* p_prev, const float* vel2, fl
                       int sharing);
 int dispatch_heat_f32(const float* u, float* u_next, const sb200_grid* grid, float alpha,
                       void* stream, bool exact, int sharing);
+// Sets up what a step of the grid launches (16-byte aligned fields): the choice of kernel,
+// tile and split, kernel attributes, the error word.  Before a stream capture, whose launches
+// must not be the first ones.
+int prepare_step(const sb200_grid* grid, bool heat, bool half, bool exact, int sharing);
 // Two acoustic steps in one sweep (out1 = t+dt, out2 = t+2dt; w1 = the host
 // sample of the second step).  outputs_may_alias: out1 == out2 is accepted
 // (timing trials only: the values are then unusable).

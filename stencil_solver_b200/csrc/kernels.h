@@ -134,7 +134,6 @@ bool ragged_ok(const GridDesc& g);
 int64_t ragged_covered(const GridDesc& g);
 PencilBoxes ragged_boxes(bool heat, const GridDesc& g);
 int ragged_resident(bool heat, const GridDesc& g);
-void ragged_prepare();
 int64_t ragged_ctas(const GridDesc& g, int zchunks);
 cudaError_t launch_wave_ragged_f32(const PencilMaps& maps, float* next, const GridDesc& g,
                                    const SourceDesc& src, int zchunks, int* err,
@@ -161,10 +160,6 @@ cudaError_t launch_leap2_f32(const PencilMaps& maps, float* out1, float* out2, c
 // Resident CTAs per SM of a variant (occupancy query; analytic if that fails).
 // The first call per device also sets the variant's shared-memory attribute.
 int pencil_f32_resident(bool heat, int v, bool exact = false);
-// Sets up every variant on the current device (before a stream capture, whose
-// launches must not be the first ones).
-void pencil_f32_prepare(bool heat, bool exact);
-void pencil_f16_prepare();
 // Number of CTAs a launch uses (for occupancy/wave reasoning in the tuner).
 int64_t pencil_f32_ctas(bool heat, int v, const GridDesc& g, int zchunks);
 

@@ -685,9 +685,6 @@ PencilBoxes pencil_f16_boxes(int v) {
     return b;
 }
 int pencil_f16_resident(int v) { return kF16[v].resident(); }
-void pencil_f16_prepare() {
-    for (int v = 0; v < kNumF16; ++v) kF16[v].resident();
-}
 int64_t pencil_f16_ctas(int v, const GridDesc& g, int zchunks) {
     const int tiles_x = static_cast<int>((g.nx - R + kF16[v].tx - 1) / kF16[v].tx);
     const int tiles_y = static_cast<int>((g.ny - 2 * R + kF16[v].ty - 1) / kF16[v].ty);

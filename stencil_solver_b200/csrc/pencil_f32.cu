@@ -740,10 +740,6 @@ int pencil_f32_resident(bool heat, int v, bool exact) {
     return exact ? x.resident_exact() : x.resident();
 }
 
-void pencil_f32_prepare(bool heat, bool exact) {
-    for (int v = 0; v < (heat ? kNumHeat : kNumWave); ++v) pencil_f32_resident(heat, v, exact);
-}
-
 int64_t pencil_f32_ctas(bool heat, int v, const GridDesc& g, int zchunks) {
     return ctas_of(base_args(variant_of(heat, v).tx, variant_of(heat, v).ty, g, zchunks, nullptr), g);
 }

@@ -440,11 +440,6 @@ int ragged_resident(bool heat, const GridDesc& g) {
     return shape_for(g).resident[heat]();
 }
 
-void ragged_prepare() {
-    for (const Shape& s : kShapes)
-        for (auto* f : s.resident) f();
-}
-
 int64_t ragged_ctas(const GridDesc& g, int zchunks) {
     return ctas_of(make_args(nullptr, g, 0.f, zchunks, nullptr), g);
 }

@@ -549,19 +549,9 @@ private:
 
     int capture(cudaGraphExec_t* out) {
         const int C = c_.graph_chunk;
-        // Everything a launch sets up on first use (kernel attributes, occupancy
-        // queries, the kernel choice, tensor maps) happens before the capture.  Only of the
-        // kernels this run can take: a kernel's first query also loads its code.
-        if (fp16_)
-            pencil_f16_prepare();
-        else if (c_.grid.nx % 4 == 0)
-            pencil_f32_prepare(heat_, c_.exact != 0);
-        else
-            ragged_prepare();
-        int v = 0, z = 0;
-        sb200_pencil_choice(heat_ ? SB200_KIND_HEAT_F32
-                                  : (fp16_ ? SB200_KIND_WAVE_F16 : SB200_KIND_WAVE_F32),
-                            &c_.grid, &v, &z);
+        // The step's kernel is chosen and set up before the capture, and no other: a kernel's
+        // first query also loads its code.
+        if (int rc = prepare_step(&c_.grid, heat_, fp16_, c_.exact != 0, share_)) return rc;
         cudaGraph_t g = nullptr;
         if (int rc = cuda(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal))) return rc;
         int rc = SB200_OK;

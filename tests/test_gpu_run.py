@@ -346,3 +346,31 @@ def test_runs_at_once_take_no_longer_than_their_steps_alone(torch_cuda):
     for r in runs:
         r.close()
     assert together < 0.95 * alone
+
+
+def test_a_small_runs_first_graph_loads_its_own_kernels_only():
+    """The first steps of a 40^3 run in the reference's order (one thread per point), in a
+    process of its own: setting up the staged kernels it cannot take, whose code is large,
+    made them 23 ms; they are 2 to 5 without."""
+    import subprocess
+    import sys
+
+    code = """
+import time, numpy as np, stencil_solver_b200 as sb
+g = sb.Grid(40, 40, 40, 10.0, 10.0, 10.0, 7e-4)
+r = sb.Run(g, exact=1, graph_chunk=20)
+z = np.zeros(g.shape, np.float32)
+r.set_fields(z, z, np.full(g.shape, 4e6, np.float32))
+t = time.perf_counter()
+r.steps(20)
+r.synchronize()
+print("MS", (time.perf_counter() - t) * 1e3)
+"""
+    root = pathlib.Path(__file__).resolve().parents[1]
+    ms = []
+    for _ in range(3):
+        out = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True,
+                             timeout=300)
+        assert out.returncode == 0, out.stderr
+        ms.append(float(out.stdout.split("MS")[1]))
+    assert min(ms) < 12, ms
