@@ -275,11 +275,14 @@ PencilConfig cheapest(int family, const GridDesc& g, int sharing) {
 PencilConfig choose(int kind, const GridDesc& g, int sharing = kAlone) {
     {
         std::lock_guard<std::mutex> lock(g_cfg_mu);
-        // an override of a kind holds for all that run on its tiles
+        // an override of a kind holds for all that run on its tiles (the reference order keeps
+        // its own tile where it has no form of the given one)
         const Override o = tiles_of(kind) < 4 ? g_override[tiles_of(kind)] : Override();
         if (o.variant >= 0) {
             PencilConfig c;
-            c.variant = o.variant;
+            c.variant = !reference_order(kind) || pencil_f32_has_exact(kind == kExactHeat, o.variant)
+                            ? o.variant
+                            : cheapest(kind, g, sharing).variant;
             c.zchunks = std::max(1, o.zchunks);
             return c;
         }

@@ -160,6 +160,8 @@ cudaError_t launch_leap2_f32(const PencilMaps& maps, float* out1, float* out2, c
 // Resident CTAs per SM of a variant (occupancy query; analytic if that fails).
 // The first call per device also sets the variant's shared-memory attribute.
 int pencil_f32_resident(bool heat, int v, bool exact = false);
+// Whether a tile runs in the reference's operation order too.
+bool pencil_f32_has_exact(bool heat, int v);
 // Number of CTAs a launch uses (for occupancy/wave reasoning in the tuner).
 int64_t pencil_f32_ctas(bool heat, int v, const GridDesc& g, int zchunks);
 

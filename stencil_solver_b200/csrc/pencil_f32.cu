@@ -37,6 +37,7 @@
 // write p_next), heat 8 B (read u, write u_next), prepass 20 B (read p, p_prev,
 // vel2; write r, p_prev).
 #include <algorithm>
+#include <utility>
 #include <mutex>
 
 #include "batch.h"
@@ -613,7 +614,7 @@ struct Variant {
     LaunchFn launch;
     ResidentFn resident;
     LaunchFn launch_prepass;  // acoustic tiles only: the same shape in prepass mode
-    LaunchFn launch_exact;    // the same shape in the reference's operation order
+    LaunchFn launch_exact;    // the same shape in the reference's operation order, or NULL
     ResidentFn resident_exact;
 };
 
@@ -626,37 +627,49 @@ constexpr LaunchFn prepass_launcher() {
         return &launch_variant<TX, TY, RPT, S, AUX, kModePrepass>;
 }
 
-#define SB200_VARIANT(TX, TY, RPT, S, AUX, HEAT, NAME)                                       \
+// The reference order's functions of a tile: instantiated for those that its untuned choice
+// takes from (capi.cu).  Nothing else reaches them, and all 17 made the code that a process'
+// first step loads take 23 ms instead of 17.
+template <int TX, int TY, int RPT, int S, int AUX, bool HEAT, bool EXACT>
+constexpr std::pair<LaunchFn, ResidentFn> exact_functions() {
+    if constexpr (EXACT)
+        return {&launch_variant<TX, TY, RPT, S, AUX, HEAT ? kModeHeatExact : kModeExact>,
+                &resident_variant<TX, TY, RPT, S, AUX, HEAT ? kModeHeatExact : kModeExact>};
+    else
+        return {nullptr, nullptr};
+}
+
+#define SB200_VARIANT(TX, TY, RPT, S, AUX, HEAT, EXACT, NAME)                                \
     Variant {                                                                                \
         TX, TY, RPT, S, AUX, NAME,                                                           \
             &launch_variant<TX, TY, RPT, S, AUX, HEAT ? kModeHeat : kModeAcoustic>,          \
             &resident_variant<TX, TY, RPT, S, AUX, HEAT ? kModeHeat : kModeAcoustic>,        \
             prepass_launcher<TX, TY, RPT, S, AUX, HEAT>(),                                   \
-            &launch_variant<TX, TY, RPT, S, AUX, HEAT ? kModeHeatExact : kModeExact>,        \
-            &resident_variant<TX, TY, RPT, S, AUX, HEAT ? kModeHeatExact : kModeExact>       \
+            exact_functions<TX, TY, RPT, S, AUX, HEAT, EXACT>().first,                       \
+            exact_functions<TX, TY, RPT, S, AUX, HEAT, EXACT>().second                       \
     }
 
-// Index 0 of each table is the default when no tuned choice exists.
+// Tiles are only appended: tuned files name them by index.
 const Variant kWave[] = {
-    SB200_VARIANT(32, 32, 2, 8, 4, false, "t32x32_r2_s8_a4"),
-    SB200_VARIANT(32, 32, 2, 8, 2, false, "t32x32_r2_s8_a2"),
-    SB200_VARIANT(32, 32, 2, 8, 0, false, "t32x32_r2_s8_ldg"),
-    SB200_VARIANT(64, 16, 2, 8, 3, false, "t64x16_r2_s8_a3"),
-    SB200_VARIANT(32, 16, 1, 8, 4, false, "t32x16_r1_s8_a4"),
-    SB200_VARIANT(64, 32, 2, 8, 3, false, "t64x32_r2_s8_a3"),
-    SB200_VARIANT(32, 64, 2, 8, 3, false, "t32x64_r2_s8_a3"),
-    SB200_VARIANT(64, 32, 2, 6, 2, false, "t64x32_r2_s6_a2"),
-    SB200_VARIANT(128, 16, 2, 6, 2, false, "t128x16_r2_s6_a2"),
-    SB200_VARIANT(128, 32, 2, 7, 2, false, "t128x32_r2_s7_a2"),
+    SB200_VARIANT(32, 32, 2, 8, 4, false, false, "t32x32_r2_s8_a4"),
+    SB200_VARIANT(32, 32, 2, 8, 2, false, false, "t32x32_r2_s8_a2"),
+    SB200_VARIANT(32, 32, 2, 8, 0, false, false, "t32x32_r2_s8_ldg"),
+    SB200_VARIANT(64, 16, 2, 8, 3, false, false, "t64x16_r2_s8_a3"),
+    SB200_VARIANT(32, 16, 1, 8, 4, false, true, "t32x16_r1_s8_a4"),
+    SB200_VARIANT(64, 32, 2, 8, 3, false, false, "t64x32_r2_s8_a3"),
+    SB200_VARIANT(32, 64, 2, 8, 3, false, false, "t32x64_r2_s8_a3"),
+    SB200_VARIANT(64, 32, 2, 6, 2, false, true, "t64x32_r2_s6_a2"),
+    SB200_VARIANT(128, 16, 2, 6, 2, false, true, "t128x16_r2_s6_a2"),
+    SB200_VARIANT(128, 32, 2, 7, 2, false, true, "t128x32_r2_s7_a2"),
 };
 const Variant kHeat[] = {
-    SB200_VARIANT(32, 32, 2, 8, 0, true, "t32x32_r2_s8"),
-    SB200_VARIANT(64, 16, 2, 8, 0, true, "t64x16_r2_s8"),
-    SB200_VARIANT(32, 16, 1, 8, 0, true, "t32x16_r1_s8"),
-    SB200_VARIANT(64, 32, 2, 8, 0, true, "t64x32_r2_s8"),
-    SB200_VARIANT(32, 64, 2, 8, 0, true, "t32x64_r2_s8"),
-    SB200_VARIANT(128, 16, 2, 8, 0, true, "t128x16_r2_s8"),
-    SB200_VARIANT(128, 32, 2, 8, 0, true, "t128x32_r2_s8"),
+    SB200_VARIANT(32, 32, 2, 8, 0, true, false, "t32x32_r2_s8"),
+    SB200_VARIANT(64, 16, 2, 8, 0, true, true, "t64x16_r2_s8"),
+    SB200_VARIANT(32, 16, 1, 8, 0, true, true, "t32x16_r1_s8"),
+    SB200_VARIANT(64, 32, 2, 8, 0, true, false, "t64x32_r2_s8"),
+    SB200_VARIANT(32, 64, 2, 8, 0, true, false, "t32x64_r2_s8"),
+    SB200_VARIANT(128, 16, 2, 8, 0, true, false, "t128x16_r2_s8"),
+    SB200_VARIANT(128, 32, 2, 8, 0, true, false, "t128x32_r2_s8"),
 };
 constexpr int kNumWave = sizeof(kWave) / sizeof(kWave[0]);
 constexpr int kNumHeat = sizeof(kHeat) / sizeof(kHeat[0]);
@@ -734,6 +747,8 @@ PencilBoxes pencil_f32_boxes(bool heat, int v) {
     b.aux_tma = !heat && x.aux > 0;
     return b;
 }
+
+bool pencil_f32_has_exact(bool heat, int v) { return variant_of(heat, v).launch_exact != nullptr; }
 
 int pencil_f32_resident(bool heat, int v, bool exact) {
     const Variant& x = variant_of(heat, v);

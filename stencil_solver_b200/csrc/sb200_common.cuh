@@ -191,20 +191,6 @@ __device__ __forceinline__ void stg_stream(float* p, float4 v) {
                  : "memory");
 }
 
-__device__ __forceinline__ uint4 ldg_stream_u4(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p));
-    return v;
-}
-
-__device__ __forceinline__ void stg_stream_u4(void* p, uint4 v) {
-    asm volatile("st.global.cs.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y),
-                 "r"(v.z), "r"(v.w)
-                 : "memory");
-}
-
 __device__ __forceinline__ float4 lds128(const float* p) {
     return *reinterpret_cast<const float4*>(p);
 }
