@@ -241,7 +241,8 @@ int sb200_field_stats_f32_noalloc(const float* field, const sb200_grid* grid, do
 int sb200_pencil_variant_count(int kind);
 const char* sb200_pencil_variant_name(int kind, int variant);
 /* Forces (variant, zchunks) for every later launch of `kind` on this process;
- * variant < 0 restores automatic selection. */
+ * variant < 0 restores automatic selection.  Steps of grids with nx % 4 != 0 take the z split of
+ * their kind only. */
 int sb200_set_pencil_override(int kind, int variant, int zchunks);
 /* The (variant, zchunks) the next launch of `kind` on `grid` would use. */
 int sb200_pencil_choice(int kind, const sb200_grid* grid, int* variant, int* zchunks);

@@ -185,11 +185,11 @@ struct Family {
 // composition pre-pass, and the ragged kernels.
 enum Internal : int { kExactWave = 4, kExactHeat, kPrepass, kRaggedWave, kRaggedHeat };
 bool reference_order(int kind) { return kind == kExactWave || kind == kExactHeat; }
-// The public kind whose tiles a kind runs on.
-int tiles_of(int kind) {
-    return kind == kExactHeat ? SB200_KIND_HEAT_F32
-           : kind == kExactWave || kind == kPrepass ? SB200_KIND_WAVE_F32
-                                                    : kind;
+// The public kind whose override holds for a kind (of the ragged kernels, its z split).
+int public_kind(int kind) {
+    return kind == kExactHeat || kind == kRaggedHeat ? SB200_KIND_HEAT_F32
+           : kind >= kExactWave                      ? SB200_KIND_WAVE_F32
+                                                     : kind;
 }
 
 const Family kFamilies[] = {
@@ -245,7 +245,7 @@ PencilConfig cheapest(int family, const GridDesc& g, int sharing) {
     if (family == kPrepass && !beyond) family = SB200_KIND_WAVE_F32;
     const Family& f = kFamilies[family];
     const bool exact = reference_order(family);
-    const int kind = tiles_of(family);
+    const int kind = public_kind(family);
     PencilConfig best;
     double cost = 0;
     for (const Candidate& c : f.tiles) {
@@ -275,9 +275,8 @@ PencilConfig cheapest(int family, const GridDesc& g, int sharing) {
 PencilConfig choose(int kind, const GridDesc& g, int sharing = kAlone) {
     {
         std::lock_guard<std::mutex> lock(g_cfg_mu);
-        // an override of a kind holds for all that run on its tiles (the reference order keeps
-        // its own tile where it has no form of the given one)
-        const Override o = tiles_of(kind) < 4 ? g_override[tiles_of(kind)] : Override();
+        // (the reference order keeps its own tile where it has no form of the given one)
+        const Override o = g_override[public_kind(kind)];
         if (o.variant >= 0) {
             PencilConfig c;
             c.variant = !reference_order(kind) || pencil_f32_has_exact(kind == kExactHeat, o.variant)
@@ -288,7 +287,7 @@ PencilConfig choose(int kind, const GridDesc& g, int sharing = kAlone) {
         }
     }
     PencilConfig c;
-    if ((kind < 4 || kind == kPrepass) && tuned_choice(tiles_of(kind), g, &c)) return c;
+    if ((kind < 4 || kind == kPrepass) && tuned_choice(public_kind(kind), g, &c)) return c;
     // Heuristic pick, memoised per (kind, extents, device, sharing): launches stay cheap
     // on the host.
     static std::mutex memo_mu;

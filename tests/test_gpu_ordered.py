@@ -127,3 +127,72 @@ def test_few_rows_take_no_longer_than_one_thread_per_point(torch_cuda, shape):
         return best
 
     assert step_us(0) <= 1.4 * step_us(1)
+
+
+# both tiles of the ragged kernel: 32 x 32 and 64 x 16
+@pytest.mark.parametrize("nx, ny, nz", [(89, 88, 88), (69, 88, 110)], ids=["32x32", "64x16"])
+@pytest.mark.parametrize("heat", [False, True], ids=["acoustic", "heat"])
+def test_ragged_splits_bit_for_bit(torch_cuda, heat, nx, ny, nz):
+    """Chunks of 1, 2, 3, 7, 8, 9, 16, 17 planes (around its groups of 4 and unroll of 8) and
+    one of all."""
+    d, dt = (10.0, 7.5, 12.0), np.float32(1e-3)
+    g = sb.Grid(nx, ny, nz, *d, float(dt))
+    cur, prev, vel2 = case(g.shape, nx)
+    dev = [torch_cuda.from_numpy(a).cuda() for a in (cur, prev, vel2)]
+    if heat:
+        k = np.full(g.shape, np.float32(900.0) * dt, np.float32)
+        ref = oracle.wave_step(cur, cur, k, *d, np.float32(1.0), out=prev.copy())
+    else:
+        ref = oracle.wave_step(cur, prev, vel2, *d, dt, out=prev.copy())
+    kind = sb.KIND_HEAT_F32 if heat else sb.KIND_WAVE_F32
+    inz = nz - 8
+    try:
+        for planes in (1, 2, 3, 7, 8, 9, 16, 17, inz):
+            sb.set_pencil_override(kind, 0, -(-inz // planes))
+            out = dev[1].clone()
+            if heat:
+                sb.heat_step(dev[0], out, g, 900.0)
+            else:
+                sb.wave_step(dev[0], out, dev[2], out, g)
+            assert np.array_equal(out.cpu().numpy(), ref), planes
+    finally:
+        sb.set_pencil_override(kind, -1, 1)
+    assert sb.device_error() == 0
+
+
+@pytest.mark.parametrize("nx, ny, nz", [(89, 88, 88), (69, 88, 110), (41, 40, 44)],
+                         ids=["32x32", "64x16", "one thread per point"])
+def test_ragged_runs_bit_for_bit(torch_cuda, nx, ny, nz):
+    """Whole runs on ragged rows: the source's sample and the trace through the device's step
+    counter, eager and in graphs entered at both parities, against the oracle; heat alike."""
+    d, dt = (10.0, 7.5, 12.0), np.float32(7e-4)
+    g = sb.Grid(nx, ny, nz, *d, float(dt))
+    cur, prev, vel2 = case(g.shape, nz)
+    src = g.index(nx - 6, 5, nz // 2)
+    pieces = (3, 20, 1, 21, 4)
+    n = sum(pieces)
+    w = np.random.default_rng(2).uniform(-1, 1, n).astype(np.float32)
+    a, b = cur.copy(), prev.copy()
+    trace = np.zeros(n, np.float32)
+    for k in range(n):
+        out = oracle.wave_step(a, b, vel2, *d, dt, out=b.copy())
+        out.reshape(-1)[src] += np.float32(dt * dt) * vel2.reshape(-1)[src] * w[k]
+        trace[k] = out.reshape(-1)[src]
+        a, b = out, a
+    kv = np.full(g.shape, np.float32(900.0) * dt, np.float32)
+    u = cur
+    for k in range(n):
+        u = oracle.wave_step(u, u, kv, *d, np.float32(1.0), out=u.copy())
+    for chunk in (0, 20):
+        with sb.Run(g, src_index=src, graph_chunk=chunk) as r:
+            r.set_fields(cur, prev, vel2)
+            r.set_wavelet(w)
+            for k in pieces:
+                r.steps(k)
+            assert np.array_equal(r.field(), a) and np.array_equal(r.trace(n), trace), chunk
+        with sb.Run(g, physics=sb.PHYSICS_HEAT, diffusivity=900.0, graph_chunk=chunk) as r:
+            r.set_fields(cur)
+            for k in pieces:
+                r.steps(k)
+            assert np.array_equal(r.field(), u), chunk
+    assert sb.device_error() == 0
