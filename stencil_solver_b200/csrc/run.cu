@@ -43,7 +43,7 @@ __global__ void monitor_kernel(const double* stats3, int* flag, double limit) {
 // Per device: runs with steps queued that nobody has waited for.
 std::atomic<int> g_busy[64] = {};
 
-constexpr int64_t kStageFloats = int64_t(1) << 24;  // host <-> device staging: up to 64 MB
+constexpr int64_t kStageFloats = int64_t(1) << 24;  // host <-> device staging: up to 64 MB kept
 
 class Run {
 public:
@@ -149,12 +149,13 @@ public:
             return wait();
         }
         // FP16: initial scale from the fields' largest magnitude, taken on the device as
-        // their chunks pass through the staging buffer, and the first window's source.
-        // Fields of one chunk stay staged (one half each); longer ones are copied again
-        // to be packed.
-        const bool same = p_prev == p, held = stage_holds();
+        // their chunks pass through the staging buffer, and the first window's source.  p of
+        // one chunk stays staged, and p_prev beside it where the device has the room for the
+        // length of this call; what does not is copied again to be packed.
+        const bool same = p_prev == p, held = n_ <= kStageFloats;
+        const Scratch beside(held && !same ? n_ * 4 : 0, st_);
         double m = 0.0;
-        if (int rc = stage_max(p, same ? nullptr : p_prev, &m)) return rc;
+        if (int rc = stage_max(p, same ? nullptr : p_prev, beside.p, &m)) return rc;
         vel2_host_src_ = c_.src_index >= 0 ? vel2[c_.src_index] : 0.f;
         rebuild_bound();
         const double bnd = bound_host_.empty() ? 0.0 : bound_host_[0];
@@ -166,18 +167,13 @@ public:
         // on the run's stream: steps still queued there read the scale
         if (int rc = cuda(cudaMemcpyAsync(scale_dev_, &s0, sizeof(s0), cudaMemcpyHostToDevice, st_)))
             return rc;
-        if (held) {
-            if (int rc = sb200_f16_pack(stage_, static_cast<uint16_t*>(a_), n_, float(a0), st_))
+        if (int rc = held ? sb200_f16_pack(stage_, static_cast<uint16_t*>(a_), n_, float(a0), st_)
+                          : stage_in(p, a_, float(a0), false))
+            return rc;
+        if (!same)
+            if (int rc = beside.p ? sb200_f16_pack(beside.p, static_cast<uint16_t*>(b_), n_, float(a0), st_)
+                                  : stage_in(p_prev, b_, float(a0), false))
                 return rc;
-            if (!same)
-                if (int rc = sb200_f16_pack(stage_ + stage_half(), static_cast<uint16_t*>(b_), n_,
-                                            float(a0), st_))
-                    return rc;
-        } else {
-            if (int rc = stage_in(p, a_, float(a0), false)) return rc;
-            if (!same)
-                if (int rc = stage_in(p_prev, b_, float(a0), false)) return rc;
-        }
         if (same)
             if (int rc = cuda(cudaMemcpyAsync(b_, a_, n_ * 2, cudaMemcpyDeviceToDevice, st_))) return rc;
         if (int rc = stage_in(vel2, k_, 1.f, true)) return rc;
@@ -336,29 +332,41 @@ private:
         return rc;
     }
 
-    // Staging: one chunk of kStageFloats values, or two whole fields where they are no
-    // longer than a chunk.
-    bool stage_holds() const { return n_ <= kStageFloats; }
-    int64_t stage_half() const { return stage_holds() ? (n_ + 63) / 64 * 64 : 0; }
+    // Device memory for the length of one call, in order on the stream; NULL where there is
+    // none to be had.
+    struct Scratch {
+        Scratch(size_t bytes, cudaStream_t st) : st(st) {
+            if (bytes && cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, st) != cudaSuccess) {
+                cudaGetLastError();
+                p = nullptr;
+            }
+        }
+        ~Scratch() {
+            if (p) cudaFreeAsync(p, st);
+        }
+        Scratch(const Scratch&) = delete;
+        Scratch& operator=(const Scratch&) = delete;
+        float* p = nullptr;
+        cudaStream_t st;
+    };
+
     int ensure_stage() {
         if (stage_) return SB200_OK;
-        return alloc(reinterpret_cast<void**>(&stage_),
-                     size_t(stage_holds() ? 2 * stage_half() : kStageFloats) * 4);
+        return alloc(reinterpret_cast<void**>(&stage_), size_t(std::min(n_, kStageFloats)) * 4);
     }
 
     // *m = max |value| of the host fields p and q (q may be NULL), chunk by chunk through
-    // the staging buffer; where it holds both fields they are left there, q in the second
-    // half.
-    int stage_max(const float* p, const float* q, double* m) {
+    // the staging buffer (q of one chunk through `beside`, unless NULL); p's last chunk is
+    // left there.
+    int stage_max(const float* p, const float* q, float* beside, double* m) {
         if (int rc = ensure_stage()) return rc;
         unsigned* bits = reinterpret_cast<unsigned*>(stats_dev_);  // free between steps
         if (int rc = cuda(cudaMemsetAsync(bits, 0, sizeof(unsigned), st_))) return rc;
-        for (int64_t off = 0; off < n_; off += kStageFloats) {
-            const int64_t c = std::min(kStageFloats, n_ - off);
-            for (int h = 0; h < (q ? 2 : 1); ++h) {
-                float* d = stage_ + h * stage_half();
-                if (int rc = cuda(cudaMemcpyAsync(d, (h ? q : p) + off, c * 4,
-                                                  cudaMemcpyHostToDevice, st_)))
+        for (const float* f : {q, p}) {
+            float* d = f == q && beside ? beside : stage_;
+            for (int64_t off = 0; f && off < n_; off += kStageFloats) {
+                const int64_t c = std::min(kStageFloats, n_ - off);
+                if (int rc = cuda(cudaMemcpyAsync(d, f + off, c * 4, cudaMemcpyHostToDevice, st_)))
                     return rc;
                 if (int rc = cuda(launch_absmax(d, c, bits, st_))) return rc;
             }

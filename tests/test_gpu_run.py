@@ -374,3 +374,30 @@ print("MS", (time.perf_counter() - t) * 1e3)
         assert out.returncode == 0, out.stderr
         ms.append(float(out.stdout.split("MS")[1]))
     assert min(ms) < 12, ms
+
+
+def test_fp16_fields_of_two_levels_keep_64_mb_of_staging(torch_cuda):
+    """A 256^3 FP16 run given two distinct levels: its bits, and what it holds on the device
+    afterwards (three fields of 2 bytes and one staging chunk; it was two)."""
+    n = 256
+    g = sb.Grid(n, n, n, 10.0, 10.0, 10.0, 7e-4)
+    p = np.random.default_rng(1).integers(-9, 10, g.shape).astype(np.float32)  # exact in FP16
+    q = np.zeros(g.shape, np.float32)
+    v = np.full(g.shape, 2.25e6, np.float32)
+
+    def make():
+        r = sb.Run(g, precision=sb.PRECISION_F16)
+        r.set_fields(p, q, v)
+        return r
+
+    make().close()  # the process' first loads its kernels
+    torch_cuda.cuda.synchronize()
+    free = torch_cuda.cuda.mem_get_info()[0]
+    with make() as r:
+        torch_cuda.cuda.synchronize()
+        held = free - torch_cuda.cuda.mem_get_info()[0]
+        assert np.array_equal(r.field(), p)
+        want = 2 * p - q  # one step but for its Laplacian term, at most 2: both levels arrived
+        r.steps(1)
+        assert np.abs(r.field() - want)[4:-4, 4:-4, 4:-4].max() < 8
+    assert held <= 3 * 2 * n ** 3 + (64 << 20) + (24 << 20), held
