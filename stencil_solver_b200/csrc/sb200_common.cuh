@@ -47,8 +47,9 @@ constexpr long long kWaitLimitCycles = 2000000000LL;
 // aside).  The launch may then begin as the blocks of the stream's previous kernel
 // exit, before its completion is flushed; launch_order() waits in hardware for that
 // completion, so stream order holds as in a plain launch.  Plain back-to-back launches
-// repeat in steps of 2.05 us on B200, 1 to 3 us above the kernel's own time (5.1 us of
-// work: 8.2 us); these repeat 0.8 us above it (5.9 us).
+// repeat in steps of 2.05 us on B200, 1 to 3 us above the kernel's own time (a spin of 5.15
+// us on 148 blocks: 8.2 us); these repeat 0.5 us above it (5.7 us).  In a graph it is 0.5
+// us either way.  A launch whose predecessor has ended gains nothing.
 // No kernel triggers its dependents early (griddepcontrol.launch_dependents): blocks of
 // the next grid then settle on the SMs the running one leaves idle, several on one,
 // instead of spreading out (120 x 153 x 115 heat: 8.2 us plain, 9.0 us with the trigger
