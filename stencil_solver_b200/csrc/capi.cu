@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <cmath>
 #include <cstdio>
@@ -220,6 +221,7 @@ const Family kFamilies[] = {
     {10, 12, {{"t64x32_r2_s8_a3", 0, 1.02}, {"t128x32_r2_s7_a2", 0, 0.96}}, "", ""},
 };
 constexpr double kL2Bytes = 126e6;
+constexpr int64_t kSharedCells = 48000000;
 
 int variant_by_name(int kind, const char* name) {
     for (int v = 0; v < variant_count(kind); ++v)
@@ -272,6 +274,32 @@ PencilConfig cheapest(int family, const GridDesc& g, int sharing) {
     return best;
 }
 
+// For steps whose caller says nothing of others: the streams, other than `stream`, that the
+// last 16 of them on the device went to.  Steps of unlike grids on several streams meet on
+// the SMs as runs do (four of 96 to 192 cells 55.8 us a round with each its own choice, 40.5
+// before the cost model, 32.9 now).
+constexpr int kFromStreams = -1;
+int streams_beside(void* stream) {
+    constexpr unsigned kLast = 16;
+    struct Ring {
+        std::atomic<uintptr_t> stream[kLast] = {};  // + 1; 0: none yet
+        std::atomic<unsigned> at{0};
+    };
+    static Ring rings[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    Ring& r = rings[dev & 63];
+    const uintptr_t mine = reinterpret_cast<uintptr_t>(stream) + 1;
+    r.stream[r.at.fetch_add(1, std::memory_order_relaxed) % kLast].store(mine, std::memory_order_relaxed);
+    uintptr_t seen[kLast];
+    int n = 0;
+    for (auto& s : r.stream) {
+        const uintptr_t v = s.load(std::memory_order_relaxed);
+        if (v && v != mine && std::find(seen, seen + n, v) == seen + n) seen[n++] = v;
+    }
+    return n;
+}
+
 PencilConfig choose(int kind, const GridDesc& g, int sharing = kAlone) {
     {
         std::lock_guard<std::mutex> lock(g_cfg_mu);
@@ -286,6 +314,10 @@ PencilConfig choose(int kind, const GridDesc& g, int sharing = kAlone) {
             return c;
         }
     }
+    // steps that fill the device many times over gain nothing by agreeing on a tile (four of
+    // 384 to 640 cells, each its own and shared: acoustic 1225 and 1289 us, heat 767 and 852,
+    // reference order 1459 and 1588; of 200 to 320 cells 148.8 and 148.6, eight 383 and 353)
+    if (g.size() > kSharedCells) sharing = kAlone;
     PencilConfig c;
     if ((kind < 4 || kind == kPrepass) && tuned_choice(public_kind(kind), g, &c)) return c;
     // Heuristic pick, memoised per (kind, extents, device, sharing): launches stay cheap
@@ -389,7 +421,7 @@ int ragged_maps(bool heat, const GridDesc& g, const void* field, const void* pre
 
 int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_next,
               const sb200_grid* grid, const SourceDesc& src, void* stream, bool exact,
-              const char* where, int sharing = kAlone) {
+              const char* where, int sharing = kFromStreams) {
     const int64_t src_index = src.idx;
     GridDesc g;
     if (int rc = to_desc(grid, &g)) return rc;
@@ -400,6 +432,7 @@ int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_n
     if (src_index >= g.size())
         return fail(SB200_ERR_INVALID, std::string(where) + ": source index outside the grid");
     if (!g.has_interior()) return SB200_OK;  // no interior point: nothing to update
+    if (sharing == kFromStreams) sharing = sharing_of(streams_beside(stream));
     auto st = static_cast<cudaStream_t>(stream);
     if ((!exact || staged_pays(g, false)) && pencil_ok(g, {p, p_prev, vel2, p_next})) {
         const PencilConfig cfg = choose(exact ? int(kExactWave) : int(SB200_KIND_WAVE_F32), g, sharing);
@@ -421,7 +454,7 @@ int wave_step(const float* p, const float* p_prev, const float* vel2, float* p_n
 }
 
 int heat_step(const float* u, float* u_next, const sb200_grid* grid, float alpha, void* stream,
-              bool exact, const char* where, int sharing = kAlone) {
+              bool exact, const char* where, int sharing = kFromStreams) {
     GridDesc g;
     if (int rc = to_desc(grid, &g)) return rc;
     if (!u || !u_next) return fail(SB200_ERR_INVALID, std::string(where) + ": NULL field pointer");
@@ -430,6 +463,7 @@ int heat_step(const float* u, float* u_next, const sb200_grid* grid, float alpha
     if (!std::isfinite(alpha))
         return fail(SB200_ERR_INVALID, std::string(where) + ": alpha must be finite");
     if (!g.has_interior()) return SB200_OK;
+    if (sharing == kFromStreams) sharing = sharing_of(streams_beside(stream));
     const float alpha_dt = alpha * g.dt;
     auto st = static_cast<cudaStream_t>(stream);
     PencilMaps maps;
@@ -494,7 +528,7 @@ SourceDesc host_source(int64_t idx, float amp) {
 
 int wave_step_f16(const uint16_t* p, uint16_t* p_prev_next, const uint16_t* k,
                   const sb200_grid* grid, const SourceDesc& src, const sb200_f16_scale* scale,
-                  int phase, void* stream, int sharing = kAlone) {
+                  int phase, void* stream, int sharing = kFromStreams) {
     const char* where = "sb200_wave_step_f16";
     GridDesc g;
     if (int rc = to_desc(grid, &g)) return rc;
@@ -511,6 +545,7 @@ int wave_step_f16(const uint16_t* p, uint16_t* p_prev_next, const uint16_t* k,
     if (g.nx % 8 != 0 || !aligned16(p) || !aligned16(p_prev_next) || !aligned16(k))
         return fail(SB200_ERR_UNSUPPORTED,
                     std::string(where) + ": needs nx % 8 == 0 and 16-byte aligned fields");
+    if (sharing == kFromStreams) sharing = sharing_of(streams_beside(stream));
     const PencilConfig cfg = choose(SB200_KIND_WAVE_F16, g, sharing);
     const PencilBoxes b = pencil_f16_boxes(cfg.variant);
     PencilMaps maps;

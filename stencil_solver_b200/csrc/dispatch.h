@@ -10,9 +10,10 @@
 
 namespace sb200 {
 
-// Beside how many other runs an untuned step is made: at most one, two or three, four and
-// more.  Its tile and z split follow that, its bits do not.
+// Beside how many others' steps an untuned step is made: at most one's, two or three, four
+// and more.  Its tile and z split follow that, its bits do not.
 enum Sharing : int { kAlone = 0, kFew, kMany };
+inline int sharing_of(int others) { return others < 2 ? kAlone : others < 4 ? kFew : kMany; }
 
 int dispatch_wave_f32(const float* p, const float* p_prev, const float* vel2, float* p_next,
                       const sb200_grid* grid, const SourceDesc& src, void* stream, bool exact,

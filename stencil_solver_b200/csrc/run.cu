@@ -202,8 +202,7 @@ public:
                 return set_error(SB200_ERR_INVALID, "sb200_run_steps: wavelet shorter than the run");
             }
         }
-        const int beside = std::max(others(), seen_);
-        share_ = beside < 2 ? kAlone : beside < 4 ? kFew : kMany;
+        share_ = sharing_of(std::max(others(), seen_));
         if (n > 0) set_busy(true);
         const int C = c_.graph_chunk;
         int64_t done = 0;

@@ -113,3 +113,51 @@ def test_steps_behind_a_join_of_two_streams(torch_cuda, captured, kind, branch):
         torch.cuda.synchronize()
         for got, w in zip((a, b, out, last), want):
             assert torch.equal(got, w)
+
+
+@pytest.mark.parametrize("kind", ["wave", "exact", "heat", "half", "ragged"])
+def test_steps_on_five_streams_give_the_bits_of_one(torch_cuda, kind):
+    """Rounds of steps of unlike grids, each on its own stream (from the third stream on they
+    take another tile and split than alone), against each grid by itself."""
+    torch = torch_cuda
+    shapes = [(96, 88, 80), (128, 64, 100), (160, 72, 61), (64, 120, 90), (200, 48, 77)]
+    sets = []
+    for k, (nx, ny, nz) in enumerate(shapes):
+        g = sb.Grid(nx + (kind == "ragged"), ny, nz, 10.0, 10.0, 10.0, 7e-4)
+        p, q, v = fields(torch, g, k, 3)
+        v.square_().add_(1.0).mul_(1e6)
+        if kind == "half":
+            halves = [torch.empty(g.shape, dtype=torch.int16, device="cuda") for _ in range(3)]
+            sb.f16_pack(p, halves[0], g.size, 256.0)
+            sb.f16_pack(q, halves[1], g.size, 256.0)
+            sb.k_field_bf16(v, halves[2], g)
+            p, q, v = halves
+        sets.append((g, p, q, v, torch.tensor([256.0, 1.0], device="cuda")))
+
+    def run(g, p, q, v, scale, stream, rounds=7):
+        for _ in range(rounds):
+            if kind == "half":
+                sb.wave_step_f16(p, q, v, g, scale, stream=stream)
+            elif kind == "heat":
+                sb.heat_step(p, q, g, 1.0, stream=stream)
+            else:
+                (sb.wave_step_exact if kind == "exact" else sb.wave_step)(p, q, v, q, g, stream=stream)
+            p, q = q, p
+        return p
+
+    want = []
+    for g, p, q, v, scale in sets:
+        for _ in range(4):  # 28 launches on one stream: alone
+            one = run(g, p.clone(), q.clone(), v, scale, None)
+        want.append(one)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in sets]
+    state = [[p.clone(), q.clone()] for _, p, q, _, _ in sets]
+    torch.cuda.synchronize()
+    for _ in range(7):
+        for (g, _, _, v, scale), s, pq in zip(sets, streams, state):
+            run(g, pq[0], pq[1], v, scale, s, 1)
+            pq.reverse()
+    torch.cuda.synchronize()
+    for pq, w in zip(state, want):
+        assert torch.equal(pq[0], w)
