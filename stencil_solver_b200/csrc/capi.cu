@@ -274,13 +274,14 @@ PencilConfig cheapest(int family, const GridDesc& g, int sharing) {
     return best;
 }
 
-// For steps whose caller says nothing of others: the streams, other than `stream`, that the
-// last 16 of them on the device went to.  Steps of unlike grids on several streams meet on
-// the SMs as runs do (four of 96 to 192 cells 55.8 us a round with each its own choice, 40.5
-// before the cost model, 32.9 now).
+// For steps whose caller says nothing of others: the other streams (up to 4) that steps on
+// the device went to since the last one on `stream`, if that is among the last 32 (the
+// first step on a stream, a capture's for instance, is taken to be alone).  Steps of unlike
+// grids on several streams meet on the SMs as runs do (four of 96 to 192 cells 55.8 us a
+// round with each its own choice, 40.5 before the cost model, 33.3 now).
 constexpr int kFromStreams = -1;
 int streams_beside(void* stream) {
-    constexpr unsigned kLast = 16;
+    constexpr unsigned kLast = 32;
     struct Ring {
         std::atomic<uintptr_t> stream[kLast] = {};  // + 1; 0: none yet
         std::atomic<unsigned> at{0};
@@ -290,14 +291,17 @@ int streams_beside(void* stream) {
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     Ring& r = rings[dev & 63];
     const uintptr_t mine = reinterpret_cast<uintptr_t>(stream) + 1;
-    r.stream[r.at.fetch_add(1, std::memory_order_relaxed) % kLast].store(mine, std::memory_order_relaxed);
-    uintptr_t seen[kLast];
+    const unsigned at = r.at.fetch_add(1, std::memory_order_relaxed);
+    uintptr_t seen[4];
     int n = 0;
-    for (auto& s : r.stream) {
-        const uintptr_t v = s.load(std::memory_order_relaxed);
-        if (v && v != mine && std::find(seen, seen + n, v) == seen + n) seen[n++] = v;
+    bool again = false;
+    for (unsigned k = 1; k < kLast && !again; ++k) {
+        const uintptr_t v = r.stream[(at - k) % kLast].load(std::memory_order_relaxed);
+        again = v == mine;
+        if (!again && v && n < 4 && std::find(seen, seen + n, v) == seen + n) seen[n++] = v;
     }
-    return n;
+    r.stream[at % kLast].store(mine, std::memory_order_relaxed);
+    return again ? n : 0;
 }
 
 PencilConfig choose(int kind, const GridDesc& g, int sharing = kAlone) {

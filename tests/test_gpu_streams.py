@@ -117,8 +117,8 @@ def test_steps_behind_a_join_of_two_streams(torch_cuda, captured, kind, branch):
 
 @pytest.mark.parametrize("kind", ["wave", "exact", "heat", "half", "ragged"])
 def test_steps_on_five_streams_give_the_bits_of_one(torch_cuda, kind):
-    """Rounds of steps of unlike grids, each on its own stream (from the third stream on they
-    take another tile and split than alone), against each grid by itself."""
+    """Rounds of steps of unlike grids, each on its own stream (beside two others they take
+    another tile and split than alone), against each grid by itself."""
     torch = torch_cuda
     shapes = [(96, 88, 80), (128, 64, 100), (160, 72, 61), (64, 120, 90), (200, 48, 77)]
     sets = []
@@ -147,9 +147,7 @@ def test_steps_on_five_streams_give_the_bits_of_one(torch_cuda, kind):
 
     want = []
     for g, p, q, v, scale in sets:
-        for _ in range(4):  # 28 launches on one stream: alone
-            one = run(g, p.clone(), q.clone(), v, scale, None)
-        want.append(one)
+        want.append(run(g, p.clone(), q.clone(), v, scale, None))
     torch.cuda.synchronize()
     streams = [torch.cuda.Stream() for _ in sets]
     state = [[p.clone(), q.clone()] for _, p, q, _, _ in sets]
