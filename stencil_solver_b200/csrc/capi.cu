@@ -214,10 +214,11 @@ const Family kFamilies[] = {
     // kExactHeat
     {2.1, 8, {{"t32x16_r1_s8", 1.0, 1.0}, {"t64x16_r2_s8", 0.96, 0.96}}, "t32x16_r1_s8",
      "t32x16_r1_s8"},
-    // kPrepass beyond L2 (smaller grids: as the acoustic step).  It writes two fields and pays
-    // more for a chunk's start; the acoustic step's choice took 10 to 14 % longer than the one
-    // 64 x 32 CTA per SM before it on some grids (192 x 1024 x 1024 805 and 715 us, 440^3 310
-    // and 283).  Over 22 grids now at most 4 % longer than the better of the two, 715 and 281.
+    // kPrepass beyond L2, 32 interior planes and more (else as the acoustic step: 2048 x 1025
+    // x 17 74 us, with this choice 81).  It writes two fields and pays more for a chunk's
+    // start; the acoustic step's choice took 10 to 14 % longer than the one 64 x 32 CTA per SM
+    // before it on some grids (192 x 1024 x 1024 805 and 715 us, 440^3 310 and 283).  Over 22
+    // grids now at most 4 % longer than the better of the two, 715 and 281.
     {10, 12, {{"t64x32_r2_s8_a3", 0, 1.02}, {"t128x32_r2_s7_a2", 0, 0.96}}, "", ""},
 };
 constexpr double kL2Bytes = 126e6;
@@ -244,7 +245,7 @@ int resident_ctas(int kind, int v) {
 // The cheapest tile and split of a family (a public kind's or a reference-order one).
 PencilConfig cheapest(int family, const GridDesc& g, int sharing) {
     const bool beyond = double(g.size()) * kFamilies[family].step_bytes > kL2Bytes;
-    if (family == kPrepass && !beyond) family = SB200_KIND_WAVE_F32;
+    if (family == kPrepass && (!beyond || g.nz < 40)) family = SB200_KIND_WAVE_F32;
     const Family& f = kFamilies[family];
     const bool exact = reference_order(family);
     const int kind = public_kind(family);
