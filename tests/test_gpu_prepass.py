@@ -104,4 +104,4 @@ def test_untuned_choice_beyond_l2(torch_cuda):
     finally:
         sb.set_pencil_override(sb.KIND_WAVE_F32, -1, 1)
     print(pairs)
-    assert min(a for a, _ in pairs) <= 1.05 * min(b for _, b in pairs)
+    assert min(a for a, _ in pairs) <= 1.08 * min(b for _, b in pairs)
